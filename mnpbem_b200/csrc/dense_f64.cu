@@ -7,6 +7,7 @@
 // other matrices in the batch.
 #include "common.cuh"
 #include "dense_f64.cuh"
+#include "lu_panel.cuh"
 
 namespace mnpb {
 
@@ -405,16 +406,38 @@ static int laswp_range(cudaStream_t s, cd *A, int64_t lda, int64_t sA, int j0, i
     return MNPB_OK;
 }
 
+// Columns of an LU leaf over m rows: what the cluster's registers hold (32, 16
+// or 8 columns of 1, 2 or 4 rows a thread); beyond that the leaf in global
+// memory takes 32.
+static int leaf_width(int m) {
+    int C, threads;
+    if (lup::panel_shape(m, 1, C, threads)) return TS;
+    if (lup::panel_shape(m, 2, C, threads)) return TS / 2;
+    if (lup::panel_shape(m, 4, C, threads)) return TS / 4;
+    return TS;
+}
+
 // Recursive LU: factor columns [off, off+w) over rows [off, n); absolute pivots.
 static int rgetrf(cudaStream_t s, int n, int off, int w, int batch, cd *A, int64_t lda,
                   int64_t sA, int32_t *ipiv, int64_t sP, int32_t *info) {
-    if (w <= TS) {
+    if (w <= leaf_width(n - off)) {
         ProfScope ps(s, PC_PANEL, 8.0 * w * w * (double)(n - off) * batch / 2);
+        const lup::F64::Mat mat{A, lda, sA};
+        int C, threads;
+        if (lup::panel_shape(n - off, 1, C, threads))
+            return lup::launch_panel<lup::F64, TS, 1>(s, n, off, w, mat, ipiv, sP, info, batch, C,
+                                                      threads);
+        if (lup::panel_shape(n - off, 2, C, threads))
+            return lup::launch_panel<lup::F64, TS / 2, 2>(s, n, off, w, mat, ipiv, sP, info,
+                                                          batch, C, threads);
+        if (lup::panel_shape(n - off, 4, C, threads))
+            return lup::launch_panel<lup::F64, TS / 4, 4>(s, n, off, w, mat, ipiv, sP, info,
+                                                          batch, C, threads);
         panel_kernel<<<batch, PANEL_THREADS, 0, s>>>(n, off, w, A, lda, sA, ipiv, sP, info);
         MNPB_LAUNCH_CHECK("panel_kernel");
         return MNPB_OK;
     }
-    const int w1 = split_point(w);
+    const int w1 = w > TS ? split_point(w) : leaf_width(n - off);
     MNPB_TRY(rgetrf(s, n, off, w1, batch, A, lda, sA, ipiv, sP, info));
     MNPB_TRY(laswp_range(s, A, lda, sA, off + w1, off + w, ipiv, sP, off, off + w1, batch));
     cd *A11 = A + off + (int64_t)off * lda;

@@ -1,0 +1,271 @@
+// LU panel with partial pivoting, held in registers and spread over a thread
+// block cluster.
+//
+// One cluster of C CTAs factors the columns [k0, k0 + kb) (kb <= W) of one
+// matrix over the rows [k0, n).  Every thread keeps R rows x W columns in
+// registers from load to store, so a column step touches no memory but the
+// pivot row: the rows are dealt to the CTAs in blocks of R * blockDim.x.
+//
+// What bounds it: the chain of kb dependent pivot steps.  A step is a warp
+// and CTA reduction of the pivot candidates, one exchange between the CTAs,
+// and the rank-1 update.  Each CTA's best row is pushed to every CTA of the
+// cluster (distributed shared memory) together with its value before the
+// exchange's one cluster barrier, so the winner's row is local to all CTAs
+// when the barrier opens.  Rows never move: each carries the row position it
+// would have after the interchanges so far (`pos`), an interchange swaps two
+// positions, and the rows are stored at their final positions at the end.
+//
+// Two buffers alternate between steps: a push into buffer (j & 1) for step
+// j + 2 comes after the barrier of step j + 1, which every thread reaches
+// only after its reads of step j.  The last remote store precedes the last
+// barrier, so no CTA of the cluster is written to after it has left.
+//
+// Measured (FP64 LU of one n x n matrix, all else equal) against the leaf it
+// replaces, one CTA per matrix working in global memory: n = 284 1.44 -> 0.94
+// ms, 1365 16.0 -> 7.5, 2884 63.7 -> 22.0, 7000 348 -> 106; 41 matrices of
+// 1148 23.1 -> 16.9.  A pivot step takes 1.4 us in one CTA and 2.1 us in a
+// cluster of 8.
+#pragma once
+#include "common.cuh"
+
+namespace mnpb {
+namespace lup {
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(const void *p, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+// FP64 interleaved storage (column-major complex128).
+struct F64 {
+    typedef cd V;
+    typedef double S;
+    struct Mat {
+        cd *A;
+        int64_t lda, sA;
+    };
+    static __device__ __forceinline__ V zero() { return cmk(0.0, 0.0); }
+    static __device__ __forceinline__ V load(const Mat &m, int64_t b, int64_t row, int64_t col) {
+        return m.A[b * m.sA + col * m.lda + row];
+    }
+    static __device__ __forceinline__ void store(const Mat &m, int64_t b, int64_t row,
+                                                 int64_t col, V v) {
+        m.A[b * m.sA + col * m.lda + row] = v;
+    }
+    static __device__ __forceinline__ S mag(V v) { return cabs1(v); }
+    static __device__ __forceinline__ V rcp(V v) { return crcp(v); }
+    static __device__ __forceinline__ V mul(V a, V b) { return cmul(a, b); }
+    static __device__ __forceinline__ V fms(V a, V b, V c) { return cfms(a, b, c); }
+    static __device__ __forceinline__ V rnd(V v) { return v; }   // storage precision of L and U
+    static __device__ __forceinline__ void push(uint32_t addr, V v) {
+        asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y)
+                     : "memory");
+    }
+    static __device__ __forceinline__ void push_s(uint32_t addr, S v) {
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+    }
+};
+
+constexpr int MAXC = 8;          // CTAs per cluster (portable limit)
+constexpr int MAXW = 12;         // warps per CTA
+constexpr int NOROW = 0x7fffffff;
+
+// larger magnitude first, then the smaller row position (the first row of the
+// maximal |re| + |im| in the interchanged order)
+template <typename S>
+__device__ __forceinline__ bool better(S v, int p, S bv, int bp) {
+    return v > bv || (v == bv && p < bp);
+}
+
+template <typename T, int W, int R>
+__global__ void __launch_bounds__(32 * MAXW, 1)
+    panel_kernel(int n, int k0, int kb, typename T::Mat A, int32_t *ipiv, int64_t sP,
+                 int32_t *info, int C) {
+    typedef typename T::V V;
+    typedef typename T::S S;
+    __shared__ __align__(16) V rowbuf[2][MAXC][W];   // every CTA's best row
+    __shared__ S cand_v[2][MAXC];
+    __shared__ int cand_p[2][MAXC];
+    __shared__ S red_v[2][MAXW];
+    __shared__ int red_p[2][MAXW];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int nw = blockDim.x >> 5;
+    const uint32_t me = C > 1 ? cluster_rank() : 0;
+    const int64_t b = blockIdx.x / C;
+    const int m = n - k0;
+    V a[R][W];
+    int pos[R];                       // row position relative to k0; done rows: < jj
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = (int)me * R * blockDim.x + r * blockDim.x + tid;
+        pos[r] = i < m ? i : NOROW;
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            a[r][j] = (i < m && j < kb) ? T::load(A, b, k0 + i, k0 + j) : T::zero();
+    }
+    if (C > 1) cluster_sync();        // every CTA of the cluster has started
+#pragma unroll
+    for (int jj = 0; jj < W; ++jj) {
+        if (jj < kb) {
+            const int buf = jj & 1;
+            // best of this thread's active rows, then of the warp, then of the CTA
+            S bv = (S)-1;
+            int bp = NOROW;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const S t = T::mag(a[r][jj]);
+                const S v = t > (S)0 ? t : (S)0;       // NaN counts as zero
+                if (pos[r] != NOROW && pos[r] >= jj && better(v, pos[r], bv, bp)) {
+                    bv = v;
+                    bp = pos[r];
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int op = __shfl_xor_sync(0xffffffffu, bp, o);
+                if (better(ov, op, bv, bp)) { bv = ov; bp = op; }
+            }
+            if (lane == 0) { red_v[buf][wid] = bv; red_p[buf][wid] = bp; }
+            __syncthreads();
+            bv = lane < nw ? red_v[buf][lane] : (S)-1;
+            bp = lane < nw ? red_p[buf][lane] : NOROW;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int op = __shfl_xor_sync(0xffffffffu, bp, o);
+                if (better(ov, op, bv, bp)) { bv = ov; bp = op; }
+            }
+            bv = __shfl_sync(0xffffffffu, bv, 0);
+            bp = __shfl_sync(0xffffffffu, bp, 0);
+            // the warp that holds the CTA's best row publishes it
+            bool mine = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (bp != NOROW && pos[r] == bp) {
+                    mine = true;
+#pragma unroll
+                    for (int j = jj; j < W; ++j) rowbuf[buf][me][j] = T::rnd(a[r][j]);
+                }
+            if (C > 1) {
+                const bool ours = __any_sync(0xffffffffu, mine);
+                if (ours) {
+                    __syncwarp();
+                    if (lane >= jj && lane < W) {
+                        const V v = rowbuf[buf][me][lane];
+                        for (int q = 0; q < C; ++q)
+                            if (q != (int)me)
+                                T::push(map_rank(&rowbuf[buf][me][lane], q), v);
+                    }
+                }
+                // CTAs without active rows publish "none"
+                if (wid == 0 && lane < C) {
+                    T::push_s(map_rank(&cand_v[buf][me], lane), bv);
+                    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(
+                                     map_rank(&cand_p[buf][me], lane)),
+                                 "r"(bp)
+                                 : "memory");
+                }
+                cluster_sync();
+            } else {
+                __syncthreads();
+            }
+            int win = 0;
+            if (C > 1) {
+                bv = lane < C ? cand_v[buf][lane] : (S)-1;
+                bp = lane < C ? cand_p[buf][lane] : NOROW;
+                win = lane;
+#pragma unroll
+                for (int o = MAXC / 2; o > 0; o >>= 1) {
+                    const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                    const int op = __shfl_xor_sync(0xffffffffu, bp, o);
+                    const int ow = __shfl_xor_sync(0xffffffffu, win, o);
+                    if (better(ov, op, bv, bp)) { bv = ov; bp = op; win = ow; }
+                }
+                bv = __shfl_sync(0xffffffffu, bv, 0);
+                bp = __shfl_sync(0xffffffffu, bp, 0);
+                win = __shfl_sync(0xffffffffu, win, 0);
+            }
+            if (me == 0 && tid == 0) {
+                ipiv[b * sP + k0 + jj] = k0 + bp;
+                if (!(bv > (S)0) && info && info[b] == 0) info[b] = k0 + jj + 1;
+            }
+            const V *u = rowbuf[buf][win];
+            const V pv = u[jj];
+            const bool nz = pv.x != (S)0 || pv.y != (S)0;
+            const V inv = nz ? T::rcp(pv) : T::zero();
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                // the interchange of positions jj and bp
+                const int p = pos[r];
+                if (p == bp) {
+                    pos[r] = jj;
+#pragma unroll
+                    for (int j = jj; j < W; ++j) a[r][j] = T::rnd(a[r][j]);
+                } else {
+                    if (p == jj) pos[r] = bp;
+                    if (pos[r] > jj && pos[r] != NOROW) {
+                        V l = a[r][jj];
+                        if (nz) l = T::rnd(T::mul(l, inv));
+                        a[r][jj] = l;
+#pragma unroll
+                        for (int j = jj + 1; j < W; ++j) a[r][j] = T::fms(l, u[j], a[r][j]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (pos[r] != NOROW) {
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+                if (j < kb) T::store(A, b, k0 + pos[r], k0 + j, a[r][j]);
+        }
+}
+
+// Launch shape for m rows of `batch` matrices: CTAs per cluster and threads
+// per CTA; false if the rows do not fit in MAXC CTAs.
+inline bool panel_shape(int m, int R, int &C, int &threads) {
+    const int per = 32 * MAXW * R;
+    C = ceil_div(m, per);
+    if (C > MAXC) return false;
+    threads = 32 * ceil_div(ceil_div(m, C * R), 32);
+    return true;
+}
+
+template <typename T, int W, int R>
+int launch_panel(cudaStream_t s, int n, int k0, int kb, typename T::Mat A, int32_t *ipiv,
+                 int64_t sP, int32_t *info, int batch, int C, int threads) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(batch * C));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, panel_kernel<T, W, R>, n, k0, kb, A, ipiv, sP, info, C) !=
+        cudaSuccess) {
+        set_error("LU panel: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        return MNPB_ECUDA;
+    }
+    MNPB_LAUNCH_CHECK("lup::panel_kernel");
+    return MNPB_OK;
+}
+
+}  // namespace lup
+}  // namespace mnpb

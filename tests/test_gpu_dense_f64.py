@@ -1,0 +1,83 @@
+"""FP64 dense building blocks at the sizes where their kernels change: LU
+panels (rows per CTA, CTAs per cluster, columns per leaf, remainders)."""
+import numpy as np
+import pytest
+import scipy.linalg as sla
+import torch
+
+from mnpbem_b200 import _lib
+from mnpbem_b200._lib import call, ptr
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+def _rand(*shape, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(shape + (2,), generator=g, dtype=torch.float64)
+    return torch.view_as_complex(x).cuda()
+
+
+def _getrf(A):
+    """LU of A (batch, n, n), stored column by column: factors, pivots, info."""
+    B, n, _ = A.shape
+    LU = A.clone()
+    piv = torch.zeros((B, n), dtype=torch.int32, device='cuda')
+    info = torch.zeros(B, dtype=torch.int32, device='cuda')
+    call('mnpb_getrf_f64', _lib.stream_handle(), n, B, ptr(LU), n, n * n, ptr(piv), n, ptr(info))
+    torch.cuda.synchronize()
+    return LU, piv, info
+
+
+def _check_lu(A, LU, piv):
+    """|P A - L U| <= 4 n eps |L| |U|, entrywise bounded by its maximum (the
+    standard backward error bound of LU, complex arithmetic)."""
+    n = A.shape[-1]
+    for a, f, p in zip(A, LU, piv.cpu().numpy()):
+        M = f.transpose(0, 1)
+        L = torch.tril(M, -1)
+        L.diagonal().fill_(1.0)
+        U = torch.triu(M)
+        perm = np.arange(n)
+        for c, r in enumerate(p):
+            perm[[c, r]] = perm[[r, c]]
+        err = (a.transpose(0, 1)[torch.from_numpy(perm).cuda()] - L @ U).abs().max()
+        bound = 4 * n * EPS * (L.abs() @ U.abs()).max()
+        assert float(err) <= float(bound)
+
+
+@pytest.mark.parametrize('n,batch', [(1, 3), (7, 2), (31, 1), (32, 2), (33, 5), (65, 150),
+                                     (384, 2), (385, 2), (417, 1), (800, 3), (1200, 1)])
+def test_lu_matches_lapack_pivots(gpu_ok, n, batch):
+    A = _rand(batch, n, n, seed=n)
+    LU, piv, info = _getrf(A)
+    assert not info.any()
+    _check_lu(A, LU, piv)
+    for a, p in zip(A[:3].cpu().numpy(), piv[:3].cpu().numpy()):
+        assert np.array_equal(sla.lu_factor(a.T)[1], p)
+
+
+@pytest.mark.parametrize('n', [3073, 3105, 6150])
+def test_lu_narrow_leaves(gpu_ok, n):
+    # more rows than 8 CTAs hold 32 (16) columns of: 16- (8-) column leaves
+    A = _rand(1, n, n, seed=n)
+    LU, piv, info = _getrf(A)
+    assert not info.any()
+    _check_lu(A, LU, piv)
+
+
+@pytest.mark.parametrize('n', [5, 40, 500])
+def test_lu_ties_and_zero_columns(gpu_ok, n):
+    # equal magnitudes: the first row wins; a zero column leaves its diagonal
+    # in place and is reported once, by its first index
+    A = torch.ones((2, n, n), dtype=torch.complex128, device='cuda')
+    A[0] = torch.tril(A[0])                      # upper triangular matrix of ones
+    A[1].zero_()
+    A[1].diagonal().fill_(1.0 + 1.0j)
+    A[1, n // 2] = 0.0                           # column n // 2
+    LU, piv, info = _getrf(A)
+    want = np.arange(n)
+    assert np.array_equal(piv.cpu().numpy(), np.stack([want, want]))
+    assert info.cpu().tolist() == [0, n // 2 + 1]
+    assert torch.equal(LU[1], A[1])
