@@ -12,98 +12,138 @@
 namespace mnpb {
 
 // ---------------------------------------------------------------------------
-// GEMM: C = alpha A B + beta C, all no-transpose.  64x64 tile per CTA,
-// 128 threads, each thread 8 rows x 4 columns (columns interleaved by 16 so
-// that the shared-memory reads of B are conflict free).
+// GEMM: C = alpha A B + beta C, all no-transpose, on the FP64 tensor path
+// (mma.sync m16n8k4, FP64 accumulation; there is no tcgen05 kind for FP64).
+// Four warps per CTA, each a (BM/2) x (BN/2) block of real and imaginary
+// accumulators; operands come through a ring of cp.async stages as they are
+// stored (interleaved complex), so one 16-byte shared load feeds both parts.
+// Shared strides: A columns are BM + 2 elements and B columns 12 elements
+// apart, so that the eight lanes of a 128-bit load phase (2 rows x 4 k) hit
+// eight different 16-byte bank groups.  Bound by the FP64 pipe (37 TFLOP/s):
+// 2884 x 2884 x 2884 8.51 -> 6.54 ms (29.3 TFLOP/s), 41 x 1148 x 512 x 512
+// 4.01 -> 3.00 ms (32.9) against the FMA kernel with one 64 x 64 tile shape
+// this replaces.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int GBM = 64, GBN = 64, GBK = 8;
+constexpr int GK = 8, GSTAGES = 4, GTHREADS = 128;
+constexpr int GBS = GK + 4;   // B column stride in shared memory
 
-__global__ void __launch_bounds__(128, 2) zgemm_kernel(int m, int n, int k, cd alpha,
-                                                       const cd *__restrict__ A, int64_t lda,
-                                                       int64_t sA, const cd *__restrict__ B,
-                                                       int64_t ldb, int64_t sB, cd beta,
-                                                       cd *__restrict__ C, int64_t ldc,
-                                                       int64_t sC) {
-    // B rows padded by one element: the loader's 8 consecutive threads store
-    // 8 different rows, which must not share shared-memory banks
-    __shared__ cd As[GBK][GBM];
-    __shared__ cd Bs[GBK][GBN + 1];
-    const int tid = threadIdx.x;
-    const int tn = tid & 15, tm = tid >> 4;
-    const int m0 = blockIdx.x * GBM, n0 = blockIdx.y * GBN;
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+                 "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
+                 "{%6}, {%0,%1,%2,%3};"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+
+template <int BM, int BN>
+__global__ void __launch_bounds__(GTHREADS) zgemm_kernel(int m, int n, int k, cd alpha,
+                                                         const cd *__restrict__ A, int64_t lda,
+                                                         int64_t sA, const cd *__restrict__ B,
+                                                         int64_t ldb, int64_t sB, cd beta,
+                                                         cd *__restrict__ C, int64_t ldc,
+                                                         int64_t sC) {
+    constexpr int AS = BM + 2;               // A column (fixed k) stride
+    constexpr int MI = BM / 32, NI = BN / 16;   // 16 x 8 fragments per warp
+    extern __shared__ __align__(16) cd zsm[];
+    cd *As = zsm;                            // [GSTAGES][GK][AS]
+    cd *Bs = zsm + GSTAGES * GK * AS;        // [GSTAGES][BN][GBS]
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int wm = (wid & 1) * (BM / 2), wn = (wid >> 1) * (BN / 2);
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     const int64_t b = blockIdx.z;
     A += b * sA;
     B += b * sB;
     C += b * sC;
-    cd acc[8][4];
+    double re[MI][NI][4], im[MI][NI][4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = cmk(0.0, 0.0);
-
-    const int ar = tid & 63, ak = tid >> 6;   // A loader: row, first k
-    const int bk = tid & 7, bc = tid >> 3;    // B loader: k, first column
-    cd pa[4], pb[4];
-    auto load = [&](int k0) {
+        for (int j = 0; j < NI; ++j)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int gr = m0 + ar, gk = k0 + ak + 2 * q;
-            pa[q] = (gr < m && gk < k) ? A[(int64_t)gk * lda + gr] : cmk(0.0, 0.0);
-        }
+            for (int e = 0; e < 4; ++e) re[i][j][e] = im[i][j][e] = 0.0;
+    const int nk = (k + GK - 1) / GK;
+    auto load = [&](int kt) {
+        if (kt < nk) {
+            const int st = kt % GSTAGES, k0 = kt * GK;
+            const uint32_t da = (uint32_t)__cvta_generic_to_shared(As + st * GK * AS);
+            const uint32_t db = (uint32_t)__cvta_generic_to_shared(Bs + st * BN * GBS);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int gc = n0 + bc + 16 * q, gk = k0 + bk;
-            pb[q] = (gc < n && gk < k) ? B[(int64_t)gc * ldb + gk] : cmk(0.0, 0.0);
-        }
-    };
-    if (k > 0) load(0);
-    for (int k0 = 0; k0 < k; k0 += GBK) {
+            for (int e = tid; e < BM * GK; e += GTHREADS) {
+                const int r = e % BM, kk = e / BM;
+                const bool ok = m0 + r < m && k0 + kk < k;
+                cp16(da + (kk * AS + r) * 16, ok ? A + (int64_t)(k0 + kk) * lda + m0 + r : A, ok);
+            }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) As[ak + 2 * q][ar] = pa[q];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) Bs[bk][bc + 16 * q] = pb[q];
-        __syncthreads();
-        if (k0 + GBK < k) load(k0 + GBK);   // next tile in flight during the math
-#pragma unroll
-        for (int kk = 0; kk < GBK; ++kk) {
-            cd bv[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) bv[c] = Bs[kk][tn + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const cd a = As[kk][tm * 8 + r];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = cfma(a, bv[c], acc[r][c]);
+            for (int e = tid; e < BN * GK; e += GTHREADS) {
+                const int kk = e % GK, c = e / GK;
+                const bool ok = n0 + c < n && k0 + kk < k;
+                cp16(db + (c * GBS + kk) * 16, ok ? B + (int64_t)(n0 + c) * ldb + k0 + kk : B, ok);
             }
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int q = 0; q < GSTAGES - 1; ++q) load(q);
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GSTAGES - 2) : "memory");
+        __syncthreads();                       // stage kt has landed; stage kt - 1 is free
+        load(kt + GSTAGES - 1);
+        const cd *as = As + (kt % GSTAGES) * GK * AS + wm + g;
+        const cd *bs = Bs + (kt % GSTAGES) * BN * GBS + (wn + g) * GBS;
+#pragma unroll
+        for (int ks = 0; ks < GK; ks += 4) {
+            cd av[MI][2], bv[NI];
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) av[i][h] = as[(ks + t) * AS + 16 * i + 8 * h];
+#pragma unroll
+            for (int j = 0; j < NI; ++j) bv[j] = bs[8 * j * GBS + ks + t];
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) {
+                    mma_f64(re[i][j], av[i][0].x, av[i][1].x, bv[j].x);
+                    mma_f64(im[i][j], av[i][0].x, av[i][1].x, bv[j].y);
+                }
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) {
+                    mma_f64(re[i][j], -av[i][0].y, -av[i][1].y, bv[j].y);
+                    mma_f64(im[i][j], av[i][0].y, av[i][1].y, bv[j].x);
+                }
+        }
     }
     const bool beta0 = (beta.x == 0.0 && beta.y == 0.0);
-    // two halves of the C fragment: all loads of a half in flight, then stores
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        cd cv[8][2];
+    for (int i = 0; i < MI; ++i) {
+        cd cv[NI][4];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int gc = n0 + tn + 16 * (2 * h + c);
+        for (int j = 0; j < NI; ++j)
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int gr = m0 + tm * 8 + r;
-                cv[r][c] = (!beta0 && gc < n && gr < m) ? __ldg(C + (int64_t)gc * ldc + gr)
+            for (int e = 0; e < 4; ++e) {
+                const int gr = m0 + wm + 16 * i + g + 8 * (e >> 1);
+                const int gc = n0 + wn + 8 * j + 2 * t + (e & 1);
+                cv[j][e] = (!beta0 && gr < m && gc < n) ? C[(int64_t)gc * ldc + gr]
                                                         : cmk(0.0, 0.0);
             }
-        }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int gc = n0 + tn + 16 * (2 * h + c);
+        for (int j = 0; j < NI; ++j)
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int gr = m0 + tm * 8 + r;
-                if (gc < n && gr < m)
-                    C[(int64_t)gc * ldc + gr] = cfma(beta, cv[r][c], cmul(alpha, acc[r][2 * h + c]));
+            for (int e = 0; e < 4; ++e) {
+                const int gr = m0 + wm + 16 * i + g + 8 * (e >> 1);
+                const int gc = n0 + wn + 8 * j + 2 * t + (e & 1);
+                if (gr < m && gc < n)
+                    C[(int64_t)gc * ldc + gr] =
+                        cfma(beta, cv[j][e], cmul(alpha, cmk(re[i][j][e], im[i][j][e])));
             }
-        }
     }
 }
 
@@ -306,20 +346,40 @@ __global__ void set_identity_kernel(cd *W, int64_t ldw, int64_t sW, int n) {
 // ---------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------
+template <int BM, int BN>
+static int launch_zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A,
+                        int64_t lda, int64_t sA, const cd *B, int64_t ldb, int64_t sB, cd beta,
+                        cd *C, int64_t ldc, int64_t sC) {
+    const int smem = GSTAGES * (GK * (BM + 2) + BN * GBS) * (int)sizeof(cd);
+    MNPB_TRY(smem_opt_in(zgemm_kernel<BM, BN>, smem, "zgemm_kernel"));
+    dim3 grid(ceil_div(m, BM), ceil_div(n, BN), batch);
+    zgemm_kernel<BM, BN><<<grid, GTHREADS, smem, s>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB,
+                                                      beta, C, ldc, sC);
+    MNPB_LAUNCH_CHECK("zgemm_kernel");
+    return MNPB_OK;
+}
+
 int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A, int64_t lda,
           int64_t sA, const cd *B, int64_t ldb, int64_t sB, cd beta, cd *C, int64_t ldc,
           int64_t sC) {
     if (m <= 0 || n <= 0 || batch <= 0) return MNPB_OK;
-    dim3 grid(ceil_div(m, GBM), ceil_div(n, GBN), batch);
     ProfScope ps(s, PC_ZGEMM, 8.0 * m * n * (double)(k > 0 ? k : 0) * batch);
-    if (k <= 0) {
-        // C = beta C
-        zgemm_kernel<<<grid, 128, 0, s>>>(m, n, 0, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
-    } else {
-        zgemm_kernel<<<grid, 128, 0, s>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
-    }
-    MNPB_LAUNCH_CHECK("zgemm_kernel");
-    return MNPB_OK;
+    // C = beta C for k <= 0
+    // 64 x 64 tiles once two CTAs per SM have one; smaller tiles until then,
+    // so that small updates and few right-hand sides spread over the SMs
+    // (2800 x 32 x 32, 2 matrices: 20.7 -> 14.6 us; 2884 x 4 x 2884, which a
+    // 64-column tile padded 16-fold: 795 -> 157 us)
+    const int kk = k > 0 ? k : 0;
+    const int64_t t64 = (int64_t)ceil_div(m, 64) * ceil_div(n, 64) * batch;
+    const int64_t t32 = (int64_t)ceil_div(m, 64) * ceil_div(n, 32) * batch;
+    if (t64 >= 2 * device_sms() && n > 32)
+        return launch_zgemm<64, 64>(s, m, n, kk, batch, alpha, A, lda, sA, B, ldb, sB, beta, C,
+                                    ldc, sC);
+    if (t32 >= 2 * device_sms())
+        return launch_zgemm<64, 32>(s, m, n, kk, batch, alpha, A, lda, sA, B, ldb, sB, beta, C,
+                                    ldc, sC);
+    return launch_zgemm<32, 32>(s, m, n, kk, batch, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,
+                                sC);
 }
 
 static int trsm_small(cudaStream_t s, int mode, int kb, const cd *T, int64_t ldt, int64_t sT,

@@ -1,5 +1,6 @@
 """FP64 dense building blocks at the sizes where their kernels change: LU
-panels (rows per CTA, CTAs per cluster, columns per leaf, remainders)."""
+panels (rows per CTA, CTAs per cluster, columns per leaf, remainders) and
+matrix products (tile edges, depth remainders, strides)."""
 import numpy as np
 import pytest
 import scipy.linalg as sla
@@ -81,3 +82,26 @@ def test_lu_ties_and_zero_columns(gpu_ok, n):
     assert np.array_equal(piv.cpu().numpy(), np.stack([want, want]))
     assert info.cpu().tolist() == [0, n // 2 + 1]
     assert torch.equal(LU[1], A[1])
+
+
+@pytest.mark.parametrize('m,n,k,batch', [(1, 1, 1, 1), (33, 31, 7, 2), (32, 32, 8, 1),
+                                         (64, 4, 33, 3), (65, 65, 25, 1), (700, 33, 40, 5),
+                                         (640, 70, 9, 40), (1300, 1290, 64, 1), (50, 40, 0, 2)])
+@pytest.mark.parametrize('alpha,beta', [(-1.0, 1.0), (0.5 - 2.0j, 0.0), (1.0j, -0.25 + 1.0j)])
+def test_zgemm_tiles(gpu_ok, m, n, k, batch, alpha, beta):
+    # leading dimensions and strides larger than the matrices
+    lda, ldb, ldc = m + 3, k + 2, m + 1
+    A = _rand(batch, k + 1, lda, seed=1)
+    B = _rand(batch, n + 2, ldb, seed=2)
+    C0 = _rand(batch, n + 1, ldc, seed=3)
+    C = C0.clone()
+    al, be = complex(alpha), complex(beta)
+    call('mnpb_zgemm', _lib.stream_handle(), m, n, k, batch, al.real, al.imag, ptr(A), lda,
+         (k + 1) * lda, ptr(B), ldb, (n + 2) * ldb, be.real, be.imag, ptr(C), ldc, (n + 1) * ldc)
+    a, b = A[:, :k, :m].transpose(1, 2), B[:, :n, :k].transpose(1, 2)
+    c = C0[:, :n, :m].transpose(1, 2)
+    ref = al * (a @ b) + be * c
+    bound = 4 * (k + 3) * EPS * (abs(al) * (a.abs() @ b.abs()) + abs(be) * c.abs())
+    got = C[:, :n, :m].transpose(1, 2)
+    assert bool(((got - ref).abs() <= bound).all())
+    assert torch.equal(C[:, n:], C0[:, n:]) and torch.equal(C[:, :, m:], C0[:, :, m:])
