@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(GTHREADS) zgemm_kernel(int m, int n, int k, cd
 // Pivot = first row of maximal |re|+|im| (LAPACK izamax rule).
 // ---------------------------------------------------------------------------
 constexpr int PANEL_THREADS = 512;
+constexpr int TS = 32;         // columns of an LU leaf
 
 __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(int n, int k0, int kb, cd *A,
                                                               int64_t lda, int64_t sA,
@@ -273,64 +274,250 @@ __global__ void colswp_kernel(cd *X, int64_t ldx, int64_t sX, int m, const int32
     }
 }
 
-// Small triangular solves on a kb x kb diagonal block (kb <= 32).
-// mode 0: left lower unit     L x = b   (one thread per column of B)
-// mode 1: left upper non-unit U x = b   (one thread per column of B)
-// mode 2: right upper non-unit x U = b  (one thread per row of B)
-// mode 3: right lower unit     x L = b  (one thread per row of B)
-constexpr int TS = 32;
+// ---------------------------------------------------------------------------
+// Row interchanges.  A sequence of interchanges (c, p_c), c ascending, p_c >= c,
+// is composed into a gather before any row moves: row c ends with the value
+// that row p_c held just before step c, which is V(c') of the last earlier
+// step c' with the same target, or the original row p_c; V(c), the value of
+// row c before step c, is V of the last earlier step that targeted c, or the
+// original row c.  Steps with one target are chained (next), so each step
+// walks the few that share its target instead of all that precede it.
+// Shared memory: head of every target row met, by its slot.
+// ---------------------------------------------------------------------------
+constexpr int SWN = 128;   // interchanges composed by one strip CTA
 
-__global__ void __launch_bounds__(128) trsm_small_kernel(int mode, int kb, const cd *T,
-                                                         int64_t ldt, int64_t sT, cd *B,
-                                                         int64_t ldb, int64_t sB, int nvec) {
-    __shared__ cd Ts[TS][TS + 1];
-    const int64_t b = blockIdx.y;
-    T += b * sT;
-    B += b * sB;
-    for (int e = threadIdx.x; e < TS * TS; e += blockDim.x) {
-        int r = e % TS, c = e / TS;
-        Ts[r][c] = (r < kb && c < kb) ? T[(int64_t)c * ldt + r] : cmk(r == c ? 1.0 : 0.0, 0.0);
+struct Swaps {             // in shared memory
+    int p[SWN];            // target of step c, relative to the first step's row
+    int par[SWN];          // last earlier step that targeted row c, or -1
+    int out[SWN];          // row (relative) whose value ends in row c
+    int tail[SWN];         // for the last step of a target below the steps' own rows:
+                           // the row whose value ends there; else -1
+};
+
+// compose steps [0, ns), ns <= SWN <= blockDim.x, one thread a step; ends with a barrier
+__device__ __forceinline__ void swaps_compose(Swaps &w, const int32_t *ipiv, int base, int ns) {
+    const int c = threadIdx.x;
+    if (c < ns) w.p[c] = ipiv[c] - base;
+    __syncthreads();
+    const int t = c < ns ? w.p[c] : -1;
+    int par = -1, prev = -1;              // last earlier step with target c / target t
+    bool last = t >= ns;
+    for (int e = 0; e < ns; ++e) {
+        const int pe = w.p[e];
+        if (e < c) {
+            if (pe == c && e != c) par = e;
+            if (pe == t) prev = e;
+        } else if (e > c && pe == t) {
+            last = false;
+        }
+    }
+    if (c < ns) w.par[c] = par;
+    __syncthreads();
+    if (c < ns) {
+        auto before = [&](int e) {        // V(e)
+            while (w.par[e] >= 0) e = w.par[e];
+            return e;
+        };
+        w.out[c] = t == c ? before(c) : prev >= 0 ? before(prev) : t;
+        w.tail[c] = last ? before(c) : -1;
     }
     __syncthreads();
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nvec) return;
-    cd x[TS];
-    const bool left = (mode < 2);
-    // element e of the vector: left -> B(e, v); right -> B(v, e)
+}
+
+// ---------------------------------------------------------------------------
+// Triangular solves on a diagonal block of up to SN = 128 rows, one CTA per
+// strip of SV = 32 right-hand sides held in shared memory.
+// mode 0: left lower unit     L x = b   (vectors: columns of B)
+// mode 1: left upper non-unit U x = b   (vectors: columns of B)
+// mode 2: right upper non-unit x U = b  (vectors: rows of B)
+// mode 3: right lower unit     x L = b  (vectors: rows of B)
+// All four are one forward substitution with the triangle in the order of the
+// solve: M(l, k) = op(T)(phys(l), phys(k)), op the transpose for the right
+// solves, phys reversed for modes 1 and 3.  Per 32-row block: four lanes per
+// vector substitute the diagonal block (each holds every fourth row), then
+// the blocks below subtract M(I, J) x_J on the tensor path, warp by warp a
+// 16 x 16 piece; M's blocks stream through two cp.async buffers.  One launch
+// replaces the 32-row leaves and the products between them (7 launches for
+// 128 rows); bound by the chain of substitutions at one strip per SM, by the
+// FP64 pipe beyond.  Measured with 32-row leaves -> strips: 284 right-hand
+// sides of a 284 x 284 LU (2 matrices) 612 -> 257 us, 1365 of 1365 3.54 ->
+// 1.90 ms, 2884 of 2884 13.2 -> 9.3 ms.
+// Mode 0 can apply the row interchanges of an LU panel to its columns first
+// (the panel's rows are the block's), which saves their launch and one pass
+// over the block's rows; strips of columns < jsolve are only interchanged.
+// ---------------------------------------------------------------------------
+constexpr int SN = 128, SV = 32, STHREADS = 128;
+constexpr int SST = SV + 2;    // row stride in shared memory (bank groups, see zgemm_kernel)
+
+struct StripArgs {
+    int mode, kb;              // triangle rows
+    const cd *T;
+    int64_t ldt, sT;
+    cd *B;                     // modes 0, 1: kb x nvec; modes 2, 3: nvec x kb
+    int64_t ldb, sB;
+    int nvec;
+    // interchanges (mode 0): pivots of the block's rows, absolute from `base`;
+    // vectors [0, jsolve) are interchanged only; [skip0, skip1) are left out
+    const int32_t *ipiv;
+    int64_t sP;
+    int base, jsolve, skip0, skip1;
+};
+
+__global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
+    extern __shared__ __align__(16) cd strip_sm[];
+    cd *X = strip_sm;                          // [SN][SST], rows in solve order
+    cd *M = strip_sm + SN * SST;               // [2][32][SST]: M(l, k) at [k][l]
+    __shared__ cd dinv[32];
+    __shared__ Swaps sw;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int kb = g.kb, mode = g.mode;
+    const bool fwd = mode == 0 || mode == 2, left = mode < 2, unit = mode == 0 || mode == 3;
+    const int64_t b = blockIdx.y;
+    const cd *T = g.T + b * g.sT;
+    cd *B = g.B + b * g.sB;
+    int v0 = blockIdx.x * SV;
+    int vend = g.nvec;
+    bool solve = true;
+    if (g.ipiv) {
+        // strips cover [0, skip0), then [skip1, nvec)
+        const int ns = (g.skip0 + SV - 1) / SV;
+        if ((int)blockIdx.x < ns) vend = g.skip0;
+        else v0 = g.skip1 + (blockIdx.x - ns) * SV;
+        solve = v0 >= g.jsolve;
+    }
+    const int nv = min(SV, vend - v0);
+    auto phys = [&](int l) { return fwd ? l : kb - 1 - l; };
+    const int nblk = (kb + 31) / 32;
+    // M block (I, J) into buffer q
+    auto stage = [&](int I, int J, int q) {
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(M + q * 32 * SST);
 #pragma unroll
-    for (int e = 0; e < TS; ++e)
-        x[e] = (e < kb) ? (left ? B[(int64_t)v * ldb + e] : B[(int64_t)e * ldb + v]) : cmk(0, 0);
-    if (mode == 0) {
-#pragma unroll
-        for (int r = 1; r < TS; ++r)
-#pragma unroll
-            for (int c = 0; c < r; ++c) x[r] = cfms(Ts[r][c], x[c], x[r]);
-    } else if (mode == 1) {
-#pragma unroll
-        for (int r = TS - 1; r >= 0; --r) {
-#pragma unroll
-            for (int c = r + 1; c < TS; ++c) x[r] = cfms(Ts[r][c], x[c], x[r]);
-            x[r] = cdiv(x[r], Ts[r][r]);
+        for (int e = tid; e < 1024; e += STHREADS) {
+            // consecutive threads along the contiguous direction of T
+            const int u = e & 31, w = e >> 5;
+            const int l = left ? u : w, k = left ? w : u;
+            const int gl = 32 * I + l, gk = 32 * J + k;
+            const bool ok = gl < kb && gk < kb;
+            const int64_t o = !ok ? 0
+                              : left ? (int64_t)phys(gk) * g.ldt + phys(gl)
+                                     : (int64_t)phys(gl) * g.ldt + phys(gk);
+            cp16(d + (k * SST + l) * 16, T + o, ok);
         }
-    } else if (mode == 2) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (solve) stage(0, 0, 0);
+    if (g.ipiv) {
+        const int32_t *pv = g.ipiv + b * g.sP;
+        swaps_compose(sw, pv, g.base, kb);
+        // gather the block's rows, then the rows below that the steps reached
+        for (int e = tid; e < kb * nv; e += STHREADS) {
+            const int c = e % kb, v = e / kb;
+            X[c * SST + v] = B[(int64_t)(v0 + v) * g.ldb + sw.out[c]];
+        }
+        cd t[SN * SV / STHREADS];
 #pragma unroll
-        for (int c = 0; c < TS; ++c) {
+        for (int q = 0; q < SN * SV / STHREADS; ++q) {
+            const int e = tid + q * STHREADS, c = e % kb, v = e / kb;
+            t[q] = (v < nv && sw.tail[c] >= 0) ? B[(int64_t)(v0 + v) * g.ldb + sw.tail[c]]
+                                                : cmk(0.0, 0.0);
+        }
+        __syncthreads();
 #pragma unroll
-            for (int r = 0; r < c; ++r) x[c] = cfms(x[r], Ts[r][c], x[c]);
-            x[c] = cdiv(x[c], Ts[c][c]);
+        for (int q = 0; q < SN * SV / STHREADS; ++q) {
+            const int e = tid + q * STHREADS, c = e % kb, v = e / kb;
+            if (v < nv && sw.tail[c] >= 0) B[(int64_t)(v0 + v) * g.ldb + sw.p[c]] = t[q];
+        }
+        if (!solve) {
+            for (int e = tid; e < kb * nv; e += STHREADS) {
+                const int c = e % kb, v = e / kb;
+                B[(int64_t)(v0 + v) * g.ldb + c] = X[c * SST + v];
+            }
+            return;
         }
     } else {
-#pragma unroll
-        for (int c = TS - 1; c >= 0; --c)
-#pragma unroll
-            for (int r = c + 1; r < TS; ++r) x[c] = cfms(x[r], Ts[r][c], x[c]);
-    }
-#pragma unroll
-    for (int e = 0; e < TS; ++e)
-        if (e < kb) {
-            if (left) B[(int64_t)v * ldb + e] = x[e];
-            else B[(int64_t)e * ldb + v] = x[e];
+        for (int e = tid; e < kb * nv; e += STHREADS) {
+            const int c = left ? e % kb : e / nv, v = left ? e / kb : e % nv;
+            X[(fwd ? c : kb - 1 - c) * SST + v] =
+                left ? B[(int64_t)(v0 + v) * g.ldb + c] : B[(int64_t)c * g.ldb + v0 + v];
         }
+    }
+    // rows past kb and vectors past nv stay finite: zero
+    for (int e = tid; e < nblk * 32 * SV; e += STHREADS) {
+        const int l = e / SV, v = e % SV;
+        if (l >= kb || v >= nv) X[l * SST + v] = cmk(0.0, 0.0);
+    }
+    int q = 0;
+    for (int J = 0; J < nblk; ++J) {
+        for (int I = J; I < nblk; ++I) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                   // block (I, J) staged; X rows of the last step
+            const cd *m = M + q * 32 * SST;
+            q ^= 1;
+            // the other buffer was last read before this barrier
+            if (I + 1 < nblk) stage(I + 1, J, q);
+            else if (J + 1 < nblk) stage(J + 1, J + 1, q);
+            if (I == J) {
+                if (!unit && tid < 32)
+                    dinv[tid] = 32 * J + tid < kb ? crcp(m[tid * SST + tid]) : cmk(0.0, 0.0);
+                if (!unit) __syncthreads();
+                const int v = wid * 8 + (lane >> 2), r = lane & 3;
+                cd y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y[i] = X[(32 * J + 4 * i + r) * SST + v];
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    if (!unit && r == (c & 3)) y[c >> 2] = cmul(y[c >> 2], dinv[c]);
+                    const int src = (lane & ~3) | (c & 3);
+                    const cd x = cmk(__shfl_sync(0xffffffffu, y[c >> 2].x, src),
+                                     __shfl_sync(0xffffffffu, y[c >> 2].y, src));
+                    if (r > (c & 3)) y[c >> 2] = cfms(m[c * SST + 4 * (c >> 2) + r], x, y[c >> 2]);
+#pragma unroll
+                    for (int i = (c >> 2) + 1; i < 8; ++i)
+                        y[i] = cfms(m[c * SST + 4 * i + r], x, y[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) X[(32 * J + 4 * i + r) * SST + v] = y[i];
+            } else {
+                const int gr = lane >> 2, t = lane & 3;
+                const int rl = (wid & 1) * 16, cv = (wid >> 1) * 16;
+                double re[2][4], im[2][4];
+                cd *xo = X + (32 * I + rl) * SST + cv;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const cd w = xo[(gr + 8 * (e >> 1)) * SST + 8 * j + 2 * t + (e & 1)];
+                        re[j][e] = w.x;
+                        im[j][e] = w.y;
+                    }
+#pragma unroll
+                for (int ks = 0; ks < 32; ks += 4) {
+                    const cd a0 = m[(ks + t) * SST + rl + gr], a1 = m[(ks + t) * SST + rl + gr + 8];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const cd x = X[(32 * J + ks + t) * SST + cv + 8 * j + gr];
+                        mma_f64(re[j], -a0.x, -a1.x, x.x);
+                        mma_f64(im[j], -a0.x, -a1.x, x.y);
+                        mma_f64(re[j], a0.y, a1.y, x.y);
+                        mma_f64(im[j], -a0.y, -a1.y, x.x);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        xo[(gr + 8 * (e >> 1)) * SST + 8 * j + 2 * t + (e & 1)] =
+                            cmk(re[j][e], im[j][e]);
+            }
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < kb * nv; e += STHREADS) {
+        const int c = left ? e % kb : e / nv, v = left ? e / kb : e % nv;
+        const cd x = X[(fwd ? c : kb - 1 - c) * SST + v];
+        if (left) B[(int64_t)(v0 + v) * g.ldb + c] = x;
+        else B[(int64_t)c * g.ldb + v0 + v] = x;
+    }
 }
 
 __global__ void set_identity_kernel(cd *W, int64_t ldw, int64_t sW, int n) {
@@ -382,26 +569,32 @@ int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A,
                                 sC);
 }
 
-static int trsm_small(cudaStream_t s, int mode, int kb, const cd *T, int64_t ldt, int64_t sT,
-                      cd *B, int64_t ldb, int64_t sB, int nvec, int batch) {
-    if (nvec <= 0 || kb <= 0) return MNPB_OK;
-    dim3 grid(ceil_div(nvec, 128), batch);
-    ProfScope ps(s, PC_TRSM, 4.0 * kb * kb * (double)nvec * batch);
-    trsm_small_kernel<<<grid, 128, 0, s>>>(mode, kb, T, ldt, sT, B, ldb, sB, nvec);
-    MNPB_LAUNCH_CHECK("trsm_small_kernel");
+static int launch_strip(cudaStream_t s, const StripArgs &g, int strips, int batch) {
+    if (strips <= 0 || g.kb <= 0) return MNPB_OK;
+    const int smem = (SN + 2 * 32) * SST * (int)sizeof(cd);
+    MNPB_TRY(smem_opt_in(trsm_strip_kernel, smem, "trsm_strip_kernel"));
+    ProfScope ps(s, PC_TRSM, 4.0 * g.kb * g.kb * (double)g.nvec * batch);
+    trsm_strip_kernel<<<dim3(strips, batch), STHREADS, smem, s>>>(g);
+    MNPB_LAUNCH_CHECK("trsm_strip_kernel");
     return MNPB_OK;
+}
+
+static int trsm_strip(cudaStream_t s, int mode, int kb, const cd *T, int64_t ldt, int64_t sT,
+                      cd *B, int64_t ldb, int64_t sB, int nvec, int batch) {
+    StripArgs g{mode, kb, T, ldt, sT, B, ldb, sB, nvec, nullptr, 0, 0, 0, 0, 0};
+    return launch_strip(s, g, ceil_div(nvec, SV), batch);
 }
 
 static int split_point(int n) {
     int h = n / 2;
-    h = (h / TS) * TS;
-    return h < TS ? TS : h;
+    h = (h / SN) * SN;
+    return h < SN ? SN : h;
 }
 
 // L X = B, L unit lower n x n; B n x m.
 int trsm_llu(cudaStream_t s, int n, int m, int batch, const cd *L, int64_t ldl, int64_t sL,
              cd *B, int64_t ldb, int64_t sB) {
-    if (n <= TS) return trsm_small(s, 0, n, L, ldl, sL, B, ldb, sB, m, batch);
+    if (n <= SN) return trsm_strip(s, 0, n, L, ldl, sL, B, ldb, sB, m, batch);
     int n1 = split_point(n);
     MNPB_TRY(trsm_llu(s, n1, m, batch, L, ldl, sL, B, ldb, sB));
     MNPB_TRY(zgemm(s, n - n1, m, n1, batch, cmk(-1, 0), L + n1, ldl, sL, B, ldb, sB, cmk(1, 0),
@@ -412,7 +605,7 @@ int trsm_llu(cudaStream_t s, int n, int m, int batch, const cd *L, int64_t ldl, 
 // U X = B, U upper non-unit.
 int trsm_lun(cudaStream_t s, int n, int m, int batch, const cd *U, int64_t ldu, int64_t sU,
              cd *B, int64_t ldb, int64_t sB) {
-    if (n <= TS) return trsm_small(s, 1, n, U, ldu, sU, B, ldb, sB, m, batch);
+    if (n <= SN) return trsm_strip(s, 1, n, U, ldu, sU, B, ldb, sB, m, batch);
     int n1 = split_point(n);
     MNPB_TRY(trsm_lun(s, n - n1, m, batch, U + n1 + (int64_t)n1 * ldu, ldu, sU, B + n1, ldb, sB));
     MNPB_TRY(zgemm(s, n1, m, n - n1, batch, cmk(-1, 0), U + (int64_t)n1 * ldu, ldu, sU, B + n1,
@@ -423,7 +616,7 @@ int trsm_lun(cudaStream_t s, int n, int m, int batch, const cd *U, int64_t ldu, 
 // X U = B, U upper non-unit n x n; X, B m x n.
 int trsm_run(cudaStream_t s, int n, int m, int batch, const cd *U, int64_t ldu, int64_t sU,
              cd *B, int64_t ldb, int64_t sB) {
-    if (n <= TS) return trsm_small(s, 2, n, U, ldu, sU, B, ldb, sB, m, batch);
+    if (n <= SN) return trsm_strip(s, 2, n, U, ldu, sU, B, ldb, sB, m, batch);
     int n1 = split_point(n);
     MNPB_TRY(trsm_run(s, n1, m, batch, U, ldu, sU, B, ldb, sB));
     MNPB_TRY(zgemm(s, m, n - n1, n1, batch, cmk(-1, 0), B, ldb, sB, U + (int64_t)n1 * ldu, ldu,
@@ -435,7 +628,7 @@ int trsm_run(cudaStream_t s, int n, int m, int batch, const cd *U, int64_t ldu, 
 // X L = B, L unit lower n x n; X, B m x n.
 int trsm_rlu(cudaStream_t s, int n, int m, int batch, const cd *L, int64_t ldl, int64_t sL,
              cd *B, int64_t ldb, int64_t sB) {
-    if (n <= TS) return trsm_small(s, 3, n, L, ldl, sL, B, ldb, sB, m, batch);
+    if (n <= SN) return trsm_strip(s, 3, n, L, ldl, sL, B, ldb, sB, m, batch);
     int n1 = split_point(n);
     MNPB_TRY(trsm_rlu(s, n - n1, m, batch, L + n1 + (int64_t)n1 * ldl, ldl, sL,
                       B + (int64_t)n1 * ldb, ldb, sB));
@@ -455,17 +648,6 @@ int laswp(cudaStream_t s, cd *A, int64_t lda, int64_t sA, int ncols, int jskip0,
     return MNPB_OK;
 }
 
-// Row interchanges piv[c0..c1) applied to the columns [j0, j1) only.
-static int laswp_range(cudaStream_t s, cd *A, int64_t lda, int64_t sA, int j0, int j1,
-                       const int32_t *ipiv, int64_t sP, int c0, int c1, int batch) {
-    if (j1 <= j0 || c1 <= c0) return MNPB_OK;
-    dim3 grid(ceil_div(j1 - j0, 128), batch);
-    ProfScope ps(s, PC_SWAP, 0.0);
-    laswp_kernel<<<grid, 128, 0, s>>>(A, lda, sA, j0, j1, 0, 0, ipiv, sP, c0, c1, 1);
-    MNPB_LAUNCH_CHECK("laswp_kernel");
-    return MNPB_OK;
-}
-
 // Columns of an LU leaf over m rows: what the cluster's registers hold (32, 16
 // or 8 columns of 1, 2 or 4 rows a thread); beyond that the leaf in global
 // memory takes 32.
@@ -477,41 +659,66 @@ static int leaf_width(int m) {
     return TS;
 }
 
-// Recursive LU: factor columns [off, off+w) over rows [off, n); absolute pivots.
-static int rgetrf(cudaStream_t s, int n, int off, int w, int batch, cd *A, int64_t lda,
-                  int64_t sA, int32_t *ipiv, int64_t sP, int32_t *info) {
-    if (w <= leaf_width(n - off)) {
-        ProfScope ps(s, PC_PANEL, 8.0 * w * w * (double)(n - off) * batch / 2);
-        const lup::F64::Mat mat{A, lda, sA};
-        int C, threads;
-        if (lup::panel_shape(n - off, 1, C, threads))
-            return lup::launch_panel<lup::F64, TS, 1>(s, n, off, w, mat, ipiv, sP, info, batch, C,
-                                                      threads);
-        if (lup::panel_shape(n - off, 2, C, threads))
-            return lup::launch_panel<lup::F64, TS / 2, 2>(s, n, off, w, mat, ipiv, sP, info,
-                                                          batch, C, threads);
-        if (lup::panel_shape(n - off, 4, C, threads))
-            return lup::launch_panel<lup::F64, TS / 4, 4>(s, n, off, w, mat, ipiv, sP, info,
-                                                          batch, C, threads);
-        panel_kernel<<<batch, PANEL_THREADS, 0, s>>>(n, off, w, A, lda, sA, ipiv, sP, info);
-        MNPB_LAUNCH_CHECK("panel_kernel");
-        return MNPB_OK;
-    }
-    const int w1 = w > TS ? split_point(w) : leaf_width(n - off);
-    MNPB_TRY(rgetrf(s, n, off, w1, batch, A, lda, sA, ipiv, sP, info));
-    MNPB_TRY(laswp_range(s, A, lda, sA, off + w1, off + w, ipiv, sP, off, off + w1, batch));
-    cd *A11 = A + off + (int64_t)off * lda;
-    cd *A12 = A + off + (int64_t)(off + w1) * lda;
-    MNPB_TRY(trsm_llu(s, w1, w - w1, batch, A11, lda, sA, A12, lda, sA));
-    MNPB_TRY(zgemm(s, n - off - w1, w - w1, w1, batch, cmk(-1, 0), A11 + w1, lda, sA, A12, lda,
-                   sA, cmk(1, 0), A12 + w1, lda, sA));
-    MNPB_TRY(rgetrf(s, n, off + w1, w - w1, batch, A, lda, sA, ipiv, sP, info));
-    return laswp_range(s, A, lda, sA, off, off + w1, ipiv, sP, off + w1, off + w, batch);
+// One LU leaf: columns [off, off + w) over rows [off, n).
+static int leaf(cudaStream_t s, int n, int off, int w, int batch, cd *A, int64_t lda, int64_t sA,
+                int32_t *ipiv, int64_t sP, int32_t *info) {
+    ProfScope ps(s, PC_PANEL, 8.0 * w * w * (double)(n - off) * batch / 2);
+    const lup::F64::Mat mat{A, lda, sA};
+    int C, threads;
+    if (lup::panel_shape(n - off, 1, C, threads))
+        return lup::launch_panel<lup::F64, TS, 1>(s, n, off, w, mat, ipiv, sP, info, batch, C,
+                                                  threads);
+    if (lup::panel_shape(n - off, 2, C, threads))
+        return lup::launch_panel<lup::F64, TS / 2, 2>(s, n, off, w, mat, ipiv, sP, info, batch,
+                                                      C, threads);
+    if (lup::panel_shape(n - off, 4, C, threads))
+        return lup::launch_panel<lup::F64, TS / 4, 4>(s, n, off, w, mat, ipiv, sP, info, batch,
+                                                      C, threads);
+    panel_kernel<<<batch, PANEL_THREADS, 0, s>>>(n, off, w, A, lda, sA, ipiv, sP, info);
+    MNPB_LAUNCH_CHECK("panel_kernel");
+    return MNPB_OK;
 }
 
+// Interchanges of the pivots of columns [off, off + w) on the columns
+// [j0, j1) without the pivots' own, and L^-1 on the rows [off, off + w) of
+// those right of them.
+static int swap_solve(cudaStream_t s, int off, int w, int j0, int j1, int batch, cd *A,
+                      int64_t lda, int64_t sA, const int32_t *ipiv, int64_t sP) {
+    const int skip0 = off - j0, skip1 = off + w - j0, nvec = j1 - j0;
+    StripArgs g{0,    w,         A + off + (int64_t)off * lda, lda, sA,
+                A + off + (int64_t)j0 * lda, lda, sA, nvec,
+                ipiv + off, sP, off, skip1, skip0, skip1};
+    return launch_strip(s, g, ceil_div(skip0, SV) + ceil_div(nvec - skip1, SV), batch);
+}
+
+// Right-looking LU in blocks of SN columns; inside a block, leaf by leaf.  A
+// block costs its leaves, two launches per leaf inside the block, and two for
+// the rest of the matrix, where halving the columns recursively took some 40
+// per 128 columns: at one matrix the launches outnumber what they do.  The
+// update's depth of 128 already runs at the GEMM's full rate.  One matrix of
+// 2884: 17.6 -> 11.2 ms, 1365 6.1 -> 4.0 ms, 284 0.79 -> 0.63 ms (with the
+// panels' reductions by redux.sync); 41 of 1148 14.5 -> 11.0 ms.
 int getrf(cudaStream_t s, int n, int batch, cd *A, int64_t lda, int64_t sA, int32_t *ipiv,
           int64_t sP, int32_t *info) {
-    return rgetrf(s, n, 0, n, batch, A, lda, sA, ipiv, sP, info);
+    for (int j0 = 0; j0 < n; j0 += SN) {
+        const int j1 = min(n, j0 + SN);
+        for (int off = j0; off < j1;) {
+            const int w = min(leaf_width(n - off), j1 - off), c1 = off + w;
+            MNPB_TRY(leaf(s, n, off, w, batch, A, lda, sA, ipiv, sP, info));
+            if (j1 - j0 > w)
+                MNPB_TRY(swap_solve(s, off, w, j0, j1, batch, A, lda, sA, ipiv, sP));
+            MNPB_TRY(zgemm(s, n - c1, j1 - c1, w, batch, cmk(-1, 0), A + c1 + (int64_t)off * lda,
+                           lda, sA, A + off + (int64_t)c1 * lda, lda, sA, cmk(1, 0),
+                           A + c1 + (int64_t)c1 * lda, lda, sA));
+            off = c1;
+        }
+        if (n == j1 && j0 == 0) break;
+        MNPB_TRY(swap_solve(s, j0, j1 - j0, 0, n, batch, A, lda, sA, ipiv, sP));
+        MNPB_TRY(zgemm(s, n - j1, n - j1, j1 - j0, batch, cmk(-1, 0), A + j1 + (int64_t)j0 * lda,
+                       lda, sA, A + j0 + (int64_t)j1 * lda, lda, sA, cmk(1, 0),
+                       A + j1 + (int64_t)j1 * lda, lda, sA));
+    }
+    return MNPB_OK;
 }
 
 int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda, int64_t sA,

@@ -23,8 +23,9 @@
 // Measured (FP64 LU of one n x n matrix, all else equal) against the leaf it
 // replaces, one CTA per matrix working in global memory: n = 284 1.44 -> 0.94
 // ms, 1365 16.0 -> 7.5, 2884 63.7 -> 22.0, 7000 348 -> 106; 41 matrices of
-// 1148 23.1 -> 16.9.  A pivot step takes 1.4 us in one CTA and 2.1 us in a
-// cluster of 8.
+// 1148 23.1 -> 16.9.  A pivot step takes 1.1 us in one CTA and 1.8 us in a
+// cluster of 8 (1.4 and 2.1 before the reductions were redux.sync on the bit
+// patterns instead of shuffles of the values).
 #pragma once
 #include "common.cuh"
 
@@ -63,7 +64,15 @@ struct F64 {
         m.A[b * m.sA + col * m.lda + row] = v;
     }
     static __device__ __forceinline__ S mag(V v) { return cabs1(v); }
-    static __device__ __forceinline__ V rcp(V v) { return crcp(v); }
+    // one division where the squares can neither overflow nor underflow
+    static __device__ __forceinline__ V rcp(V v) {
+        const double m = fmax(fabs(v.x), fabs(v.y));
+        if (m > 1e-100 && m < 1e100) {
+            const double i = 1.0 / (v.x * v.x + v.y * v.y);
+            return cmk(v.x * i, -v.y * i);
+        }
+        return crcp(v);
+    }
     static __device__ __forceinline__ V mul(V a, V b) { return cmul(a, b); }
     static __device__ __forceinline__ V fms(V a, V b, V c) { return cfms(a, b, c); }
     static __device__ __forceinline__ V rnd(V v) { return v; }   // storage precision of L and U
@@ -80,11 +89,20 @@ constexpr int MAXC = 8;          // CTAs per cluster (portable limit)
 constexpr int MAXW = 12;         // warps per CTA
 constexpr int NOROW = 0x7fffffff;
 
-// larger magnitude first, then the smaller row position (the first row of the
-// maximal |re| + |im| in the interchanged order)
-template <typename S>
-__device__ __forceinline__ bool better(S v, int p, S bv, int bp) {
-    return v > bv || (v == bv && p < bp);
+// Best (magnitude, position) of a warp: larger magnitude (>= 0), then smaller
+// position.  The bit pattern of a non-negative number orders as an integer, so
+// the reductions are redux.sync on 32-bit words.
+__device__ __forceinline__ void warp_best(double &v, int &p) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    p = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? p : NOROW);
+    v = __hiloint2double((int)mh, (int)ml);
+}
+__device__ __forceinline__ void warp_best(float &v, int &p) {
+    const unsigned k = __float_as_uint(v), m = __reduce_max_sync(0xffffffffu, k);
+    p = __reduce_min_sync(0xffffffffu, k == m ? p : NOROW);
+    v = __uint_as_float(m);
 }
 
 template <typename T, int W, int R>
@@ -119,35 +137,24 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
         if (jj < kb) {
             const int buf = jj & 1;
             // best of this thread's active rows, then of the warp, then of the CTA
-            S bv = (S)-1;
+            S bv = (S)0;
             int bp = NOROW;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const S t = T::mag(a[r][jj]);
                 const S v = t > (S)0 ? t : (S)0;       // NaN counts as zero
-                if (pos[r] != NOROW && pos[r] >= jj && better(v, pos[r], bv, bp)) {
+                if (pos[r] != NOROW && pos[r] >= jj &&
+                    (v > bv || (v == bv && pos[r] < bp))) {
                     bv = v;
                     bp = pos[r];
                 }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-                if (better(ov, op, bv, bp)) { bv = ov; bp = op; }
-            }
+            warp_best(bv, bp);
             if (lane == 0) { red_v[buf][wid] = bv; red_p[buf][wid] = bp; }
             __syncthreads();
-            bv = lane < nw ? red_v[buf][lane] : (S)-1;
+            bv = lane < nw ? red_v[buf][lane] : (S)0;
             bp = lane < nw ? red_p[buf][lane] : NOROW;
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) {
-                const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-                if (better(ov, op, bv, bp)) { bv = ov; bp = op; }
-            }
-            bv = __shfl_sync(0xffffffffu, bv, 0);
-            bp = __shfl_sync(0xffffffffu, bp, 0);
+            warp_best(bv, bp);
             // the warp that holds the CTA's best row publishes it
             bool mine = false;
 #pragma unroll
@@ -182,19 +189,11 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
             }
             int win = 0;
             if (C > 1) {
-                bv = lane < C ? cand_v[buf][lane] : (S)-1;
-                bp = lane < C ? cand_p[buf][lane] : NOROW;
-                win = lane;
-#pragma unroll
-                for (int o = MAXC / 2; o > 0; o >>= 1) {
-                    const S ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                    const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-                    const int ow = __shfl_xor_sync(0xffffffffu, win, o);
-                    if (better(ov, op, bv, bp)) { bv = ov; bp = op; win = ow; }
-                }
-                bv = __shfl_sync(0xffffffffu, bv, 0);
-                bp = __shfl_sync(0xffffffffu, bp, 0);
-                win = __shfl_sync(0xffffffffu, win, 0);
+                bv = lane < C ? cand_v[buf][lane] : (S)0;
+                const int own = lane < C ? cand_p[buf][lane] : NOROW;
+                bp = own;
+                warp_best(bv, bp);
+                win = __ffs(__ballot_sync(0xffffffffu, own == bp)) - 1;
             }
             if (me == 0 && tid == 0) {
                 ipiv[b * sP + k0 + jj] = k0 + bp;

@@ -1,6 +1,7 @@
 """FP64 dense building blocks at the sizes where their kernels change: LU
 panels (rows per CTA, CTAs per cluster, columns per leaf, remainders) and
-matrix products (tile edges, depth remainders, strides)."""
+matrix products (tile edges, depth remainders, strides), solves (few and many
+right-hand sides, interchange chains)."""
 import numpy as np
 import pytest
 import scipy.linalg as sla
@@ -105,3 +106,47 @@ def test_zgemm_tiles(gpu_ok, m, n, k, batch, alpha, beta):
     got = C[:, :n, :m].transpose(1, 2)
     assert bool(((got - ref).abs() <= bound).all())
     assert torch.equal(C[:, n:], C0[:, n:]) and torch.equal(C[:, :, m:], C0[:, :, m:])
+
+
+@pytest.mark.parametrize('n,nrhs,batch', [(1, 1, 2), (5, 2, 1), (63, 4, 1), (64, 1, 3),
+                                          (65, 5, 2), (130, 16, 1), (300, 3, 80), (700, 1, 1),
+                                          (700, 7, 1), (129, 17, 2), (200, 33, 1),
+                                          (385, 385, 2), (1100, 100, 1), (4500, 2, 1),
+                                          (5100, 1, 1)])
+def test_getrs_few_and_many(gpu_ok, n, nrhs, batch):
+    """|A x - b| <= 12 n eps |L| |U| |x| + |b| eps (backward error of the LU solve)."""
+    A = _rand(batch, n, n, seed=n + 1)
+    LU, piv, _ = _getrf(A)
+    ldb = n + 2
+    B0 = _rand(batch, nrhs + 1, ldb, seed=2)
+    X = B0.clone()
+    call('mnpb_getrs_f64', _lib.stream_handle(), n, batch, nrhs, ptr(LU), n, n * n, ptr(piv), n,
+         ptr(X), ldb, (nrhs + 1) * ldb)
+    assert torch.equal(X[:, nrhs:], B0[:, nrhs:]) and torch.equal(X[:, :, n:], B0[:, :, n:])
+    x, b = X[:, :nrhs, :n].transpose(1, 2), B0[:, :nrhs, :n].transpose(1, 2)
+    F = LU.transpose(1, 2)
+    L = torch.tril(F, -1).abs()
+    L.diagonal(dim1=1, dim2=2).fill_(1.0)
+    mag = L @ (torch.triu(F).abs() @ x.abs())
+    # row interchanges permute the bound's rows: compare with each column's largest
+    res = (A.transpose(1, 2) @ x - b).abs().amax(1)
+    assert bool((res <= 12 * n * EPS * mag.amax(1) + 4 * EPS * b.abs().amax(1)).all())
+
+
+def test_getrs_interchange_chains(gpu_ok):
+    # pivots whose targets repeat and chain: every step targets the last row, or
+    # the row after next, or itself
+    n = 300
+    A = torch.eye(n, dtype=torch.complex128, device='cuda')
+    for p in (np.full(n, n - 1), np.minimum(np.arange(n) + 2, n - 1), np.arange(n),
+              np.where(np.arange(n) % 3 == 0, n - 1, np.minimum(np.arange(n) + 5, n - 1))):
+        piv = torch.from_numpy(p.astype(np.int32)).cuda()[None]
+        for nrhs in (1, 20):
+            X = torch.arange(n, dtype=torch.float64, device='cuda').to(torch.complex128) \
+                .repeat(nrhs, 1)
+            call('mnpb_getrs_f64', _lib.stream_handle(), n, 1, nrhs, ptr(A), n, n * n, ptr(piv),
+                 n, ptr(X), n, n * nrhs)
+            want = np.arange(n)
+            for c, r in enumerate(p):
+                want[[c, r]] = want[[r, c]]
+            assert np.array_equal(X.real.cpu().numpy(), np.tile(want, (nrhs, 1)))
