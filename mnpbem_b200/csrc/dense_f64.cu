@@ -8,6 +8,8 @@
 #include "common.cuh"
 #include "dense_f64.cuh"
 #include "lu_panel.cuh"
+#include "trsv_cluster.cuh"
+#include "skinny.cuh"
 
 namespace mnpb {
 
@@ -253,6 +255,26 @@ __global__ void laswp_kernel(cd *A, int64_t lda, int64_t sA, int j0, int j1, int
             int p = pv[c];
             if (p != c) { cd t = col[c]; col[c] = col[p]; col[p] = t; }
         }
+    }
+}
+
+// Row interchanges of whole columns (all n steps) composed once per CTA, then
+// column by column through shared memory: reads and writes are coalesced and
+// independent, where laswp_kernel walks n dependent steps per column.
+__global__ void __launch_bounds__(512) permute_rows_kernel(cd *A, int64_t lda, int64_t sA, int n,
+                                                           int ncols, const int32_t *ipiv,
+                                                           int64_t sP) {
+    extern __shared__ __align__(16) int perm_sm[];
+    cd *col = (cd *)perm_sm;
+    int *w = perm_sm + 4 * n;
+    const int64_t b = blockIdx.y;
+    trc::compose(w, ipiv + b * sP, n);
+    for (int j = blockIdx.x; j < ncols; j += gridDim.x) {
+        cd *a = A + b * sA + (int64_t)j * lda;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) col[i] = a[i];
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = col[w[i]];
+        __syncthreads();
     }
 }
 
@@ -557,6 +579,9 @@ int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A,
     // (2800 x 32 x 32, 2 matrices: 20.7 -> 14.6 us; 2884 x 4 x 2884, which a
     // 64-column tile padded 16-fold: 795 -> 157 us)
     const int kk = k > 0 ? k : 0;
+    if (n <= 16 && kk > 0)
+        return skn::run<skn::F64>(s, m, n, kk, batch, alpha, {(cd *)A, lda, sA},
+                                  {(cd *)B, ldb, sB}, beta, {C, ldc, sC});
     const int64_t t64 = (int64_t)ceil_div(m, 64) * ceil_div(n, 64) * batch;
     const int64_t t32 = (int64_t)ceil_div(m, 64) * ceil_div(n, 32) * batch;
     if (t64 >= 2 * device_sms() && n > 32)
@@ -640,8 +665,8 @@ int trsm_rlu(cudaStream_t s, int n, int m, int batch, const cd *L, int64_t ldl, 
 int laswp(cudaStream_t s, cd *A, int64_t lda, int64_t sA, int ncols, int jskip0, int jskip1,
           const int32_t *ipiv, int64_t sP, int c0, int c1, bool forward, int batch) {
     if (ncols <= 0 || c1 <= c0) return MNPB_OK;
-    dim3 grid(ceil_div(ncols, 128), batch);
     ProfScope ps(s, PC_SWAP, 0.0);
+    dim3 grid(ceil_div(ncols, 128), batch);
     laswp_kernel<<<grid, 128, 0, s>>>(A, lda, sA, 0, ncols, jskip0, jskip1, ipiv, sP, c0, c1,
                                       forward ? 1 : 0);
     MNPB_LAUNCH_CHECK("laswp_kernel");
@@ -721,9 +746,48 @@ int getrf(cudaStream_t s, int n, int batch, cd *A, int64_t lda, int64_t sA, int3
     return MNPB_OK;
 }
 
+// All n interchanges of an LU on the rows of B.
+static int permute_rows(cudaStream_t s, cd *B, int64_t ldb, int64_t sB, int n, int ncols,
+                        const int32_t *ipiv, int64_t sP, int batch) {
+    const int64_t smem = 32 * (int64_t)n;          // a column and 4 n ints
+    if (smem > 200 * 1024)
+        return laswp(s, B, ldb, sB, ncols, 0, 0, ipiv, sP, 0, n, true, batch);
+    MNPB_TRY(smem_opt_in(permute_rows_kernel, 200 * 1024, "permute_rows_kernel"));
+    ProfScope ps(s, PC_SWAP, 0.0);
+    const int per = max(1, 4 * device_sms() / batch);
+    permute_rows_kernel<<<dim3(min(ncols, per), batch), 512, (size_t)smem, s>>>(B, ldb, sB, n,
+                                                                              ncols, ipiv, sP);
+    MNPB_LAUNCH_CHECK("permute_rows_kernel");
+    return MNPB_OK;
+}
+
+// Forward then backward solve of up to 16 right-hand sides, a cluster per
+// matrix and NC columns; the interchanges ride along with the forward solve.
+template <int NC>
+static int getrs_few(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda,
+                     int64_t sA, const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB,
+                     int C) {
+    const trc::F64::Mat A{(cd *)LU, lda, sA}, X{B, ldb, sB};
+    const bool ride = trc::Smem<trc::F64, NC>::composes(n);
+    if (!ride) MNPB_TRY(laswp(s, B, ldb, sB, nrhs, 0, 0, ipiv, sP, 0, n, true, batch));
+    ProfScope ps(s, PC_TRSV, 16.0 * (double)n * n * batch);   // bytes of both triangles
+    MNPB_TRY((trc::launch_trsv<trc::F64, NC>(s, true, true, n, nrhs, batch, A, nullptr, X,
+                                             ride ? ipiv : nullptr, sP, C)));
+    return trc::launch_trsv<trc::F64, NC>(s, false, false, n, nrhs, batch, A, nullptr, X, nullptr,
+                                          0, C);
+}
+
 int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda, int64_t sA,
           const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB) {
-    MNPB_TRY(laswp(s, B, ldb, sB, nrhs, 0, 0, ipiv, sP, 0, n, true, batch));
+    if (nrhs <= 16) {
+        const int C1 = trc::cluster_size<trc::F64, 1>(n, batch);
+        const int C4 = trc::cluster_size<trc::F64, 4>(n, (int64_t)batch * ceil_div(nrhs, 4));
+        if (nrhs == 1 && C1 > 0)
+            return getrs_few<1>(s, n, nrhs, batch, LU, lda, sA, ipiv, sP, B, ldb, sB, C1);
+        if (nrhs > 1 && C4 > 0)
+            return getrs_few<4>(s, n, nrhs, batch, LU, lda, sA, ipiv, sP, B, ldb, sB, C4);
+    }
+    MNPB_TRY(permute_rows(s, B, ldb, sB, n, nrhs, ipiv, sP, batch));
     MNPB_TRY(trsm_llu(s, n, nrhs, batch, LU, lda, sA, B, ldb, sB));
     return trsm_lun(s, n, nrhs, batch, LU, lda, sA, B, ldb, sB);
 }

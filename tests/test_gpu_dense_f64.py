@@ -87,6 +87,8 @@ def test_lu_ties_and_zero_columns(gpu_ok, n):
 
 @pytest.mark.parametrize('m,n,k,batch', [(1, 1, 1, 1), (33, 31, 7, 2), (32, 32, 8, 1),
                                          (64, 4, 33, 3), (65, 65, 25, 1), (700, 33, 40, 5),
+                                         (63, 1, 200, 2), (129, 5, 513, 1), (64, 12, 64, 400),
+                                         (1000, 16, 2900, 1), (2500, 13, 130, 3),
                                          (640, 70, 9, 40), (1300, 1290, 64, 1), (50, 40, 0, 2)])
 @pytest.mark.parametrize('alpha,beta', [(-1.0, 1.0), (0.5 - 2.0j, 0.0), (1.0j, -0.25 + 1.0j)])
 def test_zgemm_tiles(gpu_ok, m, n, k, batch, alpha, beta):
