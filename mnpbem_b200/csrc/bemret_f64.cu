@@ -69,8 +69,7 @@ extern "C" int mnpb_bemret_init_f64(void *stream, int64_t n, int64_t batch, doub
     form_delta_kernel<<<grid, 128, 0, s>>>(N, h1, h2, d, ld, stride, eps, kvac);
     MNPB_LAUNCH_CHECK("form_delta_kernel");
     MNPB_TRY(getrf(s, N, B, d, ld, stride, pivD, n, info));
-    MNPB_TRY(set_identity(s, N, B, W, n, sw));
-    MNPB_TRY(getrs(s, N, N, B, d, ld, stride, pivD, n, W, n, sw));
+    MNPB_TRY(getri(s, N, B, d, ld, stride, pivD, n, W, n, sw));
     form_sigma_kernel<<<grid, 128, 0, s>>>(N, h2, W, n, sw, d, ld, stride, eps, kvac,
                                            NvecView{nvec, nvec_stride});
     MNPB_LAUNCH_CHECK("form_sigma_kernel");

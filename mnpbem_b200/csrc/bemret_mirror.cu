@@ -148,9 +148,7 @@ extern "C" int mnpb_bemret_init_mirror_f64(void *stream, int64_t n, int64_t entr
     mirror_delta_kernel<<<grid, 128, 0, s>>>(N, h1, h2, D, ld, stride, n, sd);
     MNPB_LAUNCH_CHECK("mirror_delta_kernel");
     MNPB_TRY(getrf(s, N, E, D, n, sd, pivD, ps, info + 2 * entries));
-    MNPB_TRY(set_identity(s, N, E, di, ld, stride));
-    MNPB_TRY(getrs(s, N, N, E, D, n, sd, pivD, ps, di, ld, stride));
-    return MNPB_OK;
+    return getri(s, N, E, D, n, sd, pivD, ps, di, ld, stride);
 }
 
 extern "C" int mnpb_bemret_sigma_mirror_f64(void *stream, int64_t n, int64_t nsym, int64_t batch,

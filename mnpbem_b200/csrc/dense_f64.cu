@@ -278,6 +278,33 @@ __global__ void __launch_bounds__(512) permute_rows_kernel(cd *A, int64_t lda, i
     }
 }
 
+// X <- X P: the interchanges' columns c and ipiv[c], c from n - 1 down to 0, on
+// RS rows per CTA through shared memory.  The reverse order undoes the forward
+// gather (row c <- src[c]), so column c goes to column src[c].
+__global__ void __launch_bounds__(256) permute_cols_kernel(cd *X, int64_t ldx, int64_t sX, int m,
+                                                           const int32_t *ipiv, int64_t sP,
+                                                           int n, int RS) {
+    extern __shared__ __align__(16) int perm_sm[];
+    cd *buf = (cd *)perm_sm;                   // [n][RS]
+    int *w = perm_sm + 4 * (int64_t)n * RS;
+    const int64_t b = blockIdx.y;
+    const int r0 = blockIdx.x * RS, nr = min(RS, m - r0);
+    cd *x = X + b * sX + r0;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(buf);
+    for (int e = threadIdx.x; e < n * RS; e += blockDim.x) {
+        const int r = e % RS, c = e / RS;
+        cp16(d + e * 16, r < nr ? x + (int64_t)c * ldx + r : x, r < nr);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    trc::compose(w, ipiv + b * sP, n);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * RS; e += blockDim.x) {
+        const int r = e % RS, c = e / RS;
+        if (r < nr && w[c] != c) x[(int64_t)w[c] * ldx + r] = buf[e];
+    }
+}
+
 // Column interchanges of X (rows [0, m)), c from n-1 down to 0: X <- X P.
 __global__ void colswp_kernel(cd *X, int64_t ldx, int64_t sX, int m, const int32_t *ipiv,
                               int64_t sP, int n) {
@@ -348,7 +375,8 @@ __device__ __forceinline__ void swaps_compose(Swaps &w, const int32_t *ipiv, int
 
 // ---------------------------------------------------------------------------
 // Triangular solves on a diagonal block of up to SN = 128 rows, one CTA per
-// strip of SV = 32 right-hand sides held in shared memory.
+// strip of SV right-hand sides (32, or 16 while those strips are too few to
+// give every SM one) held in shared memory.
 // mode 0: left lower unit     L x = b   (vectors: columns of B)
 // mode 1: left upper non-unit U x = b   (vectors: columns of B)
 // mode 2: right upper non-unit x U = b  (vectors: rows of B)
@@ -356,7 +384,7 @@ __device__ __forceinline__ void swaps_compose(Swaps &w, const int32_t *ipiv, int
 // All four are one forward substitution with the triangle in the order of the
 // solve: M(l, k) = op(T)(phys(l), phys(k)), op the transpose for the right
 // solves, phys reversed for modes 1 and 3.  Per 32-row block: four lanes per
-// vector substitute the diagonal block (each holds every fourth row), then
+// vector (eight for 16) substitute the diagonal block, each with its own rows, then
 // the blocks below subtract M(I, J) x_J on the tensor path, warp by warp a
 // 16 x 16 piece; M's blocks stream through two cp.async buffers.  One launch
 // replaces the 32-row leaves and the products between them (7 launches for
@@ -368,8 +396,8 @@ __device__ __forceinline__ void swaps_compose(Swaps &w, const int32_t *ipiv, int
 // (the panel's rows are the block's), which saves their launch and one pass
 // over the block's rows; strips of columns < jsolve are only interchanged.
 // ---------------------------------------------------------------------------
-constexpr int SN = 128, SV = 32, STHREADS = 128;
-constexpr int SST = SV + 2;    // row stride in shared memory (bank groups, see zgemm_kernel)
+constexpr int SN = 128, STHREADS = 128;
+constexpr int MST = 34;        // M's stride in shared memory (bank groups, see zgemm_kernel)
 
 struct StripArgs {
     int mode, kb;              // triangle rows
@@ -385,10 +413,14 @@ struct StripArgs {
     int base, jsolve, skip0, skip1;
 };
 
+template <int SV>
 __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
+    constexpr int SST = SV + 2;                // X's stride
+    constexpr int LV = STHREADS / SV, RL = 32 / LV;   // lanes per vector, rows per lane
+    constexpr int NJ = SV / 16;                // 8-column fragments per warp
     extern __shared__ __align__(16) cd strip_sm[];
     cd *X = strip_sm;                          // [SN][SST], rows in solve order
-    cd *M = strip_sm + SN * SST;               // [2][32][SST]: M(l, k) at [k][l]
+    cd *M = strip_sm + SN * SST;               // [2][32][MST]: M(l, k) at [k][l]
     __shared__ cd dinv[32];
     __shared__ Swaps sw;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -412,7 +444,7 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
     const int nblk = (kb + 31) / 32;
     // M block (I, J) into buffer q
     auto stage = [&](int I, int J, int q) {
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(M + q * 32 * SST);
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(M + q * 32 * MST);
 #pragma unroll
         for (int e = tid; e < 1024; e += STHREADS) {
             // consecutive threads along the contiguous direction of T
@@ -423,31 +455,38 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
             const int64_t o = !ok ? 0
                               : left ? (int64_t)phys(gk) * g.ldt + phys(gl)
                                      : (int64_t)phys(gl) * g.ldt + phys(gk);
-            cp16(d + (k * SST + l) * 16, T + o, ok);
+            cp16(d + (k * MST + l) * 16, T + o, ok);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    const uint32_t xs = (uint32_t)__cvta_generic_to_shared(X);
     if (solve) stage(0, 0, 0);
     if (g.ipiv) {
         const int32_t *pv = g.ipiv + b * g.sP;
         swaps_compose(sw, pv, g.base, kb);
-        // gather the block's rows, then the rows below that the steps reached
-        for (int e = tid; e < kb * nv; e += STHREADS) {
-            const int c = e % kb, v = e / kb;
-            X[c * SST + v] = B[(int64_t)(v0 + v) * g.ldb + sw.out[c]];
+        // gather the block's rows, and the rows below that the steps reached;
+        // rows past kb and vectors past nv are zero
+        for (int e = tid; e < nblk * 32 * SV; e += STHREADS) {
+            const int c = e % (nblk * 32), v = e / (nblk * 32);
+            const bool ok = c < kb && v < nv;
+            cp16(xs + (c * SST + v) * 16, ok ? B + (int64_t)(v0 + v) * g.ldb + sw.out[c] : B, ok);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
         cd t[SN * SV / STHREADS];
 #pragma unroll
         for (int q = 0; q < SN * SV / STHREADS; ++q) {
-            const int e = tid + q * STHREADS, c = e % kb, v = e / kb;
-            t[q] = (v < nv && sw.tail[c] >= 0) ? B[(int64_t)(v0 + v) * g.ldb + sw.tail[c]]
-                                                : cmk(0.0, 0.0);
+            const int e = tid + q * STHREADS, c = e % SN, v = e / SN;
+            t[q] = (v < nv && c < kb && sw.tail[c] >= 0)
+                       ? B[(int64_t)(v0 + v) * g.ldb + sw.tail[c]]
+                       : cmk(0.0, 0.0);
         }
-        __syncthreads();
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                       // every row read: B may be written
 #pragma unroll
         for (int q = 0; q < SN * SV / STHREADS; ++q) {
-            const int e = tid + q * STHREADS, c = e % kb, v = e / kb;
-            if (v < nv && sw.tail[c] >= 0) B[(int64_t)(v0 + v) * g.ldb + sw.p[c]] = t[q];
+            const int e = tid + q * STHREADS, c = e % SN, v = e / SN;
+            if (v < nv && c < kb && sw.tail[c] >= 0)
+                B[(int64_t)(v0 + v) * g.ldb + sw.p[c]] = t[q];
         }
         if (!solve) {
             for (int e = tid; e < kb * nv; e += STHREADS) {
@@ -457,55 +496,55 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
             return;
         }
     } else {
-        for (int e = tid; e < kb * nv; e += STHREADS) {
-            const int c = left ? e % kb : e / nv, v = left ? e / kb : e % nv;
-            X[(fwd ? c : kb - 1 - c) * SST + v] =
-                left ? B[(int64_t)(v0 + v) * g.ldb + c] : B[(int64_t)c * g.ldb + v0 + v];
+        for (int e = tid; e < nblk * 32 * SV; e += STHREADS) {
+            const int l = left ? e % (nblk * 32) : e / SV, v = left ? e / (nblk * 32) : e % SV;
+            const bool ok = l < kb && v < nv;
+            const cd *src = !ok    ? B
+                            : left ? B + (int64_t)(v0 + v) * g.ldb + phys(l)
+                                   : B + (int64_t)phys(l) * g.ldb + v0 + v;
+            cp16(xs + (l * SST + v) * 16, src, ok);
         }
-    }
-    // rows past kb and vectors past nv stay finite: zero
-    for (int e = tid; e < nblk * 32 * SV; e += STHREADS) {
-        const int l = e / SV, v = e % SV;
-        if (l >= kb || v >= nv) X[l * SST + v] = cmk(0.0, 0.0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
     int q = 0;
     for (int J = 0; J < nblk; ++J) {
         for (int I = J; I < nblk; ++I) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();                   // block (I, J) staged; X rows of the last step
-            const cd *m = M + q * 32 * SST;
+            const cd *m = M + q * 32 * MST;
             q ^= 1;
             // the other buffer was last read before this barrier
             if (I + 1 < nblk) stage(I + 1, J, q);
             else if (J + 1 < nblk) stage(J + 1, J + 1, q);
             if (I == J) {
                 if (!unit && tid < 32)
-                    dinv[tid] = 32 * J + tid < kb ? crcp(m[tid * SST + tid]) : cmk(0.0, 0.0);
+                    dinv[tid] = 32 * J + tid < kb ? crcp(m[tid * MST + tid]) : cmk(0.0, 0.0);
                 if (!unit) __syncthreads();
-                const int v = wid * 8 + (lane >> 2), r = lane & 3;
-                cd y[8];
+                const int v = wid * (32 / LV) + lane / LV, r = lane % LV;
+                cd y[RL];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) y[i] = X[(32 * J + 4 * i + r) * SST + v];
+                for (int i = 0; i < RL; ++i) y[i] = X[(32 * J + LV * i + r) * SST + v];
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
-                    if (!unit && r == (c & 3)) y[c >> 2] = cmul(y[c >> 2], dinv[c]);
-                    const int src = (lane & ~3) | (c & 3);
-                    const cd x = cmk(__shfl_sync(0xffffffffu, y[c >> 2].x, src),
-                                     __shfl_sync(0xffffffffu, y[c >> 2].y, src));
-                    if (r > (c & 3)) y[c >> 2] = cfms(m[c * SST + 4 * (c >> 2) + r], x, y[c >> 2]);
+                    const int ci = c / LV, cr = c % LV;
+                    if (!unit && r == cr) y[ci] = cmul(y[ci], dinv[c]);
+                    const int src = (lane & ~(LV - 1)) | cr;
+                    const cd x = cmk(__shfl_sync(0xffffffffu, y[ci].x, src),
+                                     __shfl_sync(0xffffffffu, y[ci].y, src));
+                    if (r > cr) y[ci] = cfms(m[c * MST + LV * ci + r], x, y[ci]);
 #pragma unroll
-                    for (int i = (c >> 2) + 1; i < 8; ++i)
-                        y[i] = cfms(m[c * SST + 4 * i + r], x, y[i]);
+                    for (int i = ci + 1; i < RL; ++i)
+                        y[i] = cfms(m[c * MST + LV * i + r], x, y[i]);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) X[(32 * J + 4 * i + r) * SST + v] = y[i];
+                for (int i = 0; i < RL; ++i) X[(32 * J + LV * i + r) * SST + v] = y[i];
             } else {
                 const int gr = lane >> 2, t = lane & 3;
-                const int rl = (wid & 1) * 16, cv = (wid >> 1) * 16;
-                double re[2][4], im[2][4];
+                const int rl = (wid & 1) * 16, cv = (wid >> 1) * 8 * NJ;
+                double re[NJ][4], im[NJ][4];
                 cd *xo = X + (32 * I + rl) * SST + cv;
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < NJ; ++j)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const cd w = xo[(gr + 8 * (e >> 1)) * SST + 8 * j + 2 * t + (e & 1)];
@@ -514,9 +553,9 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
                     }
 #pragma unroll
                 for (int ks = 0; ks < 32; ks += 4) {
-                    const cd a0 = m[(ks + t) * SST + rl + gr], a1 = m[(ks + t) * SST + rl + gr + 8];
+                    const cd a0 = m[(ks + t) * MST + rl + gr], a1 = m[(ks + t) * MST + rl + gr + 8];
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
+                    for (int j = 0; j < NJ; ++j) {
                         const cd x = X[(32 * J + ks + t) * SST + cv + 8 * j + gr];
                         mma_f64(re[j], -a0.x, -a1.x, x.x);
                         mma_f64(im[j], -a0.x, -a1.x, x.y);
@@ -525,7 +564,7 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < NJ; ++j)
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
                         xo[(gr + 8 * (e >> 1)) * SST + 8 * j + 2 * t + (e & 1)] =
@@ -594,20 +633,32 @@ int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A,
                                 sC);
 }
 
-static int launch_strip(cudaStream_t s, const StripArgs &g, int strips, int batch) {
-    if (strips <= 0 || g.kb <= 0) return MNPB_OK;
-    const int smem = (SN + 2 * 32) * SST * (int)sizeof(cd);
-    MNPB_TRY(smem_opt_in(trsm_strip_kernel, smem, "trsm_strip_kernel"));
+template <int SV>
+static int launch_strip_sv(cudaStream_t s, const StripArgs &g, int strips, int batch) {
+    if (strips <= 0) return MNPB_OK;
+    const int smem = (SN * (SV + 2) + 2 * 32 * MST) * (int)sizeof(cd);
+    MNPB_TRY(smem_opt_in(trsm_strip_kernel<SV>, smem, "trsm_strip_kernel"));
     ProfScope ps(s, PC_TRSM, 4.0 * g.kb * g.kb * (double)g.nvec * batch);
-    trsm_strip_kernel<<<dim3(strips, batch), STHREADS, smem, s>>>(g);
+    trsm_strip_kernel<SV><<<dim3(strips, batch), STHREADS, smem, s>>>(g);
     MNPB_LAUNCH_CHECK("trsm_strip_kernel");
     return MNPB_OK;
+}
+
+// vectors [0, g.skip0) and [g.skip1, g.nvec)
+static int launch_strip(cudaStream_t s, const StripArgs &g, int batch) {
+    if (g.kb <= 0) return MNPB_OK;
+    // 16 vectors per CTA while strips of 32 would leave SMs idle: half the work
+    // per strip (one matrix of 284: LU 0.63 -> 0.56 ms, 2884 11.2 -> 10.4 ms)
+    auto strips = [&](int sv) { return ceil_div(g.skip0, sv) + ceil_div(g.nvec - g.skip1, sv); };
+    if ((int64_t)strips(32) * batch <= device_sms())
+        return launch_strip_sv<16>(s, g, strips(16), batch);
+    return launch_strip_sv<32>(s, g, strips(32), batch);
 }
 
 static int trsm_strip(cudaStream_t s, int mode, int kb, const cd *T, int64_t ldt, int64_t sT,
                       cd *B, int64_t ldb, int64_t sB, int nvec, int batch) {
     StripArgs g{mode, kb, T, ldt, sT, B, ldb, sB, nvec, nullptr, 0, 0, 0, 0, 0};
-    return launch_strip(s, g, ceil_div(nvec, SV), batch);
+    return launch_strip(s, g, batch);
 }
 
 static int split_point(int n) {
@@ -713,7 +764,7 @@ static int swap_solve(cudaStream_t s, int off, int w, int j0, int j1, int batch,
     StripArgs g{0,    w,         A + off + (int64_t)off * lda, lda, sA,
                 A + off + (int64_t)j0 * lda, lda, sA, nvec,
                 ipiv + off, sP, off, skip1, skip0, skip1};
-    return launch_strip(s, g, ceil_div(skip0, SV) + ceil_div(nvec - skip1, SV), batch);
+    return launch_strip(s, g, batch);
 }
 
 // Right-looking LU in blocks of SN columns; inside a block, leaf by leaf.  A
@@ -792,16 +843,54 @@ int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda,
     return trsm_lun(s, n, nrhs, batch, LU, lda, sA, B, ldb, sB);
 }
 
+// Column interchanges X <- X P of an m x n block.
+static int permute_cols(cudaStream_t s, cd *X, int64_t ldx, int64_t sX, int m, int n,
+                        const int32_t *ipiv, int64_t sP, int batch) {
+    ProfScope ps(s, PC_SWAP, 0.0);
+    const int RS = (int)min((int64_t)8, 200 * 1024 / (16 * (int64_t)n) - 1);
+    if (RS < 2) {
+        dim3 grid(ceil_div(m, 128), batch);
+        colswp_kernel<<<grid, 128, 0, s>>>(X, ldx, sX, m, ipiv, sP, n);
+        MNPB_LAUNCH_CHECK("colswp_kernel");
+        return MNPB_OK;
+    }
+    MNPB_TRY(smem_opt_in(permute_cols_kernel, 200 * 1024, "permute_cols_kernel"));
+    permute_cols_kernel<<<dim3(ceil_div(m, RS), batch), 256, (size_t)16 * n * (RS + 1), s>>>(
+        X, ldx, sX, m, ipiv, sP, n, RS);
+    MNPB_LAUNCH_CHECK("permute_cols_kernel");
+    return MNPB_OK;
+}
+
 // X A = B in place on B (m x n), A = P^T L U from getrf.
 int right_solve(cudaStream_t s, int n, int m, int batch, const cd *LU, int64_t lda, int64_t sA,
                 const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB) {
     MNPB_TRY(trsm_run(s, n, m, batch, LU, lda, sA, B, ldb, sB));
     MNPB_TRY(trsm_rlu(s, n, m, batch, LU, lda, sA, B, ldb, sB));
-    dim3 grid(ceil_div(m, 128), batch);
-    ProfScope ps(s, PC_SWAP, 0.0);
-    colswp_kernel<<<grid, 128, 0, s>>>(B, ldb, sB, m, ipiv, sP, n);
-    MNPB_LAUNCH_CHECK("colswp_kernel");
-    return MNPB_OK;
+    return permute_cols(s, B, ldb, sB, m, n, ipiv, sP, batch);
+}
+
+// X <- L^-1 for X = identity on entry: above the diagonal X stays zero, so
+// X11 = L11^-1, X21 = -L22^-1 (L21 X11), X22 = L22^-1: a third of the
+// operations of a solve against n full columns.
+static int trsm_llu_eye(cudaStream_t s, int n, int batch, const cd *L, int64_t ldl, int64_t sL,
+                        cd *X, int64_t ldx, int64_t sX) {
+    if (n <= SN) return trsm_strip(s, 0, n, L, ldl, sL, X, ldx, sX, n, batch);
+    const int n1 = split_point(n);
+    const cd *L22 = L + n1 + (int64_t)n1 * ldl;
+    MNPB_TRY(trsm_llu_eye(s, n1, batch, L, ldl, sL, X, ldx, sX));
+    MNPB_TRY(zgemm(s, n - n1, n1, n1, batch, cmk(-1, 0), L + n1, ldl, sL, X, ldx, sX, cmk(0, 0),
+                   X + n1, ldx, sX));
+    MNPB_TRY(trsm_llu(s, n - n1, n1, batch, L22, ldl, sL, X + n1, ldx, sX));
+    return trsm_llu_eye(s, n - n1, batch, L22, ldl, sL, X + n1 + (int64_t)n1 * ldx, ldx, sX);
+}
+
+// X <- A^-1 = U^-1 L^-1 P from getrf's factors.
+int getri(cudaStream_t s, int n, int batch, const cd *LU, int64_t lda, int64_t sA,
+          const int32_t *ipiv, int64_t sP, cd *X, int64_t ldx, int64_t sX) {
+    MNPB_TRY(set_identity(s, n, batch, X, ldx, sX));
+    MNPB_TRY(trsm_llu_eye(s, n, batch, LU, lda, sA, X, ldx, sX));
+    MNPB_TRY(trsm_lun(s, n, n, batch, LU, lda, sA, X, ldx, sX));
+    return permute_cols(s, X, ldx, sX, n, n, ipiv, sP, batch);
 }
 
 int set_identity(cudaStream_t s, int n, int batch, cd *W, int64_t ldw, int64_t sW) {

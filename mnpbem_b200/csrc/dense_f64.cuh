@@ -23,6 +23,9 @@ int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda,
           const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB);
 int right_solve(cudaStream_t s, int n, int m, int batch, const cd *LU, int64_t lda, int64_t sA,
                 const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB);
+// X <- A^-1 from getrf's factors.
+int getri(cudaStream_t s, int n, int batch, const cd *LU, int64_t lda, int64_t sA,
+          const int32_t *ipiv, int64_t sP, cd *X, int64_t ldx, int64_t sX);
 int set_identity(cudaStream_t s, int n, int batch, cd *W, int64_t ldw, int64_t sW);
 
 }  // namespace mnpb

@@ -152,3 +152,41 @@ def test_getrs_interchange_chains(gpu_ok):
             for c, r in enumerate(p):
                 want[[c, r]] = want[[r, c]]
             assert np.array_equal(X.real.cpu().numpy(), np.tile(want, (nrhs, 1)))
+
+
+@pytest.mark.parametrize('n,batch', [(5, 2), (33, 1), (128, 2), (129, 1), (300, 3), (1000, 1),
+                                     (4300, 1)])
+def test_right_solve_and_inverse(gpu_ok, n, batch):
+    """Sigma1 = H1 G1^-1 and Delta^-1 of ``mnpb_bemret_init_f64`` on random
+    matrices: |Sigma1 G1 - H1| <= 8 n eps |Sigma1| |G1| growth and
+    |Delta Delta^-1 - I| <= 8 n eps |Delta| |Delta^-1| growth in the largest
+    entry, with a growth factor of 30 for the factorisations."""
+    G1, G2, H1, H2 = [_rand(batch, n, n, seed=s) for s in (1, 2, 3, 4)]
+    GG, HH = torch.stack([G1, G2]), torch.stack([H1, H2])
+    D = torch.empty_like(G1)
+    eps = torch.tensor([[-10.0, 1.0, 1.0, 0.0]], dtype=torch.float64, device='cuda') \
+        .repeat(batch, 1)
+    kvac = torch.full((batch,), 0.01, dtype=torch.float64, device='cuda')
+    nvec = torch.zeros((n, 3), dtype=torch.float64, device='cuda')
+    piv = torch.empty((3, batch, n), dtype=torch.int32, device='cuda')
+    info = torch.zeros((2, batch), dtype=torch.int32, device='cuda')
+    wb = int(_lib.lib().mnpb_bemret_workspace_f64(n, batch))
+    work = torch.empty(wb, dtype=torch.uint8, device='cuda')
+    call('mnpb_bemret_init_f64', _lib.stream_handle(), n, batch, ptr(GG[0]), ptr(GG[1]),
+         ptr(HH[0]), ptr(HH[1]), ptr(D), n, n * n, ptr(eps), ptr(kvac), ptr(nvec), 0, ptr(piv),
+         ptr(info), ptr(work), wb)
+    assert not info.any()
+    T = lambda x: x.transpose(1, 2)
+    S1, g1 = T(HH[0]), T(G1)
+    scale = 30 * 8 * n * EPS
+    res = (S1 @ g1 - T(H1)).abs().amax()
+    assert float(res) <= scale * float((S1.abs() @ g1.abs()).amax())
+    S2 = torch.linalg.solve(T(G2), T(H2), left=False)
+    delta, inv = S1 - S2, T(D)
+    eye = torch.eye(n, dtype=delta.dtype, device='cuda')
+    # Sigma2 of the reference differs from the solver's by a relative error of
+    # the same kind, which the inverse multiplies
+    bound = scale * float((delta.abs() @ inv.abs()).amax() +
+                          ((S2.abs() @ T(G2).abs()) @ torch.linalg.inv(T(G2)).abs()
+                           @ inv.abs()).amax())
+    assert float((delta @ inv - eye).abs().amax()) <= bound
