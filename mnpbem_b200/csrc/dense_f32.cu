@@ -8,6 +8,7 @@
 // inverses and the 32-row leaves of small triangular solves run on CUDA cores.
 #include "common.cuh"
 #include "dense_f32.cuh"
+#include "lu_panel.cuh"
 
 #include <cuda.h>
 
@@ -56,6 +57,36 @@ __device__ __forceinline__ void st(float *p, int64_t plane, int64_t o, cf v) {
     p[o] = v.x;
     p[o + plane] = v.y;
 }
+
+// Planar FP32 storage for the cluster LU panels.
+struct Planar {
+    typedef cf V;
+    typedef float S;
+    struct Mat {
+        float *A;
+        int64_t lda, plane, sA;
+    };
+    static __device__ __forceinline__ V zero() { return fmk(0.f, 0.f); }
+    static __device__ __forceinline__ V load(const Mat &m, int64_t b, int64_t row, int64_t col) {
+        return ld(m.A + b * m.sA, m.plane, col * m.lda + row);
+    }
+    static __device__ __forceinline__ void store(const Mat &m, int64_t b, int64_t row,
+                                                 int64_t col, V v) {
+        st(m.A + b * m.sA, m.plane, col * m.lda + row, v);
+    }
+    static __device__ __forceinline__ S mag(V v) { return fabsf(v.x) + fabsf(v.y); }
+    static __device__ __forceinline__ V rcp(V v) { return frcp(v); }
+    static __device__ __forceinline__ V mul(V a, V b) { return fmul(a, b); }
+    static __device__ __forceinline__ V fms(V a, V b, V c) { return ffms(a, b, c); }
+    static __device__ __forceinline__ V rnd(V v) { return rna(v); }   // L and U are stored as TF32
+    static __device__ __forceinline__ void push(uint32_t addr, V v) {
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y)
+                     : "memory");
+    }
+    static __device__ __forceinline__ void push_s(uint32_t addr, S v) {
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+    }
+};
 
 // LU leaf: columns [k0, k0+kb) (kb <= 32) over rows [k0, n), one CTA per matrix.
 __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(int n, int k0, int kb, float *A,
@@ -1859,6 +1890,19 @@ static int rgetrf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, int64_t
     if (w <= TS) {
         ProfScope ps(c.s, PC_PANEL, 8.0 * w * w * (double)(n - off) * c.batch / 2);
         prof_tag("off=%d w=%d B=%d", off, w, c.batch);
+        const Planar::Mat mat{A.p, A.ld, A.plane, A.stride};
+        int C, threads;
+        // registers of a cluster while that runs in one wave: one row per
+        // thread if it does, two otherwise (LU of 2884 matrices: 1 16.4 ->
+        // 10.7 ms, 8 19.5 -> 14.1, 27 24.7 -> 21.2).  More matrices keep one
+        // CTA each and the slab in shared memory, whose pivot steps are longer
+        // but leave no second wave (54: 33.2 against 34.0, 162: 83 against 91)
+        if (lup::panel_shape(n - off, 1, C, threads) && (int64_t)C * c.batch <= dev_sms())
+            return lup::launch_panel<Planar, TS, 1>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                    C, threads);
+        if (lup::panel_shape(n - off, 2, C, threads) && (int64_t)C * c.batch <= dev_sms())
+            return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                    C, threads);
         MNPB_TRY(smem_opt_in(panel_slab_kernel<8>, 200 * 1024, "panel_slab_kernel<8>"));
         MNPB_TRY(smem_opt_in(panel_slab_kernel<4>, 200 * 1024, "panel_slab_kernel<4>"));
         // more matrices than SMs: 4-column slabs, half the shared memory, so
@@ -1876,6 +1920,9 @@ static int rgetrf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, int64_t
             MNPB_LAUNCH_CHECK("panel_slab_kernel(f32)");
             return MNPB_OK;
         }
+        if (lup::panel_shape(n - off, 2, C, threads))
+            return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                    C, threads);
         panel_kernel<<<c.batch, PANEL_THREADS, 0, c.s>>>(n, off, w, A.p, A.ld, A.plane, A.stride,
                                                          ipiv, sP, info);
         MNPB_LAUNCH_CHECK("panel_kernel(f32)");
