@@ -123,10 +123,8 @@ extern "C" int mnpb_bemret_solve_f64(void *stream, int64_t n, int64_t batch, int
                    cmk(0, 0), V, n, sAP));
     solve_out_kernel<<<g, 128, 0, s>>>(N, k, xin, sx, R, sR, V, sAP, xout, sx);
     MNPB_LAUNCH_CHECK("solve_out_kernel");
-    MNPB_TRY(getrs(s, N, 4 * k, B, (const cd *)G1, ld, stride, piv1, ps, xout, n, sx));
-    MNPB_TRY(getrs(s, N, 4 * k, B, (const cd *)G2, ld, stride, piv2, ps, xout + 4 * K * n, n,
-                   sx));
-    return MNPB_OK;
+    return getrs_pair(s, N, 4 * k, B, (const cd *)G1, (const cd *)G2, ld, stride, piv1, piv2, ps,
+                      xout, xout + 4 * K * n, n, sx);
 }
 
 extern "C" int mnpb_bemret_excitation(void *stream, int64_t n, int64_t batch, int64_t nrhs,

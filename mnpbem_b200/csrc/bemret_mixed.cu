@@ -224,7 +224,6 @@ struct Factors {
     const int32_t *pivG1, *pivG2, *pivS;            // n per batch entry
     const float *iG1L, *iG1U, *iG2L, *iG2U, *iSL, *iSU;   // diagonal-block inverses
     int64_t n, dinv_per;                            // dinv_per: floats per entry
-    int *trsv_state;      // flags + ticket of the one-launch triangular solves
     // the same factors for batch entries b0, b0 + 1, ...
     Factors at(int b0) const {
         Factors f = *this;
@@ -289,7 +288,7 @@ static int mgetrs(f32::Ctx &c, int n, int m, const float *LU, const Factors &F,
     MNPB_TRY(convert_in(c.s, n, m, c.batch, x, sx, t1));
     const int64_t pl = (int64_t)n * m;
     MNPB_TRY(f32::getrs_few(c, n, m, CMatF{(float *)LU, F.ld, F.plane, F.stride}, piv,
-                            (int64_t)n, invL, invU, CMatF{t1, n, pl, 2 * pl}, F.trsv_state));
+                            (int64_t)n, invL, invU, CMatF{t1, n, pl, 2 * pl}));
     return convert_out(c.s, n, m, c.batch, t1, x, sx);
 }
 
@@ -323,8 +322,17 @@ static int msolve(f32::Ctx &c, int n, int K, const Factors &F, const double *eps
     MNPB_TRY(mgemm(c, n, 3 * K, F.D, F, AP, sAP, V, sAP, t1, t2));
     solve_out_kernel<<<g, 128, 0, s>>>(n, K, xin, sx, R, sR, V, sAP, xout, sx);
     MNPB_LAUNCH_CHECK("solve_out_kernel");
-    MNPB_TRY(mgetrs(c, n, 4 * K, F.G1, F, F.pivG1, F.iG1L, F.iG1U, xout, sx, t1));
-    return mgetrs(c, n, 4 * K, F.G2, F, F.pivG2, F.iG2L, F.iG2U, xout + 4 * K * nn, sx, t1);
+    if (2 * B > 65535) {     // the conversions' grid
+        MNPB_TRY(mgetrs(c, n, 4 * K, F.G1, F, F.pivG1, F.iG1L, F.iG1U, xout, sx, t1));
+        return mgetrs(c, n, 4 * K, F.G2, F, F.pivG2, F.iG2L, F.iG2U, xout + 4 * K * nn, sx, t1);
+    }
+    // G1 [sig1 h1] and G2 [sig2 h2]: 2 B right-hand-side blocks back to back
+    const int64_t s4 = nn * 4 * K, pl = s4;
+    MNPB_TRY(convert_in(s, n, 4 * K, 2 * B, xout, s4, t1));
+    MNPB_TRY(f32::getrs_few_pair(c, n, 4 * K, CMatF{F.G1, F.ld, F.plane, F.stride}, F.G2, F.pivG1,
+                                 F.pivG2, (int64_t)n, F.iG1L, F.iG1U, F.iG2L - F.iG1L,
+                                 CMatF{t1, n, pl, 4 * pl}, 2 * pl));
+    return convert_out(s, n, 4 * K, 2 * B, t1, xout, s4);
 }
 
 }  // namespace mixed
@@ -524,7 +532,6 @@ extern "C" int64_t mnpb_bemret_refine_workspace(int64_t n, int64_t batch, int64_
     const int64_t K = nrhs;
     // msolve scratch (15 K n c128 + 2 x 16 K n float... per entry) + r, d, P1..Q2 + norms
     return batch * n * K * (15 * 16 + 2 * 16 * 8 + 2 * 8 * 16 + 4 * 4 * 16) + 8 * 256 +
-           align_up(f32::trsv_state_bytes((int)n, (int)batch), 256) +
            align_up(tc::cgemm_tf32_workspace((int)n, 64, (int)batch), 256);
 }
 
@@ -558,7 +565,7 @@ extern "C" int mnpb_bemret_solve_refine(
     Factors F{(float *)G1p, (float *)G2p, (float *)S1p, (float *)Sp, (float *)Dp, ld, plane,
               2 * plane, piv, piv + Bn, piv + 2 * Bn, dinv + dv.gL(0, batch),
               dinv + dv.gU(0, batch), dinv + dv.gL(1, batch), dinv + dv.gU(1, batch),
-              dinv + dv.sL(batch), dinv + dv.sU(batch), n, dv.S, nullptr};
+              dinv + dv.sL(batch), dinv + dv.sU(batch), n, dv.S};
     const int64_t per = n * K;
     char *wp = (char *)work;
     auto take = [&](int64_t bytes) {
@@ -572,7 +579,6 @@ extern "C" int mnpb_bemret_solve_refine(
     cd *dx = (cd *)take(batch * per * 8 * 16);
     cd *P = (cd *)take(batch * per * 4 * 4 * 16);
     double *nrm = (double *)take(batch * 4 * 8);
-    F.trsv_state = (int *)take(f32::trsv_state_bytes(N, B));
     const int64_t tcw = (int64_t)((char *)work + work_bytes - wp);
     f32::Ctx c(s, B, (float *)wp, tcw);
     const int64_t sx = per * 8, sP4 = per * 4;
@@ -673,12 +679,11 @@ extern "C" int mnpb_bemret_solve_refine(
     }
     // relres holds each entry's relative residual before its last correction
     // (no extra pass over the FP64 operator just to report the final one)
-    int terr = 0, gerr = 0;
-    MNPB_TRY(f32::trsv_error_read_and_clear(s, &terr));
+    int gerr = 0;
     MNPB_TRY(tc::tc_error_read_and_clear(s, &gerr));
-    if (terr || gerr) {
-        set_error("bemret_solve_refine: a bounded device wait timed out (%s)",
-                  terr ? "triangular solve" : "tensor-core GEMM of the factorisation");
+    if (gerr) {
+        set_error("bemret_solve_refine: a bounded device wait timed out (tensor-core GEMM of the "
+                  "factorisation)");
         return MNPB_ETIMEOUT;
     }
     for (int b = 0; b < B; ++b)

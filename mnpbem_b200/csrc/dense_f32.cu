@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "dense_f32.cuh"
 #include "lu_panel.cuh"
+#include "trsv_cluster.cuh"
 
 #include <cuda.h>
 
@@ -58,7 +59,7 @@ __device__ __forceinline__ void st(float *p, int64_t plane, int64_t o, cf v) {
     p[o + plane] = v.y;
 }
 
-// Planar FP32 storage for the cluster LU panels.
+// Planar FP32 storage for the cluster kernels (LU panels, triangular solves).
 struct Planar {
     typedef cf V;
     typedef float S;
@@ -78,6 +79,15 @@ struct Planar {
     static __device__ __forceinline__ V rcp(V v) { return frcp(v); }
     static __device__ __forceinline__ V mul(V a, V b) { return fmul(a, b); }
     static __device__ __forceinline__ V fms(V a, V b, V c) { return ffms(a, b, c); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) {
+        c.x = fmaf(a.x, b.x, c.x);
+        c.x = fmaf(-a.y, b.y, c.x);
+        c.y = fmaf(a.x, b.y, c.y);
+        c.y = fmaf(a.y, b.x, c.y);
+        return c;
+    }
+    static __device__ __forceinline__ V add(V a, V b) { return fmk(a.x + b.x, a.y + b.y); }
+    static __device__ __forceinline__ V sub(V a, V b) { return fmk(a.x - b.x, a.y - b.y); }
     static __device__ __forceinline__ V rnd(V v) { return rna(v); }   // L and U are stored as TF32
     static __device__ __forceinline__ void push(uint32_t addr, V v) {
         asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y)
@@ -85,6 +95,60 @@ struct Planar {
     }
     static __device__ __forceinline__ void push_s(uint32_t addr, S v) {
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+    }
+    static __device__ __forceinline__ V shfl(V v, int l) {
+        return fmk(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+    }
+    static __device__ __forceinline__ V shfl_xor(V v, int o) {
+        return fmk(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+    }
+};
+
+// Triangular solves: the 64-row diagonal blocks are solved through the
+// precomputed inverses of their two 32-row halves (dinv: diag_inv_kernel).
+struct PlanarTri : Planar {
+    typedef Planar::Mat Mat;
+    // staged diagonal block: inverse of the first half, the block below it,
+    // inverse of the second half, each column by column in solve order
+    static constexpr int DELEMS = 3 * 32 * 32;
+    static constexpr int P = 2;
+    static __device__ __forceinline__ void stage(V *D, const Mat &A, const float *dinv, int64_t b,
+                                                 int n, int blk, bool lower, int tid) {
+        const int nb32 = (n + 31) / 32;
+        const int h0 = lower ? 0 : 1, h1 = 1 - h0;       // physical halves in solve order
+        V v[DELEMS / trc::THREADS];
+#pragma unroll
+        for (int q = 0; q < DELEMS / trc::THREADS; ++q) {
+            const int e = tid + q * trc::THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
+            v[q] = fmk(0.f, 0.f);
+            if (w == 1) {
+                const int gr = blk * 64 + 32 * h1 + i, gc = blk * 64 + 32 * h0 + t;
+                if (gr < n && gc < n) v[q] = load(A, b, gr, gc);
+            } else {
+                const int sb = 2 * blk + (w == 0 ? h0 : h1);
+                if (sb < nb32) {
+                    const float *d = dinv + ((b * nb32 + sb) * 2) * 1024 + t * 32 + i;
+                    v[q] = fmk(__ldg(d), __ldg(d + 1024));
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < DELEMS / trc::THREADS; ++q) {
+            const int e = tid + q * trc::THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
+            D[lower ? e : w * 1024 + (31 - t) * 32 + 31 - i] = v[q];
+        }
+    }
+    static __device__ __forceinline__ void diag(const V *D, bool, int lane, V &r0, V &r1) {
+        V y = fmk(0.f, 0.f);
+#pragma unroll 8
+        for (int t = 0; t < 32; ++t) y = fma(D[t * 32 + lane], shfl(r0, t), y);
+        r0 = y;
+#pragma unroll 8
+        for (int t = 0; t < 32; ++t) r1 = ffms(D[1024 + t * 32 + lane], shfl(r0, t), r1);
+        y = fmk(0.f, 0.f);
+#pragma unroll 8
+        for (int t = 0; t < 32; ++t) y = fma(D[2048 + t * 32 + lane], shfl(r1, t), y);
+        r1 = y;
     }
 };
 
@@ -839,20 +903,10 @@ __global__ void __launch_bounds__(128) skinny_kernel(int m, int n, int k, float 
 
 
 // ---------------------------------------------------------------------------
-// Few-RHS triangular solves in one launch per triangle.
-//
-// Block rows of 32: block j needs the solution of every earlier block (in
-// solve order).  A CTA takes a ticket from an atomic counter and handles the
-// (block, matrix) pair of that ticket, tickets ordered block-major, so every
-// block it waits for has a lower ticket and has started: the smallest
-// unfinished ticket can always proceed.  Blocks publish their solution with a
-// release (fence + atomic flag = epoch); waiters use acquire loads, bounded
-// by a 1 s wall-clock limit after which an error word is set and the kernel
-// continues (the solve is then invalid and reported, but nothing hangs).
-// The 32 x 32 diagonal blocks are applied through precomputed inverses.
+// Few-RHS triangular solves: inverses of the 32 x 32 diagonal blocks, and the
+// bounded device waits that the failure-path probe runs.
 // ---------------------------------------------------------------------------
 constexpr int TB = 32;
-constexpr uint64_t TRSV_WAIT_NS = 1000000000ull;
 
 __device__ int g_trsv_error;
 
@@ -922,287 +976,13 @@ __global__ void __launch_bounds__(TB) diag_inv_kernel(int n, int lower, const fl
     }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(256) trsv_kernel(int n, int m, int lower, const float *A,
-                                                   int64_t lda, int64_t plane, int64_t sA,
-                                                   const float *__restrict__ Dinv, float *X,
-                                                   int64_t ldx, int64_t planeX, int64_t sX,
-                                                   int *flags, unsigned *ticket, int epoch,
-                                                   int nb, int batch) {
-    __shared__ int s_ticket;
-    __shared__ cf red[8][TB][NC];
-    __shared__ cf rhs[TB][NC];
-    __shared__ cf dinv_s[TB][TB + 1];
-    const int tid = threadIdx.x, r = tid & 31, q = tid >> 5;
-    if (tid == 0) s_ticket = (int)atomicAdd(ticket, 1u);
-    __syncthreads();
-    const int tk = s_ticket;
-    const int jj = tk / batch;
-    const int64_t b = tk % batch;
-    const int j = lower ? jj : nb - 1 - jj;
-    const int r0 = j * TB, rows = min(TB, n - r0);
-    A += b * sA;
-    X += b * sX;
-    int *fl = flags + b * nb;
-    // stage the inverse of the diagonal block (independent of other blocks)
-    const float *Di = Dinv + (b * nb + j) * 2 * TB * TB;
-    for (int e = tid; e < TB * TB; e += 256) {
-        const int rr = e % TB, k = e / TB;
-        dinv_s[rr][k] = fmk(__ldg(Di + k * TB + rr), __ldg(Di + TB * TB + k * TB + rr));
-    }
-    cf acc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] = fmk(0.f, 0.f);
-    // blocks finish in chain order, so once the last dependency is published
-    // every earlier one is too
-    int known = -1;
-    if (jj > 0 && r == 0) {
-        const int last = lower ? jj - 1 : nb - jj;
-        if (ld_acquire(fl + last) == epoch) known = jj - 1;
-    }
-    known = __shfl_sync(0xffffffffu, known, 0);
-    __syncwarp();   // orders the lanes' later reads after lane 0's acquire
-    for (int ii = 0; ii < jj; ++ii) {
-        const int i = lower ? ii : nb - 1 - ii;
-        // factor entries first: they do not depend on other blocks
-        cf a[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int col = i * TB + q + 8 * t;
-            a[t] = fmk(0.f, 0.f);
-            if (col < n && r < rows) {
-                const int64_t o = (int64_t)col * lda + r0 + r;
-                a[t] = fmk(A[o], A[o + plane]);
-            }
-        }
-        if (ii > known) {
-            // lane 0 of each warp waits (acquire); __syncwarp orders the lanes' reads
-            if (r == 0 && !wait_flag(fl + i, epoch, TRSV_WAIT_NS)) atomicCAS(&g_trsv_error, 0, 1);
-            __syncwarp();
-            known = ii;
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int col = i * TB + q + 8 * t;
-            if (col < n && r < rows) {
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if (c < m) {
-                        const int64_t xo = (int64_t)c * ldx + col;
-                        const cf xv = fmk(__ldcg(X + xo), __ldcg(X + xo + planeX));
-                        acc[c].x = fmaf(a[t].x, xv.x, acc[c].x);
-                        acc[c].x = fmaf(-a[t].y, xv.y, acc[c].x);
-                        acc[c].y = fmaf(a[t].x, xv.y, acc[c].y);
-                        acc[c].y = fmaf(a[t].y, xv.x, acc[c].y);
-                    }
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) red[q][r][c] = acc[c];
-    __syncthreads();
-    for (int e = tid; e < TB * NC; e += 256) {
-        const int rr = e % TB, c = e / TB;
-        cf v = fmk(0.f, 0.f);
-        if (rr < rows && c < m) {
-            const int64_t xo = (int64_t)c * ldx + r0 + rr;
-            v = fmk(__ldcg(X + xo), __ldcg(X + xo + planeX));
-#pragma unroll
-            for (int qq = 0; qq < 8; ++qq) {
-                v.x -= red[qq][rr][c].x;
-                v.y -= red[qq][rr][c].y;
-            }
-        }
-        rhs[rr][c] = v;
-    }
-    __syncthreads();
-    for (int e = tid; e < TB * NC; e += 256) {
-        const int rr = e % TB, c = e / TB;
-        if (rr < rows && c < m) {
-            cf y = fmk(0.f, 0.f);
-#pragma unroll 8
-            for (int k = 0; k < TB; ++k) {
-                const cf d = dinv_s[rr][k];
-                y.x = fmaf(d.x, rhs[k][c].x, y.x);
-                y.x = fmaf(-d.y, rhs[k][c].y, y.x);
-                y.y = fmaf(d.x, rhs[k][c].y, y.y);
-                y.y = fmaf(d.y, rhs[k][c].x, y.y);
-            }
-            const int64_t xo = (int64_t)c * ldx + r0 + rr;
-            X[xo] = y.x;
-            X[xo + planeX] = y.y;
-        }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        atomicExch(fl + j, epoch);
-    }
-}
-
-// Few-RHS triangular solve, one CTA per matrix, right-looking: the whole
-// right-hand side lives in shared memory (r[i][c], n x NC), each 32-row block
-// is solved through its precomputed diagonal inverse, then every row the
-// block feeds (below it for L, above it for U) subtracts T[i, block] x_block,
-// streaming that column block of the triangle once.  Two rows per thread with
-// 8-byte loads, 16 columns in flight; the next block's diagonal inverse is
-// staged while the current block's update runs.  No inter-CTA waits.
-constexpr int RL_THREADS = 512;
-template <int NC>
-__global__ void __launch_bounds__(RL_THREADS) trsv_rl_kernel(int n, int m, int lower,
-                                                             const float *__restrict__ A,
-                                                             int64_t lda, int64_t plane,
-                                                             int64_t sA,
-                                                             const float *__restrict__ Dinv,
-                                                             float *X, int64_t ldx,
-                                                             int64_t planeX, int64_t sX, int nb) {
-    extern __shared__ __align__(16) unsigned char rl_smem[];
-    cf *r = reinterpret_cast<cf *>(rl_smem);   // r[i * NC + c]
-    __shared__ cf dsm[2][TB][TB + 1];
-    __shared__ cf xj[TB][NC];
-    const int tid = threadIdx.x;
-    const int64_t b = blockIdx.x;
-    A += b * sA;
-    X += b * sX;
-    const float *Db = Dinv + b * nb * 2 * TB * TB;
-    for (int e = tid; e < n * NC; e += RL_THREADS) {
-        const int i = e % n, c = e / n;
-        r[i * NC + c] = c < m ? ld(X, planeX, (int64_t)c * ldx + i) : fmk(0.f, 0.f);
-    }
-    {
-        const int j = lower ? 0 : nb - 1;
-        const float *Di = Db + (int64_t)j * 2 * TB * TB;
-        for (int e = tid; e < TB * TB; e += RL_THREADS) {
-            const int rr = e % TB, k = e / TB;
-            dsm[0][rr][k] = fmk(__ldg(Di + k * TB + rr), __ldg(Di + TB * TB + k * TB + rr));
-        }
-    }
-    __syncthreads();
-    for (int jj = 0; jj < nb; ++jj) {
-        const int j = lower ? jj : nb - 1 - jj, r0 = j * TB, rows = min(TB, n - r0);
-        const int buf = jj & 1;
-        // diagonal block: x_j = D_j^{-1} r_j
-        if (tid < TB * NC) {
-            const int rr = tid % TB, c = tid / TB;
-            cf y = fmk(0.f, 0.f);
-            if (rr < rows && c < m) {
-#pragma unroll 8
-                for (int k = 0; k < TB; ++k) {
-                    if (k < rows) {
-                        const cf d = dsm[buf][rr][k], v = r[(r0 + k) * NC + c];
-                        y.x = fmaf(d.x, v.x, y.x);
-                        y.x = fmaf(-d.y, v.y, y.x);
-                        y.y = fmaf(d.x, v.y, y.y);
-                        y.y = fmaf(d.y, v.x, y.y);
-                    }
-                }
-                st(X, planeX, (int64_t)c * ldx + r0 + rr, y);
-            }
-            xj[rr][c] = y;
-        }
-        __syncthreads();
-        // stage the next block's inverse while this block's update runs
-        if (jj + 1 < nb) {
-            const int jn = lower ? j + 1 : j - 1;
-            const float *Di = Db + (int64_t)jn * 2 * TB * TB;
-            for (int e = tid; e < TB * TB; e += RL_THREADS) {
-                const int rr = e % TB, k = e / TB;
-                dsm[buf ^ 1][rr][k] =
-                    fmk(__ldg(Di + k * TB + rr), __ldg(Di + TB * TB + k * TB + rr));
-            }
-        }
-        const int lo = lower ? r0 + rows : 0, hi = lower ? n : r0;
-        const float *Ac = A + (int64_t)r0 * lda;
-        for (int i = lo + 2 * tid; i < hi; i += 2 * RL_THREADS) {
-            const bool two = i + 1 < hi;
-            cf a0[NC], a1[NC];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) a0[c] = a1[c] = fmk(0.f, 0.f);
-            for (int k0 = 0; k0 < rows; k0 += 16) {
-                float2 vr[16], vi[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    vr[k] = vi[k] = make_float2(0.f, 0.f);
-                    if (k0 + k < rows) {
-                        const float *p = Ac + (int64_t)(k0 + k) * lda + i;
-                        if (two) {
-                            vr[k] = __ldg(reinterpret_cast<const float2 *>(p));
-                            vi[k] = __ldg(reinterpret_cast<const float2 *>(p + plane));
-                        } else {
-                            vr[k].x = __ldg(p);
-                            vi[k].x = __ldg(p + plane);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const cf x = xj[(k0 + k) & (TB - 1)][c];
-                        a0[c].x = fmaf(vr[k].x, x.x, a0[c].x);
-                        a0[c].x = fmaf(-vi[k].x, x.y, a0[c].x);
-                        a0[c].y = fmaf(vr[k].x, x.y, a0[c].y);
-                        a0[c].y = fmaf(vi[k].x, x.x, a0[c].y);
-                        a1[c].x = fmaf(vr[k].y, x.x, a1[c].x);
-                        a1[c].x = fmaf(-vi[k].y, x.y, a1[c].x);
-                        a1[c].y = fmaf(vr[k].y, x.y, a1[c].y);
-                        a1[c].y = fmaf(vi[k].y, x.x, a1[c].y);
-                    }
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                cf &u = r[i * NC + c];
-                u.x -= a0[c].x;
-                u.y -= a0[c].y;
-                if (two) {
-                    cf &w = r[(i + 1) * NC + c];
-                    w.x -= a1[c].x;
-                    w.y -= a1[c].y;
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// ---- few-RHS triangular solve with the triangle streamed by TMA ------------
-//
-// One CTA per matrix; the right-hand sides r (n x NC) stay in shared memory.
-// Warp 9 (one lane) streams the triangle block column by block column in the
-// order the solve consumes it: for 32-column block j, the inverse of its
-// diagonal block (8 KB, bulk copy) and then every 128-row tile the block
-// updates (below it for L, above it, bottom tile first, for U), through a
-// ring of S stages; it runs ahead of the arithmetic, bounded only by the
-// ring.  Warp 8 solves the diagonal blocks (x_j = D_j^{-1} r_j) into a double
-// buffer as soon as the first tile of the previous block has updated block
-// j's rows; warps 0-7 update r with each tile: thread t takes row t % 128 and
-// half of the tile's 32 columns (t / 128); the second half's partial sums
-// meet the first half's through a double buffer in shared memory.  Every
-// mbarrier wait is bounded; on a timeout the kernel records an error in
-// g_trsv_error and stops.
-constexpr int STR_ROWS = 128;                                  // rows per tile
-constexpr int STR_TILE_BYTES = 2 * TB * STR_ROWS * 4;          // re + im planes
-constexpr int STR_CONS = 256;                                  // consumer threads
-constexpr int STR_THREADS = STR_CONS + 64;
-constexpr uint64_t STR_WAIT_NS = 1000000000ull;
-
 __device__ __forceinline__ uint32_t s_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 __device__ __forceinline__ void sbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
-__device__ __forceinline__ void sbar_expect(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void sbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool sbar_wait(uint32_t bar, uint32_t parity,
-                                          uint64_t limit = STR_WAIT_NS) {
+__device__ __forceinline__ bool sbar_wait(uint32_t bar, uint32_t parity, uint64_t limit) {
     const uint64_t t0 = gtimer();
     while (true) {
         uint32_t ok;
@@ -1217,276 +997,6 @@ __device__ __forceinline__ bool sbar_wait(uint32_t bar, uint32_t parity,
         if (gtimer() - t0 > limit) return false;
     }
 }
-__device__ __forceinline__ void s_tma3(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                       int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-        "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void s_bulk(uint32_t dst, const void *src, uint32_t bytes,
-                                       uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(dst),
-        "l"((uint64_t)src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-
-template <int NC>
-__global__ void __launch_bounds__(STR_THREADS, 1)
-    trsv_stream_kernel(const __grid_constant__ CUtensorMap tmRe,
-                       const __grid_constant__ CUtensorMap tmIm, int n, int m, int lower,
-                       const float *__restrict__ Dinv, float *X, int64_t ldx, int64_t planeX,
-                       int64_t sX, int nb, int S) {
-    extern __shared__ __align__(1024) unsigned char str_raw[];
-    unsigned char *sm = (unsigned char *)(((uintptr_t)str_raw + 1023) & ~(uintptr_t)1023);
-    float *ring = (float *)sm;                                        // S tiles
-    float *dsm = (float *)(sm + (size_t)S * STR_TILE_BYTES);          // 2 x [2][32][32]
-    cf *xb = (cf *)(dsm + 2 * 2 * TB * TB);                           // 2 x [32][NC]
-    cf *red = xb + 2 * TB * NC;                                       // 2 x [128][NC]
-    cf *r = red + 2 * STR_ROWS * NC;                                  // [n][NC]
-    uint64_t *bars = (uint64_t *)(r + (size_t)n * NC);
-    // bars: full[S], empty[S], dfull[2], dempty[2], rows_ready, xready[2],
-    // red_full[2], red_empty[2]
-    uint64_t *full = bars, *empty = bars + S, *dfull = bars + 2 * S, *dempty = dfull + 2;
-    uint64_t *rows_ready = dempty + 2, *xready = rows_ready + 1;
-    uint64_t *red_full = xready + 2, *red_empty = red_full + 2;
-    volatile int *abort_flag = (volatile int *)(red_empty + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t b = blockIdx.x;
-    X += b * sX;
-    const float *Db = Dinv + b * nb * 2 * TB * TB;
-
-    for (int e = tid; e < n * NC; e += STR_THREADS) {
-        const int i = e % n, c = e / n;
-        r[i * NC + c] = c < m ? ld(X, planeX, (int64_t)c * ldx + i) : fmk(0.f, 0.f);
-    }
-    if (tid == 0) {
-        for (int q = 0; q < S; ++q) {
-            sbar_init(s_u32(&full[q]), 1);
-            sbar_init(s_u32(&empty[q]), STR_CONS);
-        }
-        for (int q = 0; q < 2; ++q) {
-            sbar_init(s_u32(&dfull[q]), 1);
-            sbar_init(s_u32(&dempty[q]), 1);
-            sbar_init(s_u32(&xready[q]), 1);
-            sbar_init(s_u32(&red_full[q]), STR_CONS / 2);
-            sbar_init(s_u32(&red_empty[q]), STR_CONS / 2);
-        }
-        sbar_init(s_u32(rows_ready), STR_ROWS);
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-
-    // tile t of block j: first row and row range [lo, hi) that the block updates
-    auto range = [&](int j, int &lo, int &hi) {
-        if (lower) {
-            lo = (j + 1) * TB;
-            hi = n;
-        } else {
-            lo = 0;
-            hi = j * TB;
-        }
-        if (lo > hi) lo = hi;
-    };
-    auto tile_row = [&](int lo, int hi, int t) {
-        return lower ? lo + t * STR_ROWS : hi - (t + 1) * STR_ROWS;
-    };
-    auto fail = [&](int code) {
-        atomicCAS(&g_trsv_error, 0, code);
-        *abort_flag = 1;
-    };
-
-    if (warp == 9) {
-        if (lane == 0) {
-            uint32_t g = 0;
-            // the inverse of block jj's diagonal block; block jj + 1's is
-            // requested right after the first tile of block jj, so that the
-            // diagonal solve never waits for it
-            auto load_dinv = [&](int jj) -> bool {
-                const int j = lower ? jj : nb - 1 - jj, buf = jj & 1;
-                if (jj >= 2 && !sbar_wait(s_u32(&dempty[buf]), ((jj - 2) >> 1) & 1)) {
-                    fail(11);
-                    return false;
-                }
-                sbar_expect(s_u32(&dfull[buf]), 2 * TB * TB * 4);
-                s_bulk(s_u32(dsm + buf * 2 * TB * TB), Db + (int64_t)j * 2 * TB * TB,
-                       2 * TB * TB * 4, s_u32(&dfull[buf]));
-                return true;
-            };
-            bool ok = load_dinv(0);
-            for (int jj = 0; jj < nb && ok && !*abort_flag; ++jj) {
-                const int j = lower ? jj : nb - 1 - jj;
-                int lo, hi;
-                range(j, lo, hi);
-                const int nt = (hi - lo + STR_ROWS - 1) / STR_ROWS;
-                for (int t = 0; t < nt; ++t, ++g) {
-                    const int q = g % S;
-                    if (g >= (uint32_t)S && !sbar_wait(s_u32(&empty[q]), ((g / S) - 1) & 1)) {
-                        fail(12);
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = s_u32(ring) + q * STR_TILE_BYTES;
-                    sbar_expect(s_u32(&full[q]), STR_TILE_BYTES);
-                    s_tma3(dst, &tmRe, s_u32(&full[q]), tile_row(lo, hi, t), j * TB, (int)b);
-                    s_tma3(dst + STR_TILE_BYTES / 2, &tmIm, s_u32(&full[q]), tile_row(lo, hi, t),
-                           j * TB, (int)b);
-                    if (t == 0 && jj + 1 < nb && !load_dinv(jj + 1)) {
-                        ++g;
-                        ok = false;
-                        break;
-                    }
-                }
-            }
-            // copies still in flight (only after an abort): wait for them, bounded
-            if (*abort_flag) {
-                const uint32_t first = g > (uint32_t)S ? g - S : 0;
-                for (uint32_t h = first; h < g; ++h)
-                    sbar_wait(s_u32(&full[h % S]), (h / S) & 1);
-                for (int q = 0; q < 2 && q < nb; ++q) {
-                    // last use of each inverse buffer: jl = largest block index with jl % 2 == q
-                    const int jl = ((nb - 1 - q) / 2) * 2 + q;
-                    sbar_wait(s_u32(&dfull[q]), (jl >> 1) & 1);
-                }
-            }
-        }
-    } else if (warp == 8) {
-        for (int jj = 0; jj < nb && !*abort_flag; ++jj) {
-            const int j = lower ? jj : nb - 1 - jj, buf = jj & 1;
-            const int r0 = j * TB, rows = min(TB, n - r0);
-            if (jj >= 1 && !sbar_wait(s_u32(rows_ready), (jj - 1) & 1)) {
-                if (lane == 0) fail(13);
-                break;
-            }
-            if (!sbar_wait(s_u32(&dfull[buf]), (jj >> 1) & 1)) {
-                if (lane == 0) fail(14);
-                break;
-            }
-            const float *Dr = dsm + buf * 2 * TB * TB, *Di = Dr + TB * TB;
-            cf *xo = xb + buf * TB * NC;
-            cf y[NC];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) y[c] = fmk(0.f, 0.f);
-            if (lane < rows) {
-#pragma unroll 4
-                for (int k = 0; k < rows; ++k) {
-                    const cf d = fmk(Dr[k * TB + lane], Di[k * TB + lane]);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const cf v = r[(r0 + k) * NC + c];
-                        y[c].x = fmaf(d.x, v.x, y[c].x);
-                        y[c].x = fmaf(-d.y, v.y, y[c].x);
-                        y[c].y = fmaf(d.x, v.y, y[c].y);
-                        y[c].y = fmaf(d.y, v.x, y[c].y);
-                    }
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                if (c >= m) y[c] = fmk(0.f, 0.f);
-                if (lane < rows && c < m) st(X, planeX, (int64_t)c * ldx + r0 + lane, y[c]);
-                xo[lane * NC + c] = y[c];
-            }
-            __syncwarp();
-            if (lane == 0) {
-                sbar_arrive(s_u32(&xready[buf]));
-                sbar_arrive(s_u32(&dempty[buf]));
-            }
-        }
-    } else {
-        // warps 0-7: row tid % 128 of each tile, columns [16 h, 16 h + 16), h = tid / 128
-        const int row = tid & (STR_ROWS - 1), h = tid >> 7;
-        uint32_t g = 0;
-        for (int jj = 0; jj < nb && !*abort_flag; ++jj) {
-            const int j = lower ? jj : nb - 1 - jj, buf = jj & 1;
-            if (!sbar_wait(s_u32(&xready[buf]), (jj >> 1) & 1)) {
-                fail(15);
-                break;
-            }
-            const cf *xj = xb + buf * TB * NC;
-            int lo, hi;
-            range(j, lo, hi);
-            const int nt = (hi - lo + STR_ROWS - 1) / STR_ROWS;
-            bool ok = true;
-            for (int t = 0; t < nt; ++t, ++g) {
-                const int q = g % S;
-                if (!sbar_wait(s_u32(&full[q]), (g / S) & 1)) {
-                    fail(16);
-                    ok = false;
-                    break;
-                }
-                const float *tr = ring + (size_t)q * (STR_TILE_BYTES / 4), *ti = tr + TB * STR_ROWS;
-                cf acc[NC];
-#pragma unroll
-                for (int c = 0; c < NC; ++c) acc[c] = fmk(0.f, 0.f);
-#pragma unroll
-                for (int kk = 0; kk < TB / 2; ++kk) {
-                    const int k = 16 * h + kk;
-                    const float ar = tr[k * STR_ROWS + row], ai = ti[k * STR_ROWS + row];
-                    cf x[NC];
-                    if (NC % 2 == 0) {
-#pragma unroll
-                        for (int c = 0; c < NC; c += 2) {
-                            const float4 v = *reinterpret_cast<const float4 *>(xj + k * NC + c);
-                            x[c] = fmk(v.x, v.y);
-                            x[c + 1] = fmk(v.z, v.w);
-                        }
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) x[c] = xj[k * NC + c];
-                    }
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        acc[c].x = fmaf(ar, x[c].x, acc[c].x);
-                        acc[c].x = fmaf(-ai, x[c].y, acc[c].x);
-                        acc[c].y = fmaf(ar, x[c].y, acc[c].y);
-                        acc[c].y = fmaf(ai, x[c].x, acc[c].y);
-                    }
-                }
-                sbar_arrive(s_u32(&empty[q]));   // this thread's reads of the tile are done
-                // second half -> first half through a double buffer (bounded waits)
-                const int rbuf = g & 1;
-                cf *rb = red + rbuf * STR_ROWS * NC;
-                if (h == 1) {
-                    if (g >= 2 && !sbar_wait(s_u32(&red_empty[rbuf]), ((g >> 1) - 1) & 1)) {
-                        fail(17);
-                        ok = false;
-                        break;
-                    }
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) rb[row * NC + c] = acc[c];
-                    sbar_arrive(s_u32(&red_full[rbuf]));
-                } else {
-                    if (!sbar_wait(s_u32(&red_full[rbuf]), (g >> 1) & 1)) {
-                        fail(18);
-                        ok = false;
-                        break;
-                    }
-                    const int i = tile_row(lo, hi, t) + row;
-                    cf o[NC];
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) o[c] = rb[row * NC + c];
-                    sbar_arrive(s_u32(&red_empty[rbuf]));
-                    if (i >= lo && i < hi) {
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            cf &u = r[i * NC + c];
-                            u.x -= acc[c].x + o[c].x;
-                            u.y -= acc[c].y + o[c].y;
-                        }
-                    }
-                    if (t == 0 && jj < nb - 1) sbar_arrive(s_u32(rows_ready));
-                }
-            }
-            if (!ok) break;
-        }
-    }
-}
-
 __global__ void set_identity_kernel(float *W, int64_t ldw, int64_t plane, int64_t sW, int n) {
     const int64_t b = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1972,10 +1482,6 @@ int right_solve(Ctx &c, int n, int m, CMatF LU, const int32_t *ipiv, int64_t sP,
 }
 
 // ---- few-RHS solves ---------------------------------------------------------
-int64_t trsv_state_bytes(int n, int batch) {
-    return ((int64_t)ceil_div(n, TB) * batch + 64) * sizeof(int);
-}
-
 int64_t diag_inv_floats(int n, int batch) { return (int64_t)batch * ceil_div(n, TB) * 2 * TB * TB; }
 
 int diag_inv(Ctx &c, int n, CMatF LU, float *invL, float *invU) {
@@ -1989,104 +1495,67 @@ int diag_inv(Ctx &c, int n, CMatF LU, float *invL, float *invU) {
     return MNPB_OK;
 }
 
-// state: caller-provided device scratch of trsv_state_bytes(n, batch) bytes
-// (flags per block and the ticket counter), cleared before each launch.
 template <int NC>
-static int trsv_rl(Ctx &c, bool lower, int n, int m, CMatF T, const float *inv, CMatF X) {
-    const int nb = ceil_div(n, TB);
-    const int dyn = n * NC * (int)sizeof(cf);
-    if (dyn > 48 * 1024) MNPB_TRY(smem_opt_in(trsv_rl_kernel<NC>, dyn, "trsv_rl_kernel"));
-    ProfScope ps(c.s, PC_TRSV, 4.0 * (double)n * n * c.batch);   // bytes of the triangle
-    prof_tag("n=%d m=%d B=%d %s", n, m, c.batch, lower ? "L" : "U");
-    trsv_rl_kernel<NC><<<c.batch, RL_THREADS, dyn, c.s>>>(n, m, lower ? 1 : 0, T.p, T.ld, T.plane,
-                                                         T.stride, inv, X.p, X.ld, X.plane,
-                                                         X.stride, nb);
-    MNPB_LAUNCH_CHECK("trsv_rl_kernel");
-    return MNPB_OK;
-}
-
-// Shared memory of trsv_stream_kernel<NC> with S ring stages (0 if too large).
-static int stream_smem(int n, int nc, int S) {
-    const int64_t b = 1024 + (int64_t)S * STR_TILE_BYTES + 2 * 2 * TB * TB * 4 +
-                      2 * TB * nc * (int64_t)sizeof(cf) + 2 * STR_ROWS * nc * (int64_t)sizeof(cf) +
-                      (int64_t)n * nc * sizeof(cf) + (2 * S + 11) * 8 + 16;
-    return b <= 220 * 1024 ? (int)b : 0;
-}
-
-template <int NC>
-static int trsv_stream(Ctx &c, bool lower, int n, int m, CMatF T, const float *inv, CMatF X,
-                       int S) {
-    const int nb = ceil_div(n, TB);
-    const int smem = stream_smem(n, NC, S);
-    MNPB_TRY(smem_opt_in(trsv_stream_kernel<NC>, smem, "trsv_stream_kernel"));
-    CUtensorMap mr, mi;
-    const uint64_t dims[3] = {(uint64_t)n, (uint64_t)n, (uint64_t)c.batch};
-    const uint64_t strides[2] = {(uint64_t)T.ld * 4, (uint64_t)T.stride * 4};
-    const uint32_t box[3] = {STR_ROWS, TB, 1};
-    MNPB_TRY(tc::encode_map_f32(&mr, T.p, dims, strides, box, 0));
-    MNPB_TRY(tc::encode_map_f32(&mi, T.p + T.plane, dims, strides, box, 0));
-    ProfScope ps(c.s, PC_TRSV, 4.0 * (double)n * n * c.batch);   // bytes of the triangle
-    prof_tag("n=%d m=%d B=%d %s stream", n, m, c.batch, lower ? "L" : "U");
-    trsv_stream_kernel<NC><<<c.batch, STR_THREADS, smem, c.s>>>(
-        mr, mi, n, m, lower ? 1 : 0, inv, X.p, X.ld, X.plane, X.stride, nb, S);
-    MNPB_LAUNCH_CHECK("trsv_stream_kernel");
-    return MNPB_OK;
-}
-
-static int trsv(Ctx &c, bool lower, int n, int m, CMatF T, const float *inv, CMatF X,
-                int *state) {
-    // triangle streamed by TMA when it is 16-byte aligned and the ring fits
-    // beside the right-hand sides in shared memory
-    const bool a16 = ((uintptr_t)T.p & 15) == 0 && T.ld % 4 == 0 && T.plane % 4 == 0 &&
-                     T.stride % 4 == 0 && ((uintptr_t)inv & 15) == 0;
-    if (a16 && m <= 4) {
-        const int nc = m <= 1 ? 1 : 4;
-        int S = 6;
-        while (S >= 2 && stream_smem(n, nc, S) == 0) --S;
-        if (S >= 2)
-            return nc == 1 ? trsv_stream<1>(c, lower, n, m, T, inv, X, S)
-                           : trsv_stream<4>(c, lower, n, m, T, inv, X, S);
-    }
-    // one CTA per matrix when the right-hand sides fit in shared memory and
-    // the triangle allows 8-byte row-pair loads
-    const bool even = ((uintptr_t)T.p & 7) == 0 && T.ld % 2 == 0 && T.plane % 2 == 0 &&
-                      T.stride % 2 == 0;
-    if (even && m <= 8) {
-        const int nc = m <= 1 ? 1 : m <= 4 ? 4 : 8;
-        if ((int64_t)n * nc * (int64_t)sizeof(cf) <= 200 * 1024) {
-            if (nc == 1) return trsv_rl<1>(c, lower, n, m, T, inv, X);
-            if (nc == 4) return trsv_rl<4>(c, lower, n, m, T, inv, X);
-            return trsv_rl<8>(c, lower, n, m, T, inv, X);
+static int getrs_few_nc(Ctx &c, int n, int m, const trc::Groups &gr, CMatF LU,
+                        const int32_t *ipiv, int64_t sP, const float *invL, const float *invU,
+                        CMatF B, int C) {
+    const Planar::Mat A{LU.p, LU.ld, LU.plane, LU.stride}, X{B.p, B.ld, B.plane, B.stride};
+    const bool ride = trc::Smem<PlanarTri, NC>::composes(n);
+    if (!ride) {
+        Ctx ce(c.s, gr.per, c.work, c.work_bytes);
+        for (int g = 0; g < gr.groups; ++g) {
+            CMatF Bg = B;
+            Bg.p += g * gr.X;
+            MNPB_TRY(laswp(ce, Bg, 0, m, ipiv + g * gr.P, sP, 0, n, true));
         }
     }
-    const int nb = ceil_div(n, TB);
-    int *flags = state;
-    unsigned *ticket = (unsigned *)(state + (int64_t)nb * c.batch);
-    if (cudaMemsetAsync(state, 0, trsv_state_bytes(n, c.batch), c.s) != cudaSuccess) {
-        set_error("trsv: memset failed");
-        return MNPB_ECUDA;
+    ProfScope ps(c.s, PC_TRSV, 8.0 * (double)n * n * gr.per * gr.groups);   // both triangles
+    prof_tag("n=%d m=%d B=%d C=%d", n, m, gr.per * gr.groups, C);
+    MNPB_TRY((trc::launch_trsv<PlanarTri, NC>(c.s, true, true, n, m, gr, A, invL, X,
+                                              ride ? ipiv : nullptr, sP, C)));
+    return trc::launch_trsv<PlanarTri, NC>(c.s, false, false, n, m, gr, A, invU, X, nullptr, 0, C);
+}
+
+// 1: done (status in rc), 0: too many columns
+static int getrs_few_groups(Ctx &c, int n, int m, const trc::Groups &gr, CMatF LU,
+                            const int32_t *ipiv, int64_t sP, const float *invL,
+                            const float *invU, CMatF B, int &rc) {
+    if (m > 16) return 0;
+    const int64_t units = (int64_t)gr.per * gr.groups;
+    // the widest instance whose right-hand sides fit in shared memory; fewer
+    // columns per cluster (and the triangle read once for each) beyond that
+#define MNPB_FEW(NC)                                                                         \
+    if (const int C = trc::cluster_size<PlanarTri, NC>(n, units * ceil_div(m, NC))) {        \
+        rc = getrs_few_nc<NC>(c, n, m, gr, LU, ipiv, sP, invL, invU, B, C);                  \
+        return 1;                                                                            \
     }
-    const int grid = nb * c.batch;
-    ProfScope ps(c.s, PC_TRSV, 4.0 * (double)n * n * c.batch);   // bytes of the triangle
-    prof_tag("n=%d m=%d B=%d %s", n, m, c.batch, lower ? "L" : "U");
-#define MNPB_TRSV(NC)                                                                          \
-    trsv_kernel<NC><<<grid, 256, 0, c.s>>>(n, m, lower ? 1 : 0, T.p, T.ld, T.plane, T.stride,   \
-                                           inv, X.p, X.ld, X.plane, X.stride, flags, ticket, 1, \
-                                           nb, c.batch)
-    if (m <= 4) MNPB_TRSV(4);
-    else if (m <= 8) MNPB_TRSV(8);
-    else MNPB_TRSV(16);
-#undef MNPB_TRSV
-    MNPB_LAUNCH_CHECK("trsv_kernel");
-    return MNPB_OK;
+    if (m > 8) MNPB_FEW(12);
+    if (m > 4) MNPB_FEW(8);
+    if (m > 1) MNPB_FEW(4);
+    MNPB_FEW(1);
+#undef MNPB_FEW
+    return 0;
 }
 
 int getrs_few(Ctx &c, int n, int m, CMatF LU, const int32_t *ipiv, int64_t sP,
-              const float *invL, const float *invU, CMatF B, int *state) {
-    if (m > 16) return getrs(c, n, m, LU, ipiv, sP, B);
-    MNPB_TRY(laswp(c, B, 0, m, ipiv, sP, 0, n, true));
-    MNPB_TRY(trsv(c, true, n, m, LU, invL, B, state));
-    return trsv(c, false, n, m, LU, invU, B, state);
+              const float *invL, const float *invU, CMatF B) {
+    const trc::Groups gr{c.batch, 1, 0, 0, 0, 0};
+    int rc = MNPB_OK;
+    if (getrs_few_groups(c, n, m, gr, LU, ipiv, sP, invL, invU, B, rc)) return rc;
+    return getrs(c, n, m, LU, ipiv, sP, B);
+}
+
+int getrs_few_pair(Ctx &c, int n, int m, CMatF LU, const float *LU2, const int32_t *ipiv,
+                   const int32_t *ipiv2, int64_t sP, const float *invL, const float *invU,
+                   int64_t inv2, CMatF B, int64_t b2) {
+    const trc::Groups gr{c.batch, 2, LU2 - LU.p, inv2, b2, ipiv2 - ipiv};
+    int rc = MNPB_OK;
+    if (getrs_few_groups(c, n, m, gr, LU, ipiv, sP, invL, invU, B, rc)) return rc;
+    MNPB_TRY(getrs(c, n, m, LU, ipiv, sP, B));
+    CMatF L2 = LU, B2 = B;
+    L2.p = (float *)LU2;
+    B2.p += b2;
+    return getrs(c, n, m, L2, ipiv2, sP, B2);
 }
 
 // Failure-path probe of the triangular solves' two wait helpers: kind 1

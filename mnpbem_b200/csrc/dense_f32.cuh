@@ -35,14 +35,17 @@ int lu_inverse(Ctx &c, int n, tc::CMatF LU, const int32_t *ipiv, int64_t sP, tc:
 // Inverses of the 32 x 32 diagonal blocks of an LU factor (for getrs_few).
 int64_t diag_inv_floats(int n, int batch);
 int diag_inv(Ctx &c, int n, tc::CMatF LU, float *invL, float *invU);
-// LU solve for m <= 16 right-hand sides: row swaps + one launch per triangle.
-// state: device scratch of trsv_state_bytes(n, batch) bytes (per stream).
-int64_t trsv_state_bytes(int n, int batch);
+// LU solve for m <= 16 right-hand sides: one launch per triangle.
 int getrs_few(Ctx &c, int n, int m, tc::CMatF LU, const int32_t *ipiv, int64_t sP,
-              const float *invL, const float *invU, tc::CMatF B, int *state);
+              const float *invL, const float *invU, tc::CMatF B);
+// Two sets of factors (the second's inverses inv2 floats on) and right-hand
+// sides (b2 floats on) in one launch per triangle.
+int getrs_few_pair(Ctx &c, int n, int m, tc::CMatF LU, const float *LU2, const int32_t *ipiv,
+                   const int32_t *ipiv2, int64_t sP, const float *invL, const float *invU,
+                   int64_t inv2, tc::CMatF B, int64_t b2);
 int trsv_error_read_and_clear(cudaStream_t s, int *code);
-// One-thread kernel whose wait (kind 1: flag spin, kind 2: mbarrier) of the
-// triangular solves can only time out after limit_ns; records code 9.
+// One-thread kernel whose wait (kind 1: flag spin, kind 2: mbarrier) can only
+// time out after limit_ns; records code 9 in the error word.
 int trsv_wait_probe(cudaStream_t s, int kind, int *flag, uint64_t limit_ns);
 
 }  // namespace f32

@@ -815,28 +815,52 @@ static int permute_rows(cudaStream_t s, cd *B, int64_t ldb, int64_t sB, int n, i
 // Forward then backward solve of up to 16 right-hand sides, a cluster per
 // matrix and NC columns; the interchanges ride along with the forward solve.
 template <int NC>
-static int getrs_few(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda,
-                     int64_t sA, const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB,
-                     int C) {
+static int getrs_few(cudaStream_t s, int n, int nrhs, const trc::Groups &gr, const cd *LU,
+                     int64_t lda, int64_t sA, const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb,
+                     int64_t sB, int C) {
     const trc::F64::Mat A{(cd *)LU, lda, sA}, X{B, ldb, sB};
     const bool ride = trc::Smem<trc::F64, NC>::composes(n);
-    if (!ride) MNPB_TRY(laswp(s, B, ldb, sB, nrhs, 0, 0, ipiv, sP, 0, n, true, batch));
-    ProfScope ps(s, PC_TRSV, 16.0 * (double)n * n * batch);   // bytes of both triangles
-    MNPB_TRY((trc::launch_trsv<trc::F64, NC>(s, true, true, n, nrhs, batch, A, nullptr, X,
+    if (!ride)
+        for (int g = 0; g < gr.groups; ++g)
+            MNPB_TRY(laswp(s, B + g * gr.X, ldb, sB, nrhs, 0, 0, ipiv + g * gr.P, sP, 0, n, true,
+                           gr.per));
+    ProfScope ps(s, PC_TRSV, 16.0 * (double)n * n * gr.per * gr.groups);   // both triangles
+    MNPB_TRY((trc::launch_trsv<trc::F64, NC>(s, true, true, n, nrhs, gr, A, nullptr, X,
                                              ride ? ipiv : nullptr, sP, C)));
-    return trc::launch_trsv<trc::F64, NC>(s, false, false, n, nrhs, batch, A, nullptr, X, nullptr,
-                                          0, C);
+    return trc::launch_trsv<trc::F64, NC>(s, false, false, n, nrhs, gr, A, nullptr, X, nullptr, 0,
+                                          C);
+}
+
+// Clusters of the few-column solves of `batch` matrices: NC = 1 or 4 columns
+// each, C CTAs; false if the columns are too many or do not fit.
+static bool few_shape(int n, int nrhs, int64_t batch, int &NC, int &C) {
+    if (nrhs > 16) return false;
+    NC = nrhs == 1 ? 1 : 4;
+    C = NC == 1 ? trc::cluster_size<trc::F64, 1>(n, batch)
+                : trc::cluster_size<trc::F64, 4>(n, batch * ceil_div(nrhs, 4));
+    return C > 0;
+}
+
+int getrs_pair(cudaStream_t s, int n, int nrhs, int batch, const cd *LU1, const cd *LU2,
+               int64_t lda, int64_t sA, const int32_t *piv1, const int32_t *piv2, int64_t sP,
+               cd *B1, cd *B2, int64_t ldb, int64_t sB) {
+    int NC, C;
+    if (!few_shape(n, nrhs, 2 * (int64_t)batch, NC, C)) {
+        MNPB_TRY(getrs(s, n, nrhs, batch, LU1, lda, sA, piv1, sP, B1, ldb, sB));
+        return getrs(s, n, nrhs, batch, LU2, lda, sA, piv2, sP, B2, ldb, sB);
+    }
+    const trc::Groups gr{batch, 2, LU2 - LU1, 0, B2 - B1, piv2 - piv1};
+    return NC == 1 ? getrs_few<1>(s, n, nrhs, gr, LU1, lda, sA, piv1, sP, B1, ldb, sB, C)
+                   : getrs_few<4>(s, n, nrhs, gr, LU1, lda, sA, piv1, sP, B1, ldb, sB, C);
 }
 
 int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda, int64_t sA,
           const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB) {
-    if (nrhs <= 16) {
-        const int C1 = trc::cluster_size<trc::F64, 1>(n, batch);
-        const int C4 = trc::cluster_size<trc::F64, 4>(n, (int64_t)batch * ceil_div(nrhs, 4));
-        if (nrhs == 1 && C1 > 0)
-            return getrs_few<1>(s, n, nrhs, batch, LU, lda, sA, ipiv, sP, B, ldb, sB, C1);
-        if (nrhs > 1 && C4 > 0)
-            return getrs_few<4>(s, n, nrhs, batch, LU, lda, sA, ipiv, sP, B, ldb, sB, C4);
+    int NC, C;
+    if (few_shape(n, nrhs, batch, NC, C)) {
+        const trc::Groups gr{batch, 1, 0, 0, 0, 0};
+        return NC == 1 ? getrs_few<1>(s, n, nrhs, gr, LU, lda, sA, ipiv, sP, B, ldb, sB, C)
+                       : getrs_few<4>(s, n, nrhs, gr, LU, lda, sA, ipiv, sP, B, ldb, sB, C);
     }
     MNPB_TRY(permute_rows(s, B, ldb, sB, n, nrhs, ipiv, sP, batch));
     MNPB_TRY(trsm_llu(s, n, nrhs, batch, LU, lda, sA, B, ldb, sB));

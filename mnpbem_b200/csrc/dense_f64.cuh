@@ -21,6 +21,11 @@ int getrf(cudaStream_t s, int n, int batch, cd *A, int64_t lda, int64_t sA, int3
           int64_t sP, int32_t *info);
 int getrs(cudaStream_t s, int n, int nrhs, int batch, const cd *LU, int64_t lda, int64_t sA,
           const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB);
+// The same solve with two sets of factors and right-hand sides, in one launch
+// per triangle where the columns are few.
+int getrs_pair(cudaStream_t s, int n, int nrhs, int batch, const cd *LU1, const cd *LU2,
+               int64_t lda, int64_t sA, const int32_t *piv1, const int32_t *piv2, int64_t sP,
+               cd *B1, cd *B2, int64_t ldb, int64_t sB);
 int right_solve(cudaStream_t s, int n, int m, int batch, const cd *LU, int64_t lda, int64_t sA,
                 const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB);
 // X <- A^-1 from getrf's factors.

@@ -23,6 +23,11 @@
 // 5.31 -> 0.75 / 0.96 ms; 1365, 12 columns 2.49 -> 0.40; 284, 1 column 452 ->
 // 71 us, 41 matrices 4 columns 486 -> 86 us; 41 x 1148, 3 columns 2.48 -> 0.53.
 //
+// FP32 (two block rows per update, the diagonal blocks through their halves'
+// inverses, G1 and G2 in one launch) against the solves it replaces, per
+// triangle: 2884, 4 columns 1.05 -> 0.16 ms for one matrix, 1.06 -> 0.41 ms for
+// 27; 12 columns, 13 to 26 matrices of 284 to 2044 rows 0.78 -> 0.14 ms.
+//
 // An upper triangle is solved as a lower one with blocks and rows in reverse
 // order; "logical" indices below count in the order of the solve.
 #pragma once
@@ -45,6 +50,7 @@ struct F64 : lup::F64 {
     typedef lup::F64::Mat Mat;
     // staged diagonal block: the triangle in logical order, column by column
     static constexpr int DELEMS = NB * NB;
+    static constexpr int P = 1;      // block rows per update
     static __device__ __forceinline__ V fma(V a, V b, V c) { return cfma(a, b, c); }
     static __device__ __forceinline__ V shfl(V v, int l) {
         return cmk(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
@@ -93,6 +99,14 @@ struct F64 : lup::F64 {
             r1 = cmul(r1, i1);
         }
     }
+};
+
+// Systems of one launch: `groups` sets of `per` entries, the sets' triangles,
+// inverses, right-hand sides and pivots these offsets (elements) apart.  G1
+// and G2 of the BEM solve go through one launch this way.
+struct Groups {
+    int per, groups;
+    int64_t A, D, X, P;
 };
 
 template <typename T, int NC>
@@ -155,8 +169,8 @@ __device__ __forceinline__ void compose(int *w, const int32_t *ipiv, int n) {
 template <typename T, int NC>
 __global__ void __launch_bounds__(THREADS, 1)
     trsv_kernel(int n, int m, int lower_, int unit_, typename T::Mat A,
-                const float *__restrict__ Dinv, typename T::Mat X, const int32_t *ipiv,
-                int64_t sP, int C, int chunks) {
+                const float *Dinv, typename T::Mat X, const int32_t *ipiv, int64_t sP, int C,
+                int chunks, Groups gr_) {
     typedef typename T::V V;
     constexpr int XS = Smem<T, NC>::XS;
     extern __shared__ __align__(16) unsigned char trc_sm[];
@@ -168,7 +182,14 @@ __global__ void __launch_bounds__(THREADS, 1)
     const bool lower = lower_, unit = unit_;
     const int me = C > 1 ? (int)lup::cluster_rank() : 0;
     const int64_t unitid = blockIdx.x / C;
-    const int64_t b = unitid / chunks;
+    const int64_t b = (unitid / chunks) % gr_.per;
+    {
+        const int64_t g = (unitid / chunks) / gr_.per;
+        A.A += g * gr_.A;
+        X.A += g * gr_.X;
+        Dinv += g * gr_.D;
+        if (ipiv) ipiv += g * gr_.P;
+    }
     const int c0 = (int)(unitid % chunks) * NC;
     const int mc = min(NC, m - c0);
     const int nb = (n + NB - 1) / NB;
@@ -212,44 +233,60 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     };
-    // tile (i, k): 16 entries per thread (row rl, columns 4 kk + q)
-    auto fetch = [&](int i, int k, V (&t)[16]) {
-        const int gr = phys(i) * NB + rl;
+    // tiles (i, k), (i + C, k), ...: 16 entries of each per thread (row rl,
+    // columns 4 kk + q); P tiles together share the reads of x
+    constexpr int P = T::P;
+    auto fetch = [&](int i, int k, V (&t)[P][16]) {
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            const int gc = phys(k) * NB + 4 * kk + q;
-            t[kk] = (gr < n && gc < n) ? T::load(A, b, gr, gc) : T::zero();
+        for (int p = 0; p < P; ++p) {
+            const bool on = i + p * C < nb;
+            const int gr = on ? phys(i + p * C) * NB + rl : n;
+#pragma unroll
+            for (int kk = 0; kk < 16; ++kk) {
+                const int gc = phys(k) * NB + 4 * kk + q;
+                t[p][kk] = (gr < n && gc < n) ? T::load(A, b, gr, gc) : T::zero();
+            }
         }
     };
-    auto update = [&](int i, int k, const V (&t)[16]) {
+    auto update = [&](int i, int k, const V (&t)[P][16]) {
         const V *x = xs + (k % 3) * NB * XS;
-        V acc[NC];
+        V acc[P][NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = T::zero();
+        for (int p = 0; p < P; ++p)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[p][c] = T::zero();
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
 #pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const V xv = x[(4 * kk + q) * XS + c];
+#pragma unroll
+                for (int p = 0; p < P; ++p) acc[p][c] = T::fma(t[p][kk], xv, acc[p][c]);
+            }
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            if (i + p * C >= nb) break;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                acc[p][c] = T::add(acc[p][c], T::shfl_xor(acc[p][c], 8));
+                acc[p][c] = T::add(acc[p][c], T::shfl_xor(acc[p][c], 16));
+            }
+            V *r = rs + (((i - me) / C + p) * NB + rl) * NC;
+#pragma unroll
             for (int c = 0; c < NC; ++c)
-                acc[c] = T::fma(t[kk], x[(4 * kk + q) * XS + c], acc[c]);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            acc[c] = T::add(acc[c], T::shfl_xor(acc[c], 8));
-            acc[c] = T::add(acc[c], T::shfl_xor(acc[c], 16));
+                if ((c & 3) == q) r[c] = T::sub(r[c], acc[p][c]);
         }
-        V *r = rs + (((i - me) / C) * NB + rl) * NC;
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-            if ((c & 3) == q) r[c] = T::sub(r[c], acc[c]);
     };
 
-    V cur[16];
-    // the tiles in the order of their use: column k, owned block rows i > k ascending
-    int ti = me, tk = 0;             // next tile to fetch
+    V cur[P][16];
+    // the tiles in the order of their use: column k, owned block rows i > k
+    // ascending, P at a time
+    int ti = me, tk = 0;             // next tiles to fetch
     auto first_row = [&](int k) { return k + 1 + ((me - (k + 1)) % C + C) % C; };
     ti = first_row(0);
     auto valid = [&]() { return ti < nb; };
     auto advance = [&]() {
-        ti += C;
+        ti += P * C;
         if (ti >= nb) {
             ++tk;
             ti = first_row(tk);
@@ -268,15 +305,15 @@ __global__ void __launch_bounds__(THREADS, 1)
             T::stage(D, A, Dinv, b, n, phys(staged), lower, tid);
         }
         const bool next_mine = k + 1 < nb && (k + 1) % C == me;
-        V nxt[16];
+        V nxt[P][16];
         if (next_mine) {
-            // tile (k + 1, k) is the first of this column
+            // tile (k + 1, k) is among the first of this column
             const int i = ti;
             advance();
             if (valid()) fetch(ti, tk, nxt);
             update(i, k, cur);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) cur[e] = nxt[e];
+            for (int e = 0; e < P * 16; ++e) cur[e / 16][e % 16] = nxt[e / 16][e % 16];
             __syncthreads();         // rows of block k + 1 and its staged diagonal complete
             solve(k + 1, (k + 1) / C);
         }
@@ -287,7 +324,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (valid()) fetch(ti, tk, nxt);
             update(i, k, cur);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) cur[e] = nxt[e];
+            for (int e = 0; e < P * 16; ++e) cur[e / 16][e % 16] = nxt[e / 16][e % 16];
         }
     }
 }
@@ -305,14 +342,14 @@ int cluster_size(int n, int64_t units) {
 }
 
 template <typename T, int NC>
-int launch_trsv(cudaStream_t s, bool lower, bool unit, int n, int m, int batch,
+int launch_trsv(cudaStream_t s, bool lower, bool unit, int n, int m, const Groups &gr,
                 typename T::Mat A, const float *Dinv, typename T::Mat X, const int32_t *ipiv,
                 int64_t sP, int C) {
     const int chunks = ceil_div(m, NC);
     const int smem = (int)Smem<T, NC>::bytes(n, C);
     MNPB_TRY(smem_opt_in(trsv_kernel<T, NC>, smem, "trc::trsv_kernel"));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(batch * chunks * C));
+    cfg.gridDim = dim3((unsigned)(gr.per * gr.groups * chunks * C));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
@@ -324,7 +361,7 @@ int launch_trsv(cudaStream_t s, bool lower, bool unit, int n, int m, int batch,
     cfg.attrs = at;
     cfg.numAttrs = C > 1 ? 1 : 0;
     if (cudaLaunchKernelEx(&cfg, trsv_kernel<T, NC>, n, m, lower ? 1 : 0, unit ? 1 : 0, A, Dinv,
-                           X, ipiv, sP, C, chunks) != cudaSuccess) {
+                           X, ipiv, sP, C, chunks, gr) != cudaSuccess) {
         set_error("triangular solve: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         return MNPB_ECUDA;
     }

@@ -1,5 +1,6 @@
 """FP32 (TF32-stored) LU panels at the sizes where the kernel changes: one or
-two rows per thread of a cluster, the shared-memory slab of large batches."""
+two rows per thread of a cluster, the shared-memory slab of large batches; and
+the mixed solve over the widths of its few-column kernels."""
 import numpy as np
 import pytest
 import torch
@@ -68,3 +69,70 @@ def test_lu_planar_zero_column(gpu_ok):
     assert torch.equal(LU, A)
     assert info.cpu().tolist() == [0, 41]
     assert np.array_equal(piv.cpu().numpy(), np.tile(np.arange(n), (2, 1)))
+
+
+@pytest.mark.parametrize('n,batch,K', [(40, 2, 1), (64, 1, 2), (65, 3, 4), (97, 1, 3), (200, 5, 1),
+                                       (331, 40, 3), (700, 1, 2)])
+def test_mixed_solve_matches_fp64(gpu_ok, n, batch, K):
+    """The mixed factorisation's solve, refined to 1e-12 of the solution, against
+    the FP64 solve of the same random systems: 1, 2, 3, 4 excitations use the
+    1-, 4-, 8- and 12-column solves and products.  Both converge to the solution
+    of the FP64 operator; their difference is bounded by the refinement's last
+    correction and the FP64 solve's own error n eps kappa, kappa < 1e4 for
+    these diagonally shifted matrices."""
+    rng = torch.Generator().manual_seed(n)
+    ld = (n + 3) // 4 * 4
+
+    def mat(scale, shift):
+        x = torch.randn((batch, n, n, 2), generator=rng, dtype=torch.float64) * scale / n ** 0.5
+        x[..., 0] += shift * torch.eye(n, dtype=torch.float64)
+        return torch.view_as_complex(x).cuda()
+
+    G1, G2, H1, H2 = mat(0.2, 1.0), mat(0.2, 1.3), mat(0.2, 2.0), mat(0.2, -2.0)
+    eps = torch.tensor([[-8.0, 1.0, 1.0, 0.0]], dtype=torch.float64, device='cuda') \
+        .repeat(batch, 1)
+    kvac = torch.full((batch,), 0.05, dtype=torch.float64, device='cuda')
+    nv = torch.randn((n, 3), generator=rng, dtype=torch.float64)
+    nv = (nv / nv.norm(dim=1, keepdim=True)).cuda()
+    b = torch.view_as_complex(torch.randn((batch, 8, K, n, 2), generator=rng,
+                                          dtype=torch.float64)).cuda()
+    L, sh = _lib.lib(), _lib.stream_handle()
+    # FP64
+    GG, HH = torch.stack([G1, G2]), torch.stack([H1, H2])
+    D = torch.empty_like(G1)
+    piv = torch.empty((3, batch, n), dtype=torch.int32, device='cuda')
+    info = torch.zeros((2, batch), dtype=torch.int32, device='cuda')
+    work = torch.empty(int(L.mnpb_bemret_workspace_f64(n, batch)), dtype=torch.uint8,
+                       device='cuda')
+    call('mnpb_bemret_init_f64', sh, n, batch, ptr(GG[0]), ptr(GG[1]), ptr(HH[0]), ptr(HH[1]),
+         ptr(D), n, n * n, ptr(eps), ptr(kvac), ptr(nv), 0, ptr(piv), ptr(info), ptr(work),
+         work.numel())
+    x64 = torch.empty_like(b)
+    wb = batch * n * 15 * K * 16
+    w64 = torch.empty(wb, dtype=torch.uint8, device='cuda')
+    call('mnpb_bemret_solve_f64', sh, n, batch, K, ptr(GG[0]), ptr(GG[1]), ptr(HH[0]),
+         ptr(HH[1]), ptr(D), n, n * n, ptr(piv), ptr(eps), ptr(kvac), ptr(nv), 0, ptr(b),
+         ptr(x64), ptr(w64), wb)
+    # mixed: padded FP64 operator and planar copies
+    pad = lambda A: torch.nn.functional.pad(torch.view_as_real(A), (0, 0, 0, ld - n))
+    ops = [torch.view_as_complex(pad(A).contiguous()) for A in (G1, G2, H1, H2)]
+    pl = [pad(A).permute(0, 3, 1, 2).float().contiguous() for A in (G1, G2, H1, H2)]
+    GGp, HHp = torch.stack(pl[:2]), torch.stack(pl[2:])
+    Dp = torch.empty_like(pl[0])
+    dinv = torch.empty(int(L.mnpb_bemret_dinv_floats(n, batch)), device='cuda')
+    wm = torch.empty(int(L.mnpb_bemret_workspace_mixed(n, batch)), dtype=torch.uint8,
+                     device='cuda')
+    call('mnpb_bemret_init_mixed', sh, n, batch, ptr(GGp[0]), ptr(GGp[1]), ptr(HHp[0]),
+         ptr(HHp[1]), ptr(Dp), ld, ptr(eps), ptr(kvac), ptr(nv), 0, ptr(piv), ptr(info),
+         ptr(dinv), ptr(wm), wm.numel())
+    assert not info.any()
+    x = torch.empty_like(b)
+    wr = torch.empty(int(L.mnpb_bemret_refine_workspace(n, batch, K)), dtype=torch.uint8,
+                     device='cuda')
+    iters, rel = np.zeros(batch, dtype=np.int32), np.zeros(batch)
+    call('mnpb_bemret_solve_refine', sh, n, batch, K, ptr(GGp[0]), ptr(GGp[1]), ptr(HHp[0]),
+         ptr(HHp[1]), ptr(Dp), ld, ptr(piv), ptr(dinv), ptr(ops[0]), ptr(ops[1]), ptr(ops[2]),
+         ptr(ops[3]), ptr(eps), ptr(kvac), ptr(nv), 0, ptr(b), ptr(x), 30, 1e-12, ptr(iters),
+         ptr(rel), ptr(wr), wr.numel())
+    err = (x - x64).flatten(1).norm(dim=1) / x64.flatten(1).norm(dim=1)
+    assert float(err.max()) <= 1e-11 + 1e4 * n * 2.0 ** -52
