@@ -11,6 +11,7 @@
 #include <vector>
 #include "bemret_kernels.cuh"
 #include "dense_f32.cuh"
+#include "skinny.cuh"
 
 #include <cmath>
 #include <vector>
@@ -84,60 +85,6 @@ __global__ void from_f32p(int n, int m, const float *Y, int64_t sy, cd *X, int64
     if (e >= (int64_t)n * m) return;
     const float *y = Y + b * sy;
     X[b * sx + e] = cmk((double)y[e], (double)y[e + (int64_t)n * m]);
-}
-
-// FP64 matrix times a few vectors: Y = A X, A n x n (c128, column-major),
-// X n x m (m <= NC <= 16).  A CTA covers 64 rows with 4 K-lanes (warp w reads
-// 32 consecutive rows of every 4th column, 512 B per load), so each matrix
-// element is read once and many loads are in flight; the lanes' partial sums
-// are reduced in shared memory.
-constexpr int ZS_KT = 32, ZS_ROWS = 64, ZS_KL = 4;
-template <int NC>
-__global__ void __launch_bounds__(256) zskinny_kernel(int n, int m, const cd *__restrict__ A,
-                                                      int64_t lda, int64_t sA,
-                                                      const cd *__restrict__ X, int64_t sX,
-                                                      cd *__restrict__ Y, int64_t sY) {
-    __shared__ cd Xs[ZS_KT][NC];
-    __shared__ cd part[ZS_KL][ZS_ROWS][NC];
-    const int64_t b = blockIdx.y;
-    A += b * sA;
-    X += b * sX;
-    Y += b * sY;
-    const int rl = threadIdx.x % ZS_ROWS, kl = threadIdx.x / ZS_ROWS;
-    const int row = blockIdx.x * ZS_ROWS + rl;
-    cd acc[NC];
-#pragma unroll
-    for (int j = 0; j < NC; ++j) acc[j] = cmk(0, 0);
-    for (int k0 = 0; k0 < n; k0 += ZS_KT) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < ZS_KT * NC; e += blockDim.x) {
-            const int kk = e % ZS_KT, j = e / ZS_KT;
-            Xs[kk][j] = (k0 + kk < n && j < m) ? X[(int64_t)j * n + k0 + kk] : cmk(0, 0);
-        }
-        __syncthreads();
-        if (row < n) {
-            const int kend = min(ZS_KT, n - k0);
-#pragma unroll 4
-            for (int kk = kl; kk < kend; kk += ZS_KL) {
-                const cd a = __ldg(A + (int64_t)(k0 + kk) * lda + row);
-#pragma unroll
-                for (int j = 0; j < NC; ++j) acc[j] = cfma(a, Xs[kk][j], acc[j]);
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NC; ++j) part[kl][rl][j] = acc[j];
-    __syncthreads();
-    for (int e = threadIdx.x; e < ZS_ROWS * NC; e += blockDim.x) {
-        const int r = e % ZS_ROWS, j = e / ZS_ROWS;
-        const int gr = blockIdx.x * ZS_ROWS + r;
-        if (gr < n && j < m) {
-            cd v = part[0][r][j];
-#pragma unroll
-            for (int q = 1; q < ZS_KL; ++q) v = cadd(v, part[q][r][j]);
-            Y[(int64_t)j * n + gr] = v;
-        }
-    }
 }
 
 // r = b - A x for the packed operator.  P1 = G1 [sig1|h1], P2 = G2 [sig2|h2],
@@ -599,7 +546,6 @@ extern "C" int mnpb_bemret_solve_refine(
     auto residual = [&](int e0) -> int {
         const int Bp = B - e0;
         dim3 gz(ceil_div(n, 128), Bp);
-        dim3 gzs(ceil_div(n, ZS_ROWS), Bp);
         const cd *xa = xx + (int64_t)e0 * sx;
         ProfScope ps(s, PC_MATVEC, 4.0 * 16.0 * (double)n * n * Bp);   // bytes of A read
         const int64_t om = (int64_t)e0 * sG;
@@ -607,20 +553,9 @@ extern "C" int mnpb_bemret_solve_refine(
                              (const cd *)H2 + om};
         const cd *xs[4] = {xa, xa + 4 * per, xa, xa + 4 * per};
         cd *ys[4] = {P1, P2, Q1, Q2};
-        for (int q = 0; q < 4; ++q) {
-            // at most 8 columns per launch (shared-memory bound of the lane reduction)
-            for (int c0 = 0; c0 < 4 * k; c0 += 8) {
-                const int mc = min(8, 4 * k - c0);
-                const cd *xq = xs[q] + (int64_t)c0 * N;
-                cd *yq = ys[q] + (int64_t)c0 * N;
-                if (mc <= 4)
-                    zskinny_kernel<4><<<gzs, 256, 0, s>>>(N, mc, mats[q], ld, sG, xq, sx, yq, sP4);
-                else
-                    zskinny_kernel<8><<<gzs, 256, 0, s>>>(N, mc, mats[q], ld, sG, xq, sx, yq, sP4);
-            }
-        }
-        count_launch(3);
-        MNPB_LAUNCH_CHECK("zskinny_kernel");
+        for (int q = 0; q < 4; ++q)
+            MNPB_TRY(skn::run<skn::F64>(s, N, 4 * k, N, Bp, cmk(1, 0), {(cd *)mats[q], ld, sG},
+                                        {(cd *)xs[q], N, sx}, cmk(0, 0), {ys[q], N, sP4}));
         residual_kernel<<<gz, 128, 0, s>>>(N, k, P1, P2, Q1, Q2, sP4, bb + (int64_t)e0 * sx,
                                            r + (int64_t)e0 * sx, sx, eps + 4 * (int64_t)e0,
                                            kvac + e0, nv.shifted(e0));

@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "dense_f32.cuh"
 #include "lu_panel.cuh"
+#include "skinny.cuh"
 #include "trsv_cluster.cuh"
 
 #include <cuda.h>
@@ -59,10 +60,12 @@ __device__ __forceinline__ void st(float *p, int64_t plane, int64_t o, cf v) {
     p[o + plane] = v.y;
 }
 
-// Planar FP32 storage for the cluster kernels (LU panels, triangular solves).
+// Planar FP32 storage for the cluster kernels (LU panels, triangular solves,
+// products with a few vectors).
 struct Planar {
     typedef cf V;
     typedef float S;
+    typedef float Scale;
     struct Mat {
         float *A;
         int64_t lda, plane, sA;
@@ -149,6 +152,47 @@ struct PlanarTri : Planar {
 #pragma unroll 8
         for (int t = 0; t < 32; ++t) y = fma(D[2048 + t * 32 + lane], shfl(r1, t), y);
         r1 = y;
+    }
+};
+
+// Products with a few vectors: R rows per thread in one vector load per plane
+// (16-byte or 8-byte; leading dimension, plane and stride multiples of R and
+// the base aligned to it), or R = 1 for any alignment.
+template <int RR>
+struct PlanarRows : Planar {
+    typedef Planar::Mat Mat;
+    static constexpr int R = RR, U = RR == 1 ? 8 : 4;
+    struct Scale {
+        float a;
+        int rnd;        // store rounded to TF32
+    };
+    static __device__ __forceinline__ void rows(const Mat &m, int64_t b, int64_t row, int64_t col,
+                                                V (&a)[R]) {
+        const float *p = m.A + b * m.sA + col * m.lda + row;
+        if constexpr (R == 4) {
+            const float4 x = __ldg(reinterpret_cast<const float4 *>(p));
+            const float4 y = __ldg(reinterpret_cast<const float4 *>(p + m.plane));
+            a[0] = fmk(x.x, y.x);
+            a[1] = fmk(x.y, y.y);
+            a[2] = fmk(x.z, y.z);
+            a[3] = fmk(x.w, y.w);
+        } else if constexpr (R == 2) {
+            const float2 x = __ldg(reinterpret_cast<const float2 *>(p));
+            const float2 y = __ldg(reinterpret_cast<const float2 *>(p + m.plane));
+            a[0] = fmk(x.x, y.x);
+            a[1] = fmk(x.y, y.y);
+        } else {
+            a[0] = fmk(__ldg(p), __ldg(p + m.plane));
+        }
+    }
+    static __device__ __forceinline__ void out(const Mat &m, int64_t b, int64_t row, int64_t col,
+                                               Scale al, V v, Scale be) {
+        float *y = m.A + b * m.sA + col * m.lda + row;
+        V w = fmk(al.a * v.x, al.a * v.y);
+        if (be.a != 0.f) w = fmk(w.x + be.a * y[0], w.y + be.a * y[m.plane]);
+        if (al.rnd) w = rna(w);
+        y[0] = w.x;
+        y[m.plane] = w.y;
     }
 };
 
@@ -842,66 +886,6 @@ __global__ void __launch_bounds__(128) round_tf32_kernel(float *B, int64_t ldb, 
     }
 }
 
-// Skinny GEMM C = alpha A B + beta C for at most NC (<= 16) columns (matrix
-// times a few vectors): one thread per row, A streamed once with coalesced
-// column reads, B broadcast from shared memory.  Real alpha, beta.
-constexpr int SK_N = 16, SK_KT = 64;
-
-template <int NC>
-__global__ void __launch_bounds__(128) skinny_kernel(int m, int n, int k, float alpha,
-                                                     const float *__restrict__ A, int64_t lda,
-                                                     int64_t planeA, int64_t sA,
-                                                     const float *__restrict__ B, int64_t ldb,
-                                                     int64_t planeB, int64_t sB, float beta,
-                                                     float *__restrict__ C, int64_t ldc,
-                                                     int64_t planeC, int64_t sC, int rnd) {
-    __shared__ cf Bs[SK_KT][NC];
-    const int64_t b = blockIdx.y;
-    A += b * sA;
-    B += b * sB;
-    C += b * sC;
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    cf acc[NC];
-#pragma unroll
-    for (int j = 0; j < NC; ++j) acc[j] = fmk(0.f, 0.f);
-    for (int k0 = 0; k0 < k; k0 += SK_KT) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < SK_KT * NC; e += blockDim.x) {
-            const int kk = e % SK_KT, j = e / SK_KT;
-            Bs[kk][j] = (k0 + kk < k && j < n) ? ld(B, planeB, (int64_t)j * ldb + k0 + kk)
-                                               : fmk(0.f, 0.f);
-        }
-        __syncthreads();
-        if (row < m) {
-            const int kend = min(SK_KT, k - k0);
-            const float *ar = A + (int64_t)k0 * lda + row;
-#pragma unroll 4
-            for (int kk = 0; kk < kend; ++kk) {
-                const cf a = fmk(__ldg(ar + (int64_t)kk * lda), __ldg(ar + (int64_t)kk * lda + planeA));
-#pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    acc[j].x = fmaf(a.x, Bs[kk][j].x, acc[j].x);
-                    acc[j].x = fmaf(-a.y, Bs[kk][j].y, acc[j].x);
-                    acc[j].y = fmaf(a.x, Bs[kk][j].y, acc[j].y);
-                    acc[j].y = fmaf(a.y, Bs[kk][j].x, acc[j].y);
-                }
-            }
-        }
-    }
-    if (row >= m) return;
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-        if (j < n) {
-            const int64_t o = (int64_t)j * ldc + row;
-            cf c = beta != 0.f ? ld(C, planeC, o) : fmk(0.f, 0.f);
-            cf v = fmk(alpha * acc[j].x + beta * c.x, alpha * acc[j].y + beta * c.y);
-            if (rnd) v = fmk(tf32_rna(v.x), tf32_rna(v.y));
-            st(C, planeC, o, v);
-        }
-    }
-}
-
-
 // ---------------------------------------------------------------------------
 // Few-RHS triangular solves: inverses of the 32 x 32 diagonal blocks, and the
 // bounded device waits that the failure-path probe runs.
@@ -1009,76 +993,6 @@ __global__ void set_identity_kernel(float *W, int64_t ldw, int64_t plane, int64_
 
 }  // namespace
 
-// Same product with four rows per thread and 16-byte loads (A's leading
-// dimension, planes and batch stride multiples of 4 floats, A 16-byte
-// aligned, m a multiple of 4): one vector load per plane brings four rows,
-// so a thread keeps more of the matrix stream in flight per instruction.
-template <int NC>
-__global__ void __launch_bounds__(128) skinny4_kernel(int m, int n, int k, float alpha,
-                                                      const float *__restrict__ A, int64_t lda,
-                                                      int64_t planeA, int64_t sA,
-                                                      const float *__restrict__ B, int64_t ldb,
-                                                      int64_t planeB, int64_t sB, float beta,
-                                                      float *__restrict__ C, int64_t ldc,
-                                                      int64_t planeC, int64_t sC, int rnd) {
-    __shared__ cf Bs[SK_KT][NC];
-    const int64_t b = blockIdx.y;
-    A += b * sA;
-    B += b * sB;
-    C += b * sC;
-    const int row = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    cf acc[4][NC];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[r][j] = fmk(0.f, 0.f);
-    for (int k0 = 0; k0 < k; k0 += SK_KT) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < SK_KT * NC; e += blockDim.x) {
-            const int kk = e % SK_KT, j = e / SK_KT;
-            Bs[kk][j] = (k0 + kk < k && j < n) ? ld(B, planeB, (int64_t)j * ldb + k0 + kk)
-                                               : fmk(0.f, 0.f);
-        }
-        __syncthreads();
-        if (row < m) {
-            const int kend = min(SK_KT, k - k0);
-            const float *ar = A + (int64_t)k0 * lda + row;
-#pragma unroll 4
-            for (int kk = 0; kk < kend; ++kk) {
-                const float4 re = __ldg(reinterpret_cast<const float4 *>(ar + (int64_t)kk * lda));
-                const float4 im =
-                    __ldg(reinterpret_cast<const float4 *>(ar + (int64_t)kk * lda + planeA));
-                const float ar4[4] = {re.x, re.y, re.z, re.w}, ai4[4] = {im.x, im.y, im.z, im.w};
-#pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    const cf bv = Bs[kk][j];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        acc[r][j].x = fmaf(ar4[r], bv.x, acc[r][j].x);
-                        acc[r][j].x = fmaf(-ai4[r], bv.y, acc[r][j].x);
-                        acc[r][j].y = fmaf(ar4[r], bv.y, acc[r][j].y);
-                        acc[r][j].y = fmaf(ai4[r], bv.x, acc[r][j].y);
-                    }
-                }
-            }
-        }
-    }
-    if (row >= m) return;
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-        if (j < n) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int64_t o = (int64_t)j * ldc + row + r;
-                cf c = beta != 0.f ? ld(C, planeC, o) : fmk(0.f, 0.f);
-                cf v = fmk(alpha * acc[r][j].x + beta * c.x, alpha * acc[r][j].y + beta * c.y);
-                if (rnd) v = fmk(tf32_rna(v.x), tf32_rna(v.y));
-                st(C, planeC, o, v);
-            }
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------
@@ -1093,43 +1007,25 @@ int gemm(Ctx &c, int m, int n, int k, float alpha, CMatF A, CMatF B, float beta,
         set_error("f32 gemm: k = 0 with beta != 1 is not supported");
         return MNPB_EINVAL;
     }
-    // four rows per thread only where that still leaves enough threads to
-    // keep the GPU's memory pipes full (small batches of small matrices keep
-    // one row per thread)
-    const bool vec4 = n <= 4 && m % 4 == 0 && A.ld % 4 == 0 && A.plane % 4 == 0 &&
-                      A.stride % 4 == 0 && ((uintptr_t)A.p & 15) == 0 &&
-                      (int64_t)c.batch * (m / 4) >= (int64_t)device_sms() * 256;
-    if (vec4) {
-        dim3 grid(ceil_div(m, 512), c.batch);
-        ProfScope ps(c.s, PC_SGEMM, 8.0 * (double)m * k * c.batch);   // bytes of A streamed
-        prof_tag("M=%d N=%d K=%d B=%d v4", m, n, k, c.batch);
-#define MNPB_SKINNY4(NC)                                                                        \
-    skinny4_kernel<NC><<<grid, 128, 0, c.s>>>(m, n, k, alpha, A.p, A.ld, A.plane, A.stride,   \
-                                              B.p, B.ld, B.plane, B.stride, beta, C.p, C.ld,  \
-                                              C.plane, C.stride, round_out ? 1 : 0)
-        if (n <= 1) MNPB_SKINNY4(1);
-        else if (n <= 2) MNPB_SKINNY4(2);
-        else MNPB_SKINNY4(4);
-#undef MNPB_SKINNY4
-        MNPB_LAUNCH_CHECK("skinny4_kernel");
-        return MNPB_OK;
-    }
-    if (n <= SK_N) {
-        dim3 grid(ceil_div(m, 128), c.batch);
+    if (n <= 16) {
         ProfScope ps(c.s, PC_SGEMM, 8.0 * (double)m * k * c.batch);   // bytes of A streamed
         prof_tag("M=%d N=%d K=%d B=%d", m, n, k, c.batch);
-#define MNPB_SKINNY(NC)                                                                        \
-    skinny_kernel<NC><<<grid, 128, 0, c.s>>>(m, n, k, alpha, A.p, A.ld, A.plane, A.stride, B.p, \
-                                             B.ld, B.plane, B.stride, beta, C.p, C.ld, C.plane, \
-                                             C.stride, round_out ? 1 : 0)
-        if (n <= 1) MNPB_SKINNY(1);
-        else if (n <= 2) MNPB_SKINNY(2);
-        else if (n <= 4) MNPB_SKINNY(4);
-        else if (n <= 8) MNPB_SKINNY(8);
-        else MNPB_SKINNY(16);
-#undef MNPB_SKINNY
-        MNPB_LAUNCH_CHECK("skinny_kernel");
-        return MNPB_OK;
+        // vector loads where A allows them and the row blocks (split eightfold
+        // along k at most) still give every SM two CTAs; two rows at most for
+        // the wide instances, whose accumulators fill the registers
+        auto fits = [&](int R) {
+            return m % R == 0 && A.ld % R == 0 && A.plane % R == 0 && A.stride % R == 0 &&
+                   ((uintptr_t)A.p & (4 * R - 1)) == 0 &&
+                   (int64_t)ceil_div(m, skn::ROWT * R) * c.batch * skn::MAXC >= 2 * device_sms();
+        };
+        const Planar::Mat a{A.p, A.ld, A.plane, A.stride}, x{B.p, B.ld, B.plane, B.stride},
+            y{C.p, C.ld, C.plane, C.stride};
+        const int rnd = round_out ? 1 : 0;
+        if (n <= 4 && fits(4))
+            return skn::run<PlanarRows<4>>(c.s, m, n, k, c.batch, {alpha, rnd}, a, x, {beta, 0}, y);
+        if (fits(2))
+            return skn::run<PlanarRows<2>>(c.s, m, n, k, c.batch, {alpha, rnd}, a, x, {beta, 0}, y);
+        return skn::run<PlanarRows<1>>(c.s, m, n, k, c.batch, {alpha, rnd}, a, x, {beta, 0}, y);
     }
     return tc::cgemm_tf32(c.s, m, n, k, c.batch, alpha, A, B, beta, C, c.work, c.work_bytes,
                           round_out, a_tf32);
