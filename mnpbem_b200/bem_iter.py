@@ -95,7 +95,10 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
     kmax = len(augment) if augment else 0
     W = torch.empty((kmax + restart + 1, L), dtype=torch.complex128, device=dev)
     hcol = torch.zeros(kmax + restart + 2, dtype=torch.complex128, device=dev)
-    nrm = torch.zeros(1, dtype=torch.float64, device=dev)
+    # |w| of the Arnoldi step and the least-squares residual, read together
+    nr = torch.zeros(2, dtype=torch.float64, device=dev)
+    nrm, res = nr[0:1], nr[1:2]
+    nr_host = torch.zeros(2, dtype=torch.float64, pin_memory=dev.type == 'cuda')
     wb = int(_lib.lib().mnpb_gmres_workspace(L, kmax + restart))
     work = torch.empty(wb, dtype=torch.uint8, device=dev)
     # augmentation: C = A U orthonormalised in W[0:kc], Uc = U R^-1
@@ -140,7 +143,6 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
     sn = torch.zeros(restart, dtype=torch.complex128, device=dev)
     g = torch.zeros(restart + 1, dtype=torch.complex128, device=dev)
     y = torch.zeros(restart, dtype=torch.complex128, device=dev)
-    res = torch.zeros(1, dtype=torch.float64, device=dev)
     flag, cycles, iters = 1, 0, 0
     beta = float(_norm(r, stream).item())
     checked = False
@@ -166,8 +168,15 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
         g[0] = beta
         H.zero_()
         m = 0
+        ahead = None            # A M v_j issued before the residual of step j - 1 was known
+        known = [beta]          # residuals of this cycle
         for j in range(restart):
-            w = A(M(V[j])).reshape(-1).contiguous()
+            if ahead is None:
+                w = A(M(V[j]))
+            else:
+                w, ahead = ahead, None
+                count.matvecs += 1
+            w = w.reshape(-1).contiguous()
             if kc == 0:
                 call('mnpb_gmres_arnoldi', sh, L, j, ptr(V), L, ptr(w), ptr(H[j]), ptr(nrm),
                      ptr(work), wb)
@@ -180,7 +189,20 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
                  ptr(res))
             iters += 1
             m = j + 1
-            if float(res.item()) <= tol * bnorm or float(nrm.item()) == 0.0:
+            nr_host.copy_(nr, non_blocking=True)
+            done = torch.cuda.Event()
+            done.record()
+            # the next product keeps the device busy while the host waits for
+            # this step's residual; only where the last steps' decrease,
+            # squared, still leaves the residual above the tolerance, so that
+            # a solve that converges at once pays for no product it drops
+            if m < restart and len(known) >= 3 and \
+                    known[-1] * (known[-1] / known[-2]) ** 2 > tol * bnorm:
+                ahead = apply_A(M(V[m]))
+            done.synchronize()
+            hn, hr = nr_host.tolist()
+            known.append(hr)
+            if hr <= tol * bnorm or hn == 0.0:
                 break
         z = torch.zeros_like(b)
         call('mnpb_gmres_update', sh, L, m, ptr(H), restart + 1, ptr(g), ptr(V), L, ptr(y),
@@ -335,8 +357,7 @@ class BEMRetIter(object):
         X = x.reshape(8, K, n)
         v1 = X[0:4].reshape(4 * K, n).contiguous()
         v2 = X[4:8].reshape(4 * K, n).contiguous()
-        P1, P2, Q1, Q2 = [torch.empty((4 * K, n), dtype=torch.complex128, device=self.device)
-                          for _ in range(4)]
+        P1, P2, Q1, Q2 = torch.empty((4, 4 * K, n), dtype=torch.complex128, device=self.device)
         if self.hmatrix:
             hmat_matvec([self.G1, self.G2, self.H1, self.H2], [v1, v2, v1, v2], [P1, P2, Q1, Q2],
                         4 * K)

@@ -254,29 +254,33 @@ def hmat_matvec(hms, xs, ys, nc, stream=None):
     topo = hms[0].topo
     dev = topo.device
     n = topo.n
-    # one V^T x scratch per matrix (the matrices run in the same launch)
-    per = 2 * max(1, max(h.sum_rank for h in hms)) * min(nc, 4)
-    T = torch.empty(per * len(hms), dtype=torch.float64, device=dev)
-    pxc = 2 * n * min(nc, 4)
-    Xc = torch.empty(pxc * len(hms), dtype=torch.float64, device=dev)
-    partial = torch.empty(len(hms) * topo.nitem * 32 * 4 * 2, dtype=torch.float64, device=dev)
-    ptp = 2 * 4 * max(1, max(h.tp_entries for h in hms))
-    TP = torch.empty(ptp * len(hms), dtype=torch.float64, device=dev)
-    desc = np.zeros((len(hms), 13), dtype=np.uint64)
-    keep = []
+    # scratch of the four parts (V^T x, x in cluster order, row partials, V^T x
+    # partials) in one allocation, 256-byte aligned pieces per matrix (the
+    # matrices run in the same launch)
+    m = len(hms)
+    up = lambda k: (k + 31) // 32 * 32
+    per = up(2 * max(1, max(h.sum_rank for h in hms)) * min(nc, 4))
+    pxc = up(2 * n * min(nc, 4))
+    ptp = up(2 * 4 * max(1, max(h.tp_entries for h in hms)))
+    npart = up(m * topo.nitem * 32 * 4 * 2)
+    buf = torch.empty(m * (per + pxc + ptp) + npart, dtype=torch.float64, device=dev)
+    partial = buf.data_ptr()
+    oT = partial + 8 * npart
+    oX = oT + 8 * m * per
+    oTP = oX + 8 * m * pxc
+    desc = np.zeros((m, 13), dtype=np.uint64)
     for i, (h, x, y) in enumerate(zip(hms, xs, ys)):
         if h.topo is not topo:
             raise ValueError("hmat_matvec: all matrices must share one topology")
         if x.dtype != torch.complex128 or y.dtype != torch.complex128 or not x.is_contiguous() \
                 or not y.is_contiguous() or x.numel() < n * nc or y.numel() < n * nc:
             raise ValueError("hmat_matvec: x, y must be contiguous complex128 (nc, n)")
-        desc[i] = [h.D.data_ptr(), h.U.data_ptr(), h.V.data_ptr(), h.rank.data_ptr(),
-                   h.offT.data_ptr(), x.data_ptr(), y.data_ptr(), T[i * per:].data_ptr(),
-                   Xc[i * pxc:].data_ptr(), h.offTP.data_ptr(), TP[i * ptp:].data_ptr(),
-                   h.rent.data_ptr(), h.vent.data_ptr()]
-        keep.append((x, y))
+        desc[i] = (h.D.data_ptr(), h.U.data_ptr(), h.V.data_ptr(), h.rank.data_ptr(),
+                   h.offT.data_ptr(), x.data_ptr(), y.data_ptr(), oT + 8 * i * per,
+                   oX + 8 * i * pxc, h.offTP.data_ptr(), oTP + 8 * i * ptp,
+                   h.rent.data_ptr(), h.vent.data_ptr())
     call('mnpb_hmat_matvec', _lib.stream_handle(stream), n, nc, len(hms), ptr(desc),
          ptr(topo.c2p), topo.nlr, topo.nchunk, ptr(topo.chunks), ptr(topo.leaf_rows),
-         topo.nitem, ptr(topo.items), ptr(topo.cptr), ptr(partial), topo.nvitem,
+         topo.nitem, ptr(topo.items), ptr(topo.cptr), partial, topo.nvitem,
          ptr(topo.vptr))
     return ys
