@@ -68,7 +68,7 @@ class BatchedBEMRet(object):
             mem_bytes = int(0.7 * free)
         self.mem_bytes = int(mem_bytes)
         self.groups = self.buckets([t.n for t in self.tables], pad_ratio)
-        self._bufs = None
+        self._bufs = self._arena = None
         self.stats = []
 
     # ------------------------------------------------------------------ sizes
@@ -116,21 +116,54 @@ class BatchedBEMRet(object):
         return [(s, min(s + size, nentries)) for s in range(0, nentries, size)], size
 
     # --------------------------------------------------------------- buffers
+    @staticmethod
+    def _allocate(dev, n, B, K, empty):
+        """The buffers of one launch batch, in memory from ``empty(shape, dtype)``."""
+        bt = _MixedBatch(type('Size', (), {'device': dev, 'n': n})(), [0.0] * B, empty)
+        bt.nv = empty((B, n, 3), torch.float64)
+        bt.pots = empty((B, 16, K, n), torch.complex128)
+        bt.xin = empty((B, 8, K, n), torch.complex128)
+        bt.x = empty((B, 8, K, n), torch.complex128)
+        bt.rwork = empty((int(_lib.lib().mnpb_bemret_refine_workspace(n, B, K)),), torch.uint8)
+        bt.n_of = empty((B,), torch.int32)
+        return bt
+
+    def _reserve(self, shapes):
+        """One arena that holds the largest of the launch batches ``shapes``
+        ((n, B, K)): every batch is carved from it, so that going from one
+        face count to the next neither returns device memory nor asks for it
+        (which took about 40 ms a time), and each shape keeps its addresses
+        and with them its CUDA graph."""
+        need = 0
+        for n, B, K in shapes:
+            total = [0]
+
+            def measure(shape, dtype):
+                t = torch.empty(shape, dtype=dtype, device='meta')
+                total[0] += -(-t.numel() * t.element_size() // 256) * 256
+                return t
+
+            self._allocate('meta', n, B, K, measure)
+            need = max(need, total[0])
+        if self._arena is None or self._arena.numel() < need:
+            self._bufs = self._arena = None
+            torch.cuda.empty_cache()
+            self._arena = torch.empty(need, dtype=torch.uint8, device=self.tables[0].device)
+
     def _buffers(self, n, B, K):
         key = (n, B, K)
         if self._bufs is not None and self._bufs[0] == key:
             return self._bufs[1]
-        self._bufs = None
-        torch.cuda.empty_cache()
-        dev = self.tables[self.groups[n][0]].device
-        bt = _MixedBatch(type('Size', (), {'device': dev, 'n': n})(), [0.0] * B)
-        bt.nv = torch.empty((B, n, 3), dtype=torch.float64, device=dev)
-        bt.pots = torch.empty((B, 16, K, n), dtype=torch.complex128, device=dev)
-        bt.xin = torch.empty((B, 8, K, n), dtype=torch.complex128, device=dev)
-        bt.x = torch.empty_like(bt.xin)
-        wb = int(_lib.lib().mnpb_bemret_refine_workspace(n, B, K))
-        bt.rwork = torch.empty(wb, dtype=torch.uint8, device=dev)
-        bt.n_of = torch.empty(B, dtype=torch.int32, device=dev)
+        off = [0]
+
+        def carve(shape, dtype):
+            m = int(np.prod(shape, dtype=np.int64))
+            size = m * torch.empty(0, dtype=dtype).element_size()
+            t = self._arena[off[0]:off[0] + size].view(dtype).view(shape)
+            off[0] += -(-size // 256) * 256
+            return t
+
+        bt = self._allocate(self._arena.device, n, B, K, carve)
         self._bufs = (key, bt)
         return bt
 
@@ -189,15 +222,13 @@ class BatchedBEMRet(object):
         sols = [[None] * L for _ in range(P)] if keep_solutions else None
         nvec_s, area_s = pinfty()
         self.stats = []
-        bt = None
+        self._reserve([(n, self._batches(n, len(m) * L, K)[1], K)
+                       for n, m in self.groups.items()])
         for n in sorted(self.groups):
             members = self.groups[n]
             spans, B = self._batches(n, len(members) * L, K)
             for s0, s1 in spans:
                 nb = s1 - s0
-                # drop this frame's reference first: a new buffer shape must be
-                # able to free the previous set before it allocates its own
-                bt = None
                 bt = self._buffers(n, B, K)
                 runs = self._runs(members, eneis, s0, s1)
                 eps = np.zeros((B, 4))

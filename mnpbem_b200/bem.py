@@ -106,32 +106,33 @@ class _RetBatch(object):
 class _MixedBatch(object):
     """Device buffers of a mixed-precision batch: FP64 G1, G2, H1, H2 (the
     exact operator for refinement) and their planar FP32 copies, factorised on
-    the tensor cores.  Leading dimension ld = n rounded up to 4."""
+    the tensor cores.  Leading dimension ld = n rounded up to 4.
+    ``empty(shape, dtype)`` provides the memory (default: new tensors)."""
 
     mixed = True
 
-    def __init__(self, tables, eneis):
+    def __init__(self, tables, eneis, empty=None):
         dev = tables.device
+        if empty is None:
+            empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=dev)
         n = tables.n
         B = len(eneis)
         ld = (n + 3) // 4 * 4
         self.n, self.B, self.ld, self.eneis = n, B, ld, list(eneis)
-        c128 = dict(dtype=torch.complex128, device=dev)
-        f32 = dict(dtype=torch.float32, device=dev)
-        self.G1, self.G2, self.H1, self.H2 = [torch.empty((B, n, ld), **c128) for _ in range(4)]
+        c128, f32, f64, i32 = torch.complex128, torch.float32, torch.float64, torch.int32
+        self.G1, self.G2, self.H1, self.H2 = [empty((B, n, ld), c128) for _ in range(4)]
         # planar copies; G1p/G2p and H1p/H2p back to back (factorised as one batch)
-        self.GGp = torch.empty((2, B, 2, n, ld), **f32)
-        self.HHp = torch.empty((2, B, 2, n, ld), **f32)
+        self.GGp = empty((2, B, 2, n, ld), f32)
+        self.HHp = empty((2, B, 2, n, ld), f32)
         self.G1p, self.G2p = self.GGp[0], self.GGp[1]
         self.H1p, self.H2p = self.HHp[0], self.HHp[1]
-        self.Dp = torch.empty((B, 2, n, ld), **f32)
-        self.piv = torch.empty((3, B, n), dtype=torch.int32, device=dev)
-        self.info = torch.zeros((2, B), dtype=torch.int32, device=dev)
-        self.dinv = torch.empty(int(_lib.lib().mnpb_bemret_dinv_floats(n, B)), **f32)
-        wb = int(_lib.lib().mnpb_bemret_workspace_mixed(n, B))
-        self.work = torch.empty(wb, dtype=torch.uint8, device=dev)
-        self.eps = torch.empty((B, 4), dtype=torch.float64, device=dev)
-        self.kvac = torch.empty(B, dtype=torch.float64, device=dev)
+        self.Dp = empty((B, 2, n, ld), f32)
+        self.piv = empty((3, B, n), i32)
+        self.info = empty((2, B), i32).zero_()
+        self.dinv = empty((int(_lib.lib().mnpb_bemret_dinv_floats(n, B)),), f32)
+        self.work = empty((int(_lib.lib().mnpb_bemret_workspace_mixed(n, B)),), torch.uint8)
+        self.eps = empty((B, 4), f64)
+        self.kvac = empty((B,), f64)
         self.iters = None
         self.relres = None
 

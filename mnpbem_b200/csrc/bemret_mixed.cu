@@ -373,7 +373,7 @@ struct InitGraph {
     int64_t launches;       // kernels in the graph (for the launch counter)
     uint64_t used;
 };
-constexpr int kGraphs = 4;
+constexpr int kGraphs = 8;
 constexpr int kMaxDev = 64;
 // one non-blocking stream per device for the captures (created once)
 cudaStream_t capture_stream(int dev) {
