@@ -228,17 +228,18 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
                     else if (p == jj) pos[r] = bp;
                     // a finished row keeps its values (as stored), the others subtract
                     const bool upd = !done && pos[r] > jj && pos[r] != NOROW;
-                    V l = a[r][w];
-                    if (nz) l = T::rnd(T::mul(l, inv));
-                    if (upd) a[r][w] = l;
+                    if (upd) {
+                        V l = a[r][w];
+                        if (nz) l = T::rnd(T::mul(l, inv));
+                        a[r][w] = l;
 #pragma unroll
-                    for (int g = 0; g < W; g += WIN)
-                        if (g < W - o) {
+                        for (int g = 0; g < W; g += WIN)
+                            if (g < W - o) {
 #pragma unroll
-                            for (int j = g == 0 ? w + 1 : g; j < g + WIN; ++j) {
-                                if (upd) a[r][j] = T::fms(l, u[j], a[r][j]);
+                                for (int j = g == 0 ? w + 1 : g; j < g + WIN; ++j)
+                                    a[r][j] = T::fms(l, u[j], a[r][j]);
                             }
-                        }
+                    }
                     if (done) {
 #pragma unroll
                         for (int g = 0; g < W; g += WIN)
