@@ -267,24 +267,19 @@ struct HMats {
     HMat h[4];
 };
 
-// Warps per block of the product kernels (one work item per warp) and the
-// launch-bound block count per SM.  Measured on the four matrices of the
-// 25,152-face rod (4 right-hand sides): 4 warps x >= 6 blocks 0.971 ms per
-// product, 4 x 4 1.05 ms, 8 x 3 1.06 ms, 8 x 4 (64 registers, spills)
-// 1.24 ms, 4 x 6 with 2 columns in flight 1.18 ms.
-#ifndef HM_WPB
-#define HM_WPB 4
-#endif
-#ifndef HM_MINB
-#define HM_MINB 6
-#endif
-// Matrix columns in flight per lane in the row sums (software pipeline depth).
-#ifndef HM_RUN
-#define HM_RUN 4
-#endif
+// The products run on the FP64 tensor path (mma.sync m16n8k4): up to four
+// complex columns x fill its eight columns as [Xr | Xi], and with
+// [-Xi | Xr] a block A contributes  [Yr | Yi] += Ar [Xr | Xi] + Ai [-Xi | Xr]
+// -- two instructions per 16 x 4 entries, where lanes of FMAs took 32 and a
+// 16-byte shared load of x per entry and column.  What bounds the kernels is
+// issue and the FP64 pipe once the complex64 stream's latency is hidden: a warp
+// works in units of 512 entries, 32 rows x 16 columns or, where there are at
+// most 16 rows, 16 x 32, the next unit's entries (16 loads of 8 bytes per lane)
+// in flight while this one is multiplied, across the ends of blocks.  Measured
+// on the four matrices of the 9600-face rod (four columns): row sums 218 -> 164
+// us (16-row units for short chunks cost it 22), V^T x 115 -> 89.
+constexpr int HM_WPB = 4;        // warps per block, one work item each
 constexpr int HM_VSEG = 64;      // columns per V^T x item (the host cuts segments this long)
-constexpr int HM_XS = 32;        // x columns per shared-memory stage of the row sums
-
 // 16-byte asynchronous copies global -> shared (completion per thread via
 // commit / wait groups; a __syncwarp after the wait publishes the warp's copies)
 __device__ __forceinline__ void cp16(void *dst, const void *src) {
@@ -299,20 +294,111 @@ __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ float2 ld_stream(const float2 *p) { return __ldcs(p); }
+__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
+                 "{%6}, {%0,%1,%2,%3};"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+
+// A unit of MT 16-row tiles and 4 S columns, S = 8 / MT, in the fragment
+// layout: a[s][m][h] is row 16 m + g + 8 h, column 4 s + t (g = lane / 4,
+// t = lane % 4); zero beyond rows and ncol.
+template <int MT>
+struct Unit {
+    static constexpr int S = 8 / MT, COLS = 4 * S;
+    float2 a[S][MT][2];
+    __device__ __forceinline__ void load(const float2 *A, int64_t lda, int rows, int ncol, int g,
+                                         int t) {
+        const float2 *p = A + g + (int64_t)t * lda;
+#pragma unroll
+        for (int s = 0; s < S; ++s, p += 4 * lda)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = 16 * m + 8 * h;
+                    a[s][m][h] = (g + r < rows && 4 * s + t < ncol) ? ld_stream(p + r)
+                                                                    : make_float2(0.f, 0.f);
+                }
+    }
+    // acc[m] (16 x 8: real parts of the columns, then imaginary parts) += unit
+    // times x, xb[column][4]; columns of x from nc on are not read
+    __device__ __forceinline__ void mul(double (&acc)[MT][4], const cd *xb, int rows, int ncol,
+                                        int nc, int g, int t) const {
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            if (4 * s < ncol) {
+                const int c = 4 * s + t;
+                const bool ok = c < ncol && (g & 3) < nc;
+                const cd x = ok ? xb[c * 4 + (g & 3)] : cmk(0.0, 0.0);
+                const double b1 = g < 4 ? x.x : x.y, b2 = g < 4 ? -x.y : x.x;
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+                    if (16 * m < rows) {
+                        mma_f64(acc[m], (double)a[s][m][0].x, (double)a[s][m][1].x, b1);
+                        mma_f64(acc[m], (double)a[s][m][0].y, (double)a[s][m][1].y, b2);
+                    }
+            }
+    }
+};
+// the complex values of a tile's row g + 8 h, columns 2 t and 2 t + 1, in lanes t < 2
+__device__ __forceinline__ void tile_out(const double (&acc)[4], int h, cd &v0, cd &v1) {
+    v0.x = acc[2 * h];
+    v1.x = acc[2 * h + 1];
+    v0.y = __shfl_down_sync(0xffffffffu, v0.x, 2, 4);
+    v1.y = __shfl_down_sync(0xffffffffu, v1.x, 2, 4);
+}
 
 // t_b = V_b^T x in two steps.  One warp per VtxEnt item: the item's x
-// columns (<= 64, all right-hand sides) are staged in shared memory with
-// asynchronous copies while the first factor loads are in flight; lane =
-// factor column q (V is stored transposed, so the lanes of one j read
-// consecutive words) and the x values are shared-memory broadcasts.  Blocks
-// of rank <= 16 put 2 or 4 columns in flight per warp (groups of 16 or 8
-// lanes, summed in a fixed order at the end).  hm_vtx_reduce_kernel adds a
-// block's segments in order (deterministic).
-template <int NC>
-__global__ void __launch_bounds__(32 * HM_WPB, HM_MINB) hm_vtx_kernel(HMats P, int n, int nc,
-                                                                       int nvitem) {
-    __shared__ __align__(16) cd xsm[HM_WPB][HM_VSEG * NC];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+// columns (<= 64, all right-hand sides) are staged in shared memory; V is
+// stored transposed, so an item is a column-major block of r rows.
+// hm_vtx_reduce_kernel adds a block's segments in order (deterministic).
+template <int MT>
+__device__ __forceinline__ void vtx_item(const float2 *V, cd *out, const cd *xb, int r, int cnt,
+                                         int nc, int g, int t) {
+    constexpr int COLS = Unit<MT>::COLS;
+    Unit<MT> cur, nxt;
+    cur.load(V, r, r, min(COLS, cnt), g, t);
+    cp_wait<0>();
+    __syncwarp();
+    double acc[MT][4] = {};
+    int q0 = 0, j0 = 0;
+    while (q0 < r) {
+        int qn = q0, jn = j0 + COLS;
+        if (jn >= cnt) {
+            jn = 0;
+            qn += 16 * MT;
+        }
+        if (qn < r) nxt.load(V + (int64_t)jn * r + qn, r, r - qn, min(COLS, cnt - jn), g, t);
+        cur.mul(acc, xb + j0 * 4, r - q0, min(COLS, cnt - j0), nc, g, t);
+        if (jn == 0) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    cd v0, v1;
+                    tile_out(acc[m], h, v0, v1);
+                    const int q = q0 + 16 * m + g + 8 * h;
+                    if (q < r && t < 2) {
+                        out[(int64_t)q * 4 + 2 * t] = v0;
+                        out[(int64_t)q * 4 + 2 * t + 1] = v1;
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][e] = 0.0;
+            }
+        }
+        cur = nxt;
+        q0 = qn;
+        j0 = jn;
+    }
+}
+
+__global__ void __launch_bounds__(32 * HM_WPB, 4) hm_vtx_kernel(HMats P, int n, int nc,
+                                                                int nvitem) {
+    __shared__ __align__(16) cd xsm[HM_WPB][HM_VSEG * 4];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, g = l >> 2, t = l & 3;
     const int it = blockIdx.x * HM_WPB + w;
     if (it >= nvitem) return;
     const HMat &H = P.h[blockIdx.y];
@@ -322,95 +408,13 @@ __global__ void __launch_bounds__(32 * HM_WPB, HM_MINB) hm_vtx_kernel(HMats P, i
     cd *xb = xsm[w];
     for (int j = l; j < cnt; j += 32)
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-            if (c < nc) cp16(xb + j * NC + c, H.Xc + ve.xo + j + (int64_t)c * n);
+        for (int c = 0; c < 4; ++c)
+            if (c < nc) cp16(xb + j * 4 + c, H.Xc + ve.xo + j + (int64_t)c * n);
     cp_commit();
     const float2 *V = H.V + ve.v;
     cd *out = H.TP + ve.out * 4;
-    if (r <= 16) {
-        const int Pl = r <= 8 ? 8 : 16, G = 32 / Pl;
-        const int g = l / Pl, q = l - g * Pl;
-        const bool live = q < r;
-        constexpr int U4 = 4;
-        cd acc[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = cmk(0, 0);
-        float2 v[U4];
-#pragma unroll
-        for (int u = 0; u < U4; ++u) {
-            const int j = g + u * G;
-            v[u] = (live && j < cnt) ? ld_stream(V + (int64_t)j * r + q) : make_float2(0.f, 0.f);
-        }
-        cp_wait<0>();
-        __syncwarp();
-        for (int j = g; j < cnt; j += U4 * G) {
-            float2 nx[U4];
-#pragma unroll
-            for (int u = 0; u < U4; ++u) {
-                const int jj = j + (U4 + u) * G;
-                nx[u] = (live && jj < cnt) ? ld_stream(V + (int64_t)jj * r + q)
-                                           : make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < U4; ++u) {
-                const int jj = j + u * G;
-                if (jj < cnt) {
-                    const cd vv = cmk(v[u].x, v[u].y);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        if (c < nc) acc[c] = cfma(vv, xb[jj * NC + c], acc[c]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U4; ++u) v[u] = nx[u];
-        }
-        for (int o = Pl; o < 32; o <<= 1)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-                acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-            }
-        if (g == 0 && live)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) out[(int64_t)q * 4 + c] = acc[c];
-        return;
-    }
-    cp_wait<0>();
-    __syncwarp();
-    constexpr int UN = 8;
-    for (int q0 = 0; q0 < r; q0 += 32) {
-        const int q = q0 + l;
-        const bool live = q < r;
-        cd acc[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = cmk(0, 0);
-        float2 v[UN];
-#pragma unroll
-        for (int u = 0; u < UN; ++u)
-            v[u] = (live && u < cnt) ? ld_stream(V + (int64_t)u * r + q) : make_float2(0.f, 0.f);
-        for (int j = 0; j < cnt; j += UN) {
-            float2 nx[UN];
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const int jj = j + UN + u;
-                nx[u] = (live && jj < cnt) ? ld_stream(V + (int64_t)jj * r + q)
-                                           : make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < UN; ++u)
-                if (j + u < cnt) {
-                    const cd vv = cmk(v[u].x, v[u].y);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        if (c < nc) acc[c] = cfma(vv, xb[(j + u) * NC + c], acc[c]);
-                }
-#pragma unroll
-            for (int u = 0; u < UN; ++u) v[u] = nx[u];
-        }
-        if (live)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) out[(int64_t)q * 4 + c] = acc[c];
-    }
+    if (r <= 16) vtx_item<1>(V, out, xb, r, cnt, nc, g, t);
+    else vtx_item<2>(V, out, xb, r, cnt, nc, g, t);
 }
 
 // T[offT[b] * nc + q * nc + c] = sum over the block's segments (in order);
@@ -443,111 +447,106 @@ __global__ void __launch_bounds__(256) hm_vtx_reduce_kernel(HMats P, int nc, int
 // Row sums in two steps.  Work items (shared by the matrices): (chunk,
 // first entry, end entry, first row within the leaf << 6 | live rows) -- a
 // 32-row piece of a leaf and a segment of at most a few entries of the
-// leaf's contribution list.  One warp per item, lane = row.  The entries'
-// columns are walked in stages of HM_XS: the x values of the next stage
-// (X in cluster order for a dense block, t for a low-rank one) are copied
-// to shared memory asynchronously while the current stage is multiplied, so
-// the only long-latency loads in the inner loop are the streamed matrix
-// columns (prefetched UN at a time).  The warp writes a 32 x NC partial;
-// hm_reduce_kernel adds the partials of each chunk in item order (so the
-// result is deterministic) and scatters the rows to face order.
-template <int NC>
-__global__ void __launch_bounds__(32 * HM_WPB, HM_MINB) hm_rows_kernel(
-    HMats P, int n, int nitem, const int4 *__restrict__ items, cd *__restrict__ partial) {
-    __shared__ __align__(16) cd xsm[HM_WPB][2][HM_XS * NC];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+// leaf's contribution list.  One warp per item walks the entries' columns in
+// units; the x values (X in cluster order for a dense block, t for a low-rank
+// one) are copied to shared memory two units ahead, the entries loaded one
+// unit ahead.  The warp writes a 32 x nc partial; hm_reduce_kernel adds the
+// partials of each chunk in item order (so the result is deterministic) and
+// scatters the rows to face order.
+__global__ void __launch_bounds__(32 * HM_WPB, 4) hm_rows_kernel(HMats P, int n, int nc,
+                                                                 int nitem,
+                                                                 const int4 *__restrict__ items,
+                                                                 cd *__restrict__ partial) {
+    constexpr int MT = 2, COLS = Unit<MT>::COLS;
+    __shared__ __align__(16) cd xsm[HM_WPB][3][COLS * 4];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, g = l >> 2, t = l & 3;
     const int it = blockIdx.x * HM_WPB + w;
     if (it >= nitem) return;
     const HMat &H = P.h[blockIdx.y];
     const int4 item = items[it];
     const int ne = item.z - item.y;           // <= 32 (host cuts the lists)
-    const int r0 = item.w >> 6;
-    const bool live = l < (item.w & 63);
+    const int r0 = item.w >> 6, rows = item.w & 63;
     // lane q holds the record of entry item.y + q
     RowEnt mine;
     mine.a = 0; mine.xo = 0; mine.lda = 0; mine.cnt = 0; mine.kind = 0; mine.pad = 0;
     if (l < ne) mine = H.rent[item.y + l];
     const unsigned FULL = 0xffffffffu;
-    // (e, j0): current stage = columns j0 .. j0 + HM_XS of entry e
-    auto advance = [&](int &e, int &j0, int &cnt) -> bool {
-        j0 += HM_XS;
-        if (j0 < cnt) return true;
-        j0 = 0;
+    struct At {
+        int e, j0, cnt;                       // columns j0 .. j0 + COLS of entry e
+    };
+    auto advance = [&](At &u) -> bool {
+        u.j0 += COLS;
+        if (u.j0 < u.cnt) return true;
+        u.j0 = 0;
         do {
-            if (++e >= ne) return false;
-            cnt = __shfl_sync(FULL, mine.cnt, e);
-        } while (cnt == 0);
+            if (++u.e >= ne) return false;
+            u.cnt = __shfl_sync(FULL, mine.cnt, u.e);
+        } while (u.cnt == 0);
         return true;
     };
-    auto stage_x = [&](int e, int j0, int cnt, cd *buf) {
-        const long long xo = __shfl_sync(FULL, mine.xo, e);
-        const int kind = __shfl_sync(FULL, mine.kind, e);
-        const int ncol = min(HM_XS, cnt - j0);
-        if (l < ncol) {
-            if (kind == 0) {
-                const cd *src = H.Xc + xo + j0 + l;
+    auto stage_x = [&](const At &u, cd *buf) {
+        const long long xo = __shfl_sync(FULL, mine.xo, u.e);
+        const int kind = __shfl_sync(FULL, mine.kind, u.e);
+        const int ncol = min(COLS, u.cnt - u.j0);
+        const int j = l % COLS;
 #pragma unroll
-                for (int c = 0; c < NC; ++c) cp16(buf + l * NC + c, src + (int64_t)c * n);
-            } else {
-                const cd *src = H.T + (xo + j0 + l) * NC;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) cp16(buf + l * NC + c, src + c);
-            }
-        }
-        cp_commit();
+        for (int c = l / COLS; c < 4; c += 32 / COLS)
+            if (j < ncol && c < nc)
+                cp16(buf + j * 4 + c, kind == 0 ? H.Xc + xo + u.j0 + j + (int64_t)c * n
+                                                : H.T + (xo + u.j0 + j) * nc + c);
     };
-    cd acc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] = cmk(0, 0);
-    int e = -1, j0 = 0, cnt = 0, buf = 0;
-    bool have = advance(e, j0, cnt);
-    if (have) stage_x(e, j0, cnt, xsm[w][0]);
-    constexpr int UN = HM_RUN;
-    while (have) {
-        int en = e, jn = j0, cn = cnt;
-        const bool more = advance(en, jn, cn);
-        if (more) stage_x(en, jn, cn, xsm[w][buf ^ 1]);
-        else cp_commit();                       // an empty group keeps the count uniform
-        const long long ao = __shfl_sync(FULL, mine.a, e);
-        const int lda = __shfl_sync(FULL, mine.lda, e);
-        const int kind = __shfl_sync(FULL, mine.kind, e);
-        const int ncol = min(HM_XS, cnt - j0);
-        const float2 *A = (kind == 0 ? H.D : H.U) + ao + r0 + l + (int64_t)j0 * lda;
-        float2 a[UN];
-#pragma unroll
-        for (int u = 0; u < UN; ++u)
-            a[u] = (live && u < ncol) ? ld_stream(A + (int64_t)u * lda) : make_float2(0.f, 0.f);
-        cp_wait<1>();
+    auto load = [&](const At &u, Unit<MT> &a) {
+        const long long ao = __shfl_sync(FULL, mine.a, u.e);
+        const int lda = __shfl_sync(FULL, mine.lda, u.e);
+        const int kind = __shfl_sync(FULL, mine.kind, u.e);
+        a.load((kind == 0 ? H.D : H.U) + ao + r0 + (int64_t)u.j0 * lda, lda, rows,
+               min(COLS, u.cnt - u.j0), g, t);
+    };
+    double acc[MT][4] = {};
+    Unit<MT> cur, nxt;
+    At u0{-1, 0, 0}, u1, u2;
+    bool h0 = advance(u0), h1 = false, h2;
+    u1 = u0;
+    if (h0) {
+        stage_x(u0, xsm[w][0]);
+        load(u0, cur);
+        h1 = advance(u1);
+    }
+    cp_commit();
+    if (h1) stage_x(u1, xsm[w][1]);
+    cp_commit();
+    int b0 = 0, b2 = 2;
+    while (h0) {
+        u2 = u1;
+        h2 = h1 && advance(u2);
+        if (h2) stage_x(u2, xsm[w][b2]);
+        cp_commit();                          // empty groups keep the count uniform
+        if (h1) load(u1, nxt);
+        cp_wait<2>();
         __syncwarp();
-        const cd *xb = xsm[w][buf];
-        for (int j = 0; j < ncol; j += UN) {
-            float2 nx[UN];
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const int jj = j + UN + u;
-                nx[u] = (live && jj < ncol) ? ld_stream(A + (int64_t)jj * lda)
-                                            : make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < UN; ++u)
-                if (j + u < ncol) {
-                    const cd av = cmk(a[u].x, a[u].y);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) acc[c] = cfma(av, xb[(j + u) * NC + c], acc[c]);
-                }
-#pragma unroll
-            for (int u = 0; u < UN; ++u) a[u] = nx[u];
-        }
-        __syncwarp();                           // stage buffer free for the copy after next
-        buf ^= 1;
-        e = en;
-        j0 = jn;
-        cnt = cn;
-        have = more;
+        cur.mul(acc, xsm[w][b0], rows, min(COLS, u0.cnt - u0.j0), nc, g, t);
+        cur = nxt;
+        u0 = u1;
+        u1 = u2;
+        h0 = h1;
+        h1 = h2;
+        b0 = b0 == 2 ? 0 : b0 + 1;
+        b2 = b2 == 2 ? 0 : b2 + 1;
+        __syncwarp();                         // the unit's buffer is free
     }
     cd *out = partial + ((int64_t)blockIdx.y * nitem + it) * 32 * 4;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) out[c * 32 + l] = acc[c];
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            cd v0, v1;
+            tile_out(acc[m], h, v0, v1);
+            const int r = 16 * m + g + 8 * h;
+            if (t < 2) {
+                out[(2 * t) * 32 + r] = v0;
+                out[(2 * t + 1) * 32 + r] = v1;
+            }
+        }
 }
 
 // y rows of chunk k = sum of the partials of items cptr[k] .. cptr[k+1]-1
@@ -720,28 +719,28 @@ extern "C" int mnpb_hmat_matvec(void *stream, int64_t n, int64_t nc, int64_t nma
             Q, (int)n, ncc, c2p);
         MNPB_LAUNCH_CHECK("hm permute_kernel");
         if (nlr > 0) {
-            dim3 g((unsigned)ceil_div(nvitem, HM_WPB), (unsigned)nmat);
-            hm::hm_vtx_kernel<4><<<g, 32 * HM_WPB, 0, s>>>(Q, (int)n, ncc, (int)nvitem);
+            dim3 g((unsigned)ceil_div(nvitem, hm::HM_WPB), (unsigned)nmat);
+            hm::hm_vtx_kernel<<<g, 32 * hm::HM_WPB, 0, s>>>(Q, (int)n, ncc, (int)nvitem);
             MNPB_LAUNCH_CHECK("hm_vtx_kernel");
             dim3 gr((unsigned)ceil_div(nlr, 8), (unsigned)nmat);
             hm::hm_vtx_reduce_kernel<4><<<gr, 256, 0, s>>>(Q, ncc, (int)nlr, vptr);
             MNPB_LAUNCH_CHECK("hm_vtx_reduce_kernel");
         }
-        dim3 g((unsigned)ceil_div(nitem, HM_WPB), (unsigned)nmat);
+        dim3 g((unsigned)ceil_div(nitem, hm::HM_WPB), (unsigned)nmat);
         dim3 gr((unsigned)ceil_div(nchunk, 8), (unsigned)nmat);
-#define MNPB_HM_ROWS(NCV)                                                                       \
-    hm::hm_rows_kernel<NCV><<<g, 32 * HM_WPB, 0, s>>>(Q, (int)n, (int)nitem,                     \
-                                                     (const int4 *)items, (cd *)partial);        \
+        hm::hm_rows_kernel<<<g, 32 * hm::HM_WPB, 0, s>>>(Q, (int)n, ncc, (int)nitem,
+                                                         (const int4 *)items, (cd *)partial);
+#define MNPB_HM_REDUCE(NCV)                                                                     \
     hm::hm_reduce_kernel<NCV><<<gr, 256, 0, s>>>(Q, (int)n, NCV, (int)nchunk, (int)nitem, cptr,  \
                                                  (const int2 *)chunks, (const int2 *)leaf_rows,  \
                                                  c2p, (const cd *)partial)
         switch (ncc) {
-        case 1: MNPB_HM_ROWS(1); break;
-        case 2: MNPB_HM_ROWS(2); break;
-        case 3: MNPB_HM_ROWS(3); break;
-        default: MNPB_HM_ROWS(4); break;
+        case 1: MNPB_HM_REDUCE(1); break;
+        case 2: MNPB_HM_REDUCE(2); break;
+        case 3: MNPB_HM_REDUCE(3); break;
+        default: MNPB_HM_REDUCE(4); break;
         }
-#undef MNPB_HM_ROWS
+#undef MNPB_HM_REDUCE
         MNPB_LAUNCH_CHECK("hm_rows_kernel");
     }
     return MNPB_OK;

@@ -83,7 +83,11 @@ class HTopology(object):
         # 32-row chunks of the leaves, and work items (chunk, segment of at
         # most SEG entries of the leaf's list, first row << 6 | rows): one
         # warp per item
-        SEG = 6
+        # (6, fewer while that leaves the GPU short of warps: four matrices run
+        # in one launch, and about 32 warps per SM keep its loads in flight)
+        total = sum(int(lptr[L + 1] - lptr[L]) * -(-int(lsize[L]) // 32)
+                    for L in range(self.nleaf))
+        SEG = min(6, max(2, 4 * total // (32 * 148)))
         ch, items, cptr = [], [], [0]
         for L in range(self.nleaf):
             for r0 in range(0, int(lsize[L]), 32):
