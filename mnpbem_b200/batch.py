@@ -147,7 +147,6 @@ class BatchedBEMRet(object):
             need = max(need, total[0])
         if self._arena is None or self._arena.numel() < need:
             self._bufs = self._arena = None
-            torch.cuda.empty_cache()
             self._arena = torch.empty(need, dtype=torch.uint8, device=self.tables[0].device)
 
     def _buffers(self, n, B, K):

@@ -335,15 +335,17 @@ __device__ __forceinline__ int64_t find_pair(const PointTables &t, int64_t i, in
 // formula G = e^{ikd}/d a_j, Gp = (ik - 1/d)/d^2 (pt_i - pos_j) a_j e^{ikd},
 // or for refined pairs sum_n (ik)^n g_n e^{ikd} and the same with f_n
 // (greenret_refined.py:727-845).
-__device__ __forceinline__ void point_entry(const PointTables &t, cd k, int64_t i, int64_t j,
-                                            cd &G, cd Gp[3]) {
+// p: the pair's index in the refined list, or -1.
+__device__ __forceinline__ void point_entry_at(const PointTables &t, cd k, int64_t i, int64_t j,
+                                               int64_t p, cd &G, cd Gp[3]) {
     const double x = t.ptpos[3 * i] - t.pos[3 * j];
     const double y = t.ptpos[3 * i + 1] - t.pos[3 * j + 1];
     const double z = t.ptpos[3 * i + 2] - t.pos[3 * j + 2];
     double d = sqrt(x * x + y * y + z * z);
     if (d < kEpsP) d = kEpsP;
-    const cd ph = cexpi(k, d);
-    const int64_t p = find_pair(t, i, j);
+    cd ph;
+    if (k.y == 0.0) sincos(k.x * d, &ph.y, &ph.x);    // lossless medium: |ph| = 1
+    else ph = cexpi(k, d);
     if (p >= 0) {
         const cd ik = cmk(-k.y, k.x);
         cd pw = cmk(1.0, 0.0), s0 = cmk(0, 0), s1 = s0, s2 = s0, s3 = s0;
@@ -369,6 +371,11 @@ __device__ __forceinline__ void point_entry(const PointTables &t, cd k, int64_t 
     Gp[2] = cmul(cscale(cscale(faux, z), a), ph);
 }
 
+__device__ __forceinline__ void point_entry(const PointTables &t, cd k, int64_t i, int64_t j,
+                                            cd &G, cd Gp[3]) {
+    point_entry_at(t, k, i, j, find_pair(t, i, j), G, Gp);
+}
+
 // Fields (mode 0) or potentials (mode 1) at the points, one CTA per (point,
 // column chunk, wavelength); faces whose side s borders the point's medium
 // contribute with the charges / currents of side s:
@@ -378,20 +385,31 @@ __device__ __forceinline__ void point_entry(const PointTables &t, cd k, int64_t 
 // (mode 1: o1 = phi [b][npt][KC], o2 = a [b][npt][3][KC]).  With diag > 0
 // point i reads only columns [i diag, (i + 1) diag) and KC = diag, else
 // KC = K.
+//
+// Bound by the FP64 pipe (sine and cosine, the square root and the division of
+// every pair) once enough warps are resident: the accumulators are those of NC
+// columns, not of the most a chunk can have (102 registers for one column, 166
+// for four).  Membership in the refined list is one bit per face in shared
+// memory; only set bits search the list.  3072 points x 1564 faces, one column:
+// 131 -> 89 us; two points per CTA sharing a face's loads took 110 (156
+// registers).
 constexpr int PG_T = 128;
 constexpr int PG_CH = 4;
+constexpr int PG_BITS = 32 * 1024;        // shared memory for the bits
 
-__global__ void __launch_bounds__(PG_T) point_green_kernel(PointTables t, int mode, int K,
-                                                           int diag,
+template <int NC>
+__global__ void __launch_bounds__(PG_T, NC == 1 ? 5 : NC == 2 ? 4 : 3) point_green_kernel(PointTables t, int mode, int K,
+                                                           int diag, int use_bits,
                                                            const double *__restrict__ k0v,
                                                            const cd *__restrict__ sol,
                                                            cd *__restrict__ o1,
                                                            cd *__restrict__ o2) {
+    extern __shared__ uint32_t pg_bits[];
     const int64_t i = blockIdx.x;
     const int64_t b = blockIdx.z;
     const int KC = diag > 0 ? diag : K;
     const int c_lo = blockIdx.y * PG_CH;                 // within the point's KC columns
-    const int nc = min(PG_CH, KC - c_lo);
+    const int nc = min(NC, KC - c_lo);
     const int col0 = (diag > 0 ? (int)i * diag : 0) + c_lo;
     const int mpt = t.pt_med[i] <= t.nmed ? t.pt_med[i] : 0;
     const cd k = mpt > 0 ? cmk(t.k_t[2 * (b * t.nmed + mpt - 1)], t.k_t[2 * (b * t.nmed + mpt - 1) + 1])
@@ -399,20 +417,29 @@ __global__ void __launch_bounds__(PG_T) point_green_kernel(PointTables t, int mo
     const double k0 = k0v[b];
     const int64_t n = t.n;
     const cd *x = sol + b * (int64_t)8 * K * n;
-    double acc[PG_CH * 12];
+    double acc[NC * 12];
 #pragma unroll
-    for (int q = 0; q < PG_CH * 12; ++q) acc[q] = 0.0;
+    for (int q = 0; q < NC * 12; ++q) acc[q] = 0.0;
+    if (use_bits && mpt > 0) {
+        for (int64_t e = threadIdx.x; e < (n + 31) / 32; e += PG_T) pg_bits[e] = 0u;
+        __syncthreads();
+        for (int64_t e = t.rptr[i] + threadIdx.x; e < t.rptr[i + 1]; e += PG_T)
+            atomicOr(&pg_bits[t.cols[e] / 32], 1u << (t.cols[e] & 31));
+        __syncthreads();
+    }
     if (mpt > 0 && nc > 0) {
         for (int64_t j = threadIdx.x; j < n; j += PG_T) {
             const int s0 = t.face_med[2 * j] == mpt, s1 = t.face_med[2 * j + 1] == mpt;
             if (!s0 && !s1) continue;
+            int64_t pair = -1;
+            if (!use_bits || (pg_bits[j / 32] >> (j & 31)) & 1) pair = find_pair(t, i, j);
             cd G, Gp[3];
-            point_entry(t, k, i, j, G, Gp);
+            point_entry_at(t, k, i, j, pair, G, Gp);
             for (int s = 0; s < 2; ++s) {
                 if (!(s == 0 ? s0 : s1)) continue;
                 const int base = 4 * s;
 #pragma unroll
-                for (int c = 0; c < PG_CH; ++c) {
+                for (int c = 0; c < NC; ++c) {
                     if (c >= nc) break;
                     const int col = col0 + c;
                     const cd sg = x[(int64_t)(base * K + col) * n + j];
@@ -445,10 +472,10 @@ __global__ void __launch_bounds__(PG_T) point_green_kernel(PointTables t, int mo
             }
         }
     }
-    __shared__ double red[PG_T / 32][PG_CH * 12];
+    __shared__ double red[PG_T / 32][NC * 12];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-    for (int q = 0; q < PG_CH * 12; ++q) {
+    for (int q = 0; q < NC * 12; ++q) {
         const double w = wsum(acc[q]);
         if (lane == 0) red[warp][q] = w;
     }
@@ -632,10 +659,18 @@ extern "C" int mnpb_point_green(void *stream, int64_t npt, const double *ptpos,
                  "point_green: diag = %lld needs npt * diag <= K", (long long)diag);
     MNPB_REQUIRE(k0 && sol && o1 && o2, "point_green: null pointer");
     const int64_t KC = diag > 0 ? diag : K;
+    MNPB_REQUIRE(ceil_div(KC, PG_CH) < 65536, "point_green: too many columns");
+    const int64_t bits = (n + 31) / 32 * 4;
+    const int use_bits = bits <= PG_BITS ? 1 : 0;
     dim3 grid((unsigned)npt, ceil_div(KC, PG_CH), (unsigned)batch);
-    MNPB_REQUIRE(grid.y < 65536, "point_green: too many columns");
-    point_green_kernel<<<grid, PG_T, 0, as_stream(stream)>>>(t, mode, (int)K, (int)diag, k0,
-                                                            (const cd *)sol, (cd *)o1, (cd *)o2);
+#define MNPB_PG(NC)                                                                          \
+    point_green_kernel<NC><<<grid, PG_T, use_bits ? (size_t)bits : 0, as_stream(stream)>>>(   \
+        t, mode, (int)K, (int)diag, use_bits, k0, (const cd *)sol, (cd *)o1, (cd *)o2)
+    if (KC == 1) MNPB_PG(1);
+    else if (KC == 2) MNPB_PG(2);
+    else if (KC == 3) MNPB_PG(3);
+    else MNPB_PG(4);
+#undef MNPB_PG
     MNPB_LAUNCH_CHECK("point_green_kernel");
     return MNPB_OK;
 }
