@@ -1,13 +1,16 @@
 // Batched dense complex linear algebra in FP32 on planar storage (real plane,
 // imaginary plane), column-major, for the mixed-precision solver.
 //
-// LU is recursive (split the columns in halves; factor the left half; update
-// the right half with a triangular solve and a GEMM; factor the rest), so
-// nearly all flops land in large GEMMs that run on the tensor cores
-// (tc::cgemm_tf32); only the 32-column LU leaves, the 128 x 128 diagonal-block
-// inverses and the 32-row leaves of small triangular solves run on CUDA cores.
+// LU is recursive down to blocks of 128 columns (split the columns in halves;
+// factor the left half; update the right half with a triangular solve and a
+// GEMM; factor the rest), so nearly all flops land in large GEMMs that run on
+// the tensor cores (tc::cgemm_tf32).  A block goes leaf by leaf: 32-column LU
+// panel, fused interchange and solve of the block's other columns, GEMM.  Only
+// the panels, those strips, the 128 x 128 diagonal-block inverses and the
+// 32-row leaves of small triangular solves run on CUDA cores.
 #include "common.cuh"
 #include "dense_f32.cuh"
+#include "interchange.cuh"
 #include "lu_panel.cuh"
 #include "skinny.cuh"
 #include "trsv_cluster.cuh"
@@ -597,6 +600,84 @@ __global__ void __launch_bounds__(SLAB_THREADS, SW == 4 ? 2 : 1) panel_slab_kern
             }
         }
         __syncthreads();
+    }
+}
+
+// The pivots of a leaf's columns [off, off + kb) (kb <= 32) on the other columns
+// [j0, j1) of its block: the interchanges, composed into a gather, and for the
+// columns right of the leaf U12 = L11^-1 A12 on its rows, stored as TF32 (later
+// rows are eliminated with the stored values).  One CTA per 32 columns, four
+// lanes per column with eight rows each.  It replaces, inside a block of 128
+// columns, an interchange launch and one or more 32-row solve leaves per level
+// of the recursion (about 11 launches of 5 to 10 us per block become 4).
+// Latency-bound (4 to 8 us a launch).  LU of n, batch, before -> after: 2884 x 1
+// 10.8 -> 9.8 ms, 2884 x 27 20.7 -> 18.9 ms, 2884 x 162 82.3 -> 81.1 ms, 1148 x 54
+// 5.35 -> 4.95 ms; 284 x 1 the same (0.65 ms).  Blocks of 128 columns: what is
+// left to the recursion above has products deep enough for the tensor cores.
+constexpr int SSV = 32, SST = SSV + 1;
+__global__ void __launch_bounds__(128) swap_solve_kernel(int off, int kb, int j0, int j1, float *A,
+                                                         int64_t lda, int64_t plane, int64_t sA,
+                                                         const int32_t *ipiv, int64_t sP) {
+    __shared__ cf X[32][SST], L[32][SST];
+    __shared__ swp::Swaps sw;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int64_t b = blockIdx.y;
+    A += b * sA;
+    // columns [j0, off), then [off + kb, j1)
+    const int nl = (off - j0 + SSV - 1) / SSV;
+    const bool solve = (int)blockIdx.x >= nl;
+    const int v0 = solve ? off + kb + ((int)blockIdx.x - nl) * SSV : j0 + (int)blockIdx.x * SSV;
+    const int nv = min(SSV, (solve ? j1 : off) - v0);
+    if (solve)
+        for (int e = tid; e < 1024; e += 128) {
+            const int r = e & 31, c = e >> 5;
+            L[c][r] = (r < kb && c < r) ? ld(A, plane, (int64_t)(off + c) * lda + off + r)
+                                        : fmk(0.f, 0.f);
+        }
+    swp::compose(sw, ipiv + b * sP + off, off, kb);
+    cf t[8], u[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int e = tid + 128 * q, c = e & 31, v = e >> 5;
+        const int64_t o = (int64_t)(v0 + v) * lda + off;
+        const bool on = c < kb && v < nv;
+        t[q] = on ? ld(A, plane, o + sw.out[c]) : fmk(0.f, 0.f);
+        u[q] = on && sw.tail[c] >= 0 ? ld(A, plane, o + sw.tail[c]) : fmk(0.f, 0.f);
+    }
+    __syncthreads();                 // every row read: A may be written
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int e = tid + 128 * q, c = e & 31, v = e >> 5;
+        const int64_t o = (int64_t)(v0 + v) * lda + off;
+        if (c < kb && v < nv) {
+            if (sw.tail[c] >= 0) st(A, plane, o + sw.p[c], u[q]);
+            if (!solve) st(A, plane, o + c, t[q]);
+        }
+        X[c][v] = t[q];
+    }
+    if (!solve) return;
+    __syncthreads();
+    const int v = wid * 8 + (lane >> 2), r = lane & 3;
+    cf y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = X[4 * i + r][v];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+        if (r == (c & 3)) y[c >> 2] = rna(y[c >> 2]);
+        const int src = (lane & ~3) | (c & 3);
+        const cf x = fmk(__shfl_sync(0xffffffffu, y[c >> 2].x, src),
+                         __shfl_sync(0xffffffffu, y[c >> 2].y, src));
+        if (r > (c & 3)) y[c >> 2] = ffms(L[c][4 * (c >> 2) + r], x, y[c >> 2]);
+#pragma unroll
+        for (int i = (c >> 2) + 1; i < 8; ++i) y[i] = ffms(L[c][4 * i + r], x, y[i]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) X[4 * i + r][v] = y[i];
+    __syncthreads();
+    for (int e = tid; e < kb * nv; e += 128) {
+        const int c = e % kb, w = e / kb;
+        st(A, plane, (int64_t)(v0 + w) * lda + off + c, X[c][w]);
     }
 }
 
@@ -1283,6 +1364,74 @@ static int seg_push(SwpSegs &t, int j0, int j1, int cs) {
     return MNPB_OK;
 }
 
+// One LU leaf: columns [off, off + w) (w <= 32) over rows [off, n).
+static int leaf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, int64_t sP,
+                int32_t *info) {
+    ProfScope ps(c.s, PC_PANEL, 8.0 * w * w * (double)(n - off) * c.batch / 2);
+    prof_tag("off=%d w=%d B=%d", off, w, c.batch);
+    const Planar::Mat mat{A.p, A.ld, A.plane, A.stride};
+    int C, threads;
+    // registers of a cluster while that runs in one wave: one row per
+    // thread if it does, two otherwise (LU of 2884 matrices: 1 16.4 ->
+    // 10.7 ms, 8 19.5 -> 14.1, 27 24.7 -> 21.2).  More matrices keep one
+    // CTA each and the slab in shared memory, whose pivot steps are longer
+    // but leave no second wave (54: 33.2 against 34.0, 162: 83 against 91)
+    if (lup::panel_shape(n - off, 1, C, threads) && (int64_t)C * c.batch <= dev_sms())
+        return lup::launch_panel<Planar, TS, 1>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                C, threads);
+    if (lup::panel_shape(n - off, 2, C, threads) && (int64_t)C * c.batch <= dev_sms())
+        return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                C, threads);
+    MNPB_TRY(smem_opt_in(panel_slab_kernel<8>, 200 * 1024, "panel_slab_kernel<8>"));
+    MNPB_TRY(smem_opt_in(panel_slab_kernel<4>, 200 * 1024, "panel_slab_kernel<4>"));
+    // more matrices than SMs: 4-column slabs, half the shared memory, so
+    // that two CTAs share an SM and the batch runs in one wave
+    const int64_t slab8 = (int64_t)8 * (n - off) * 8, slab4 = slab8 / 2;
+    if (c.batch > dev_sms() && w % 4 == 0 && w <= TS && slab4 <= 100 * 1024) {
+        panel_slab_kernel<4><<<c.batch, SLAB_THREADS, (size_t)slab4, c.s>>>(
+            n, off, w, A.p, A.ld, A.plane, A.stride, ipiv, sP, info);
+        MNPB_LAUNCH_CHECK("panel_slab_kernel<4>(f32)");
+        return MNPB_OK;
+    }
+    if (w % 8 == 0 && w <= TS && slab8 <= 200 * 1024) {
+        panel_slab_kernel<8><<<c.batch, SLAB_THREADS, (size_t)slab8, c.s>>>(
+            n, off, w, A.p, A.ld, A.plane, A.stride, ipiv, sP, info);
+        MNPB_LAUNCH_CHECK("panel_slab_kernel(f32)");
+        return MNPB_OK;
+    }
+    if (lup::panel_shape(n - off, 2, C, threads))
+        return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
+                                                C, threads);
+    panel_kernel<<<c.batch, PANEL_THREADS, 0, c.s>>>(n, off, w, A.p, A.ld, A.plane, A.stride,
+                                                     ipiv, sP, info);
+    MNPB_LAUNCH_CHECK("panel_kernel(f32)");
+    return MNPB_OK;
+}
+
+// Blocks of up to LB columns are factored leaf by leaf (right-looking), wider
+// ones by halves.
+constexpr int LB = 128;
+static int block_getrf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, int64_t sP,
+                       int32_t *info) {
+    const int end = off + w;
+    for (int c0 = off; c0 < end; c0 += TS) {
+        const int kb = min(TS, end - c0), c1 = c0 + kb;
+        MNPB_TRY(leaf(c, n, c0, kb, A, ipiv, sP, info));
+        if (w == kb) break;
+        {
+            ProfScope ps(c.s, PC_SWAP, 0.0);
+            const int strips = ceil_div(c0 - off, SSV) + ceil_div(end - c1, SSV);
+            swap_solve_kernel<<<dim3(strips, c.batch), 128, 0, c.s>>>(
+                c0, kb, off, end, A.p, A.ld, A.plane, A.stride, ipiv, sP);
+            MNPB_LAUNCH_CHECK("swap_solve_kernel");
+        }
+        // L21 and U12 are stored rounded to TF32: read in place
+        MNPB_TRY(gemm(c, n - c1, end - c1, kb, -1.f, A.sub(c1, c0), A.sub(c0, c1), 1.f,
+                      A.sub(c1, c1), false, true));
+    }
+    return MNPB_OK;
+}
+
 // Factor columns [off, off+w) over rows [off, n) of the full matrix A;
 // pivots are absolute row indices.  The backward interchanges this node's
 // columns still owe (its right half's pivots on its left half, and what its
@@ -1293,48 +1442,8 @@ static int rgetrf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, int64_t
                   int32_t *info, SwpSegs &owed) {
     owed.n = 0;
     owed.end = off + w;
-    if (w <= TS) {
-        ProfScope ps(c.s, PC_PANEL, 8.0 * w * w * (double)(n - off) * c.batch / 2);
-        prof_tag("off=%d w=%d B=%d", off, w, c.batch);
-        const Planar::Mat mat{A.p, A.ld, A.plane, A.stride};
-        int C, threads;
-        // registers of a cluster while that runs in one wave: one row per
-        // thread if it does, two otherwise (LU of 2884 matrices: 1 16.4 ->
-        // 10.7 ms, 8 19.5 -> 14.1, 27 24.7 -> 21.2).  More matrices keep one
-        // CTA each and the slab in shared memory, whose pivot steps are longer
-        // but leave no second wave (54: 33.2 against 34.0, 162: 83 against 91)
-        if (lup::panel_shape(n - off, 1, C, threads) && (int64_t)C * c.batch <= dev_sms())
-            return lup::launch_panel<Planar, TS, 1>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
-                                                    C, threads);
-        if (lup::panel_shape(n - off, 2, C, threads) && (int64_t)C * c.batch <= dev_sms())
-            return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
-                                                    C, threads);
-        MNPB_TRY(smem_opt_in(panel_slab_kernel<8>, 200 * 1024, "panel_slab_kernel<8>"));
-        MNPB_TRY(smem_opt_in(panel_slab_kernel<4>, 200 * 1024, "panel_slab_kernel<4>"));
-        // more matrices than SMs: 4-column slabs, half the shared memory, so
-        // that two CTAs share an SM and the batch runs in one wave
-        const int64_t slab8 = (int64_t)8 * (n - off) * 8, slab4 = slab8 / 2;
-        if (c.batch > dev_sms() && w % 4 == 0 && w <= TS && slab4 <= 100 * 1024) {
-            panel_slab_kernel<4><<<c.batch, SLAB_THREADS, (size_t)slab4, c.s>>>(
-                n, off, w, A.p, A.ld, A.plane, A.stride, ipiv, sP, info);
-            MNPB_LAUNCH_CHECK("panel_slab_kernel<4>(f32)");
-            return MNPB_OK;
-        }
-        if (w % 8 == 0 && w <= TS && slab8 <= 200 * 1024) {
-            panel_slab_kernel<8><<<c.batch, SLAB_THREADS, (size_t)slab8, c.s>>>(
-                n, off, w, A.p, A.ld, A.plane, A.stride, ipiv, sP, info);
-            MNPB_LAUNCH_CHECK("panel_slab_kernel(f32)");
-            return MNPB_OK;
-        }
-        if (lup::panel_shape(n - off, 2, C, threads))
-            return lup::launch_panel<Planar, TS, 2>(c.s, n, off, w, mat, ipiv, sP, info, c.batch,
-                                                    C, threads);
-        panel_kernel<<<c.batch, PANEL_THREADS, 0, c.s>>>(n, off, w, A.p, A.ld, A.plane, A.stride,
-                                                         ipiv, sP, info);
-        MNPB_LAUNCH_CHECK("panel_kernel(f32)");
-        return MNPB_OK;
-    }
-    const int w1 = split_point(w);
+    if (w <= LB) return block_getrf(c, n, off, w, A, ipiv, sP, info);
+    const int w1 = split_tl(w);
     SwpSegs pl;
     MNPB_TRY(rgetrf(c, n, off, w1, A, ipiv, sP, info, pl));
     // one launch: what the left half owes (pivots up to off + w1) and the

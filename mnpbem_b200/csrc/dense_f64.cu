@@ -8,6 +8,7 @@
 #include "common.cuh"
 #include "dense_f64.cuh"
 #include "lu_panel.cuh"
+#include "interchange.cuh"
 #include "trsv_cluster.cuh"
 #include "skinny.cuh"
 
@@ -324,56 +325,6 @@ __global__ void colswp_kernel(cd *X, int64_t ldx, int64_t sX, int m, const int32
 }
 
 // ---------------------------------------------------------------------------
-// Row interchanges.  A sequence of interchanges (c, p_c), c ascending, p_c >= c,
-// is composed into a gather before any row moves: row c ends with the value
-// that row p_c held just before step c, which is V(c') of the last earlier
-// step c' with the same target, or the original row p_c; V(c), the value of
-// row c before step c, is V of the last earlier step that targeted c, or the
-// original row c.  Steps with one target are chained (next), so each step
-// walks the few that share its target instead of all that precede it.
-// Shared memory: head of every target row met, by its slot.
-// ---------------------------------------------------------------------------
-constexpr int SWN = 128;   // interchanges composed by one strip CTA
-
-struct Swaps {             // in shared memory
-    int p[SWN];            // target of step c, relative to the first step's row
-    int par[SWN];          // last earlier step that targeted row c, or -1
-    int out[SWN];          // row (relative) whose value ends in row c
-    int tail[SWN];         // for the last step of a target below the steps' own rows:
-                           // the row whose value ends there; else -1
-};
-
-// compose steps [0, ns), ns <= SWN <= blockDim.x, one thread a step; ends with a barrier
-__device__ __forceinline__ void swaps_compose(Swaps &w, const int32_t *ipiv, int base, int ns) {
-    const int c = threadIdx.x;
-    if (c < ns) w.p[c] = ipiv[c] - base;
-    __syncthreads();
-    const int t = c < ns ? w.p[c] : -1;
-    int par = -1, prev = -1;              // last earlier step with target c / target t
-    bool last = t >= ns;
-    for (int e = 0; e < ns; ++e) {
-        const int pe = w.p[e];
-        if (e < c) {
-            if (pe == c && e != c) par = e;
-            if (pe == t) prev = e;
-        } else if (e > c && pe == t) {
-            last = false;
-        }
-    }
-    if (c < ns) w.par[c] = par;
-    __syncthreads();
-    if (c < ns) {
-        auto before = [&](int e) {        // V(e)
-            while (w.par[e] >= 0) e = w.par[e];
-            return e;
-        };
-        w.out[c] = t == c ? before(c) : prev >= 0 ? before(prev) : t;
-        w.tail[c] = last ? before(c) : -1;
-    }
-    __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
 // Triangular solves on a diagonal block of up to SN = 128 rows, one CTA per
 // strip of SV right-hand sides (32, or 16 while those strips are too few to
 // give every SM one) held in shared memory.
@@ -422,7 +373,7 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
     cd *X = strip_sm;                          // [SN][SST], rows in solve order
     cd *M = strip_sm + SN * SST;               // [2][32][MST]: M(l, k) at [k][l]
     __shared__ cd dinv[32];
-    __shared__ Swaps sw;
+    __shared__ swp::Swaps sw;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int kb = g.kb, mode = g.mode;
     const bool fwd = mode == 0 || mode == 2, left = mode < 2, unit = mode == 0 || mode == 3;
@@ -463,7 +414,7 @@ __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
     if (solve) stage(0, 0, 0);
     if (g.ipiv) {
         const int32_t *pv = g.ipiv + b * g.sP;
-        swaps_compose(sw, pv, g.base, kb);
+        swp::compose(sw, pv, g.base, kb);
         // gather the block's rows, and the rows below that the steps reached;
         // rows past kb and vectors past nv are zero
         for (int e = tid; e < nblk * 32 * SV; e += STHREADS) {

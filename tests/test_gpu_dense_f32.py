@@ -71,13 +71,15 @@ def test_lu_planar_zero_column(gpu_ok):
     assert np.array_equal(piv.cpu().numpy(), np.tile(np.arange(n), (2, 1)))
 
 
-@pytest.mark.parametrize('n,batch,K', [(40, 2, 1), (64, 1, 2), (65, 3, 4), (97, 1, 3), (200, 5, 1),
-                                       (331, 40, 3), (700, 1, 2)])
-def test_mixed_solve_matches_fp64(gpu_ok, n, batch, K):
+@pytest.mark.parametrize('n,batch,K,shift', [(40, 2, 1, 0), (64, 1, 2, 0), (65, 3, 4, 0),
+                                             (97, 1, 3, 1), (200, 5, 1, 1), (331, 40, 3, 0),
+                                             (700, 1, 2, 0), (700, 1, 4, 3), (1500, 2, 1, 0)])
+def test_mixed_solve_matches_fp64(gpu_ok, n, batch, K, shift):
     """The mixed factorisation's solve, refined to 1e-12 of the solution, against
     the FP64 solve of the same random systems: 1, 2, 3, 4 excitations use the
     1-, 4-, 8- and 12-column solves and products.  Both converge to the solution
-    of the FP64 operator; their difference is bounded by the refinement's last
+    of the FP64 operator (``shift`` moves the factors off 16-byte alignment after
+    the factorisation); their difference is bounded by the refinement's last
     correction and the FP64 solve's own error n eps kappa, kappa < 1e4 for
     these diagonally shifted matrices."""
     rng = torch.Generator().manual_seed(n)
@@ -126,6 +128,13 @@ def test_mixed_solve_matches_fp64(gpu_ok, n, batch, K):
          ptr(HHp[1]), ptr(Dp), ld, ptr(eps), ptr(kvac), ptr(nv), 0, ptr(piv), ptr(info),
          ptr(dinv), ptr(wm), wm.numel())
     assert not info.any()
+    if shift:
+        def moved(t):
+            buf = torch.empty(t.numel() + 4, device='cuda')
+            out = buf[shift:shift + t.numel()].view(t.shape)
+            return out.copy_(t)
+
+        GGp, HHp, Dp = moved(GGp), moved(HHp), moved(Dp)
     x = torch.empty_like(b)
     wr = torch.empty(int(L.mnpb_bemret_refine_workspace(n, batch, K)), dtype=torch.uint8,
                      device='cuda')
