@@ -11,7 +11,7 @@
 // 40 us here (3.3 TB/s); the refinement's residual, one 2884 matrix 190 -> 33
 // us, 27 matrices 0.68 -> 0.61 ms (5.9 TB/s), 12 columns of mixed sizes in one
 // pass over the matrix instead of two.  FP32, 4 columns: one 2884 matrix 460 ->
-// 23 us; 12 columns of mixed sizes 0.42 -> 0.17 ms.
+// 23 us; 12 columns of mixed sizes 0.42 -> 0.12 ms.
 #pragma once
 #include "lu_panel.cuh"
 
