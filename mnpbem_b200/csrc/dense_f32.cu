@@ -117,15 +117,18 @@ struct PlanarTri : Planar {
     // staged diagonal block: inverse of the first half, the block below it,
     // inverse of the second half, each column by column in solve order
     static constexpr int DELEMS = 3 * 32 * 32;
-    static constexpr int P = 2;
+    // two thread groups with a block row each: against one group with two block
+    // rows per thread, 12 columns (whose diagonal solves get a warp each) take
+    // 0.240 instead of 0.277 ms, 1 and 4 columns 1 to 3 % less
+    static constexpr int P = 1, H = 2, THREADS = trc::GROUP * H;
     static __device__ __forceinline__ void stage(V *D, const Mat &A, const float *dinv, int64_t b,
                                                  int n, int blk, bool lower, int tid) {
         const int nb32 = (n + 31) / 32;
         const int h0 = lower ? 0 : 1, h1 = 1 - h0;       // physical halves in solve order
-        V v[DELEMS / trc::THREADS];
+        V v[DELEMS / THREADS];
 #pragma unroll
-        for (int q = 0; q < DELEMS / trc::THREADS; ++q) {
-            const int e = tid + q * trc::THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
+        for (int q = 0; q < DELEMS / THREADS; ++q) {
+            const int e = tid + q * THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
             v[q] = fmk(0.f, 0.f);
             if (w == 1) {
                 const int gr = blk * 64 + 32 * h1 + i, gc = blk * 64 + 32 * h0 + t;
@@ -139,8 +142,8 @@ struct PlanarTri : Planar {
             }
         }
 #pragma unroll
-        for (int q = 0; q < DELEMS / trc::THREADS; ++q) {
-            const int e = tid + q * trc::THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
+        for (int q = 0; q < DELEMS / THREADS; ++q) {
+            const int e = tid + q * THREADS, w = e >> 10, i = e & 31, t = (e >> 5) & 31;
             D[lower ? e : w * 1024 + (31 - t) * 32 + 31 - i] = v[q];
         }
     }

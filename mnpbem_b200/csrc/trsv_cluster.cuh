@@ -23,10 +23,10 @@
 // 5.31 -> 0.75 / 0.96 ms; 1365, 12 columns 2.49 -> 0.40; 284, 1 column 452 ->
 // 71 us, 41 matrices 4 columns 486 -> 86 us; 41 x 1148, 3 columns 2.48 -> 0.53.
 //
-// FP32 (two block rows per update, the diagonal blocks through their halves'
+// FP32 (512 threads, two block rows per update, the diagonal blocks through their halves'
 // inverses, G1 and G2 in one launch) against the solves it replaces, per
 // triangle: 2884, 4 columns 1.05 -> 0.16 ms for one matrix, 1.06 -> 0.41 ms for
-// 27; 12 columns, 13 to 26 matrices of 284 to 2044 rows 0.78 -> 0.14 ms.
+// 27; 12 columns, 13 to 26 matrices of 284 to 2044 rows 0.78 -> 0.12 ms.
 //
 // An upper triangle is solved as a lower one with blocks and rows in reverse
 // order; "logical" indices below count in the order of the solve.
@@ -36,7 +36,7 @@
 namespace mnpb {
 namespace trc {
 
-constexpr int NB = 64, THREADS = 256, MAXC = 8;
+constexpr int NB = 64, GROUP = 256, MAXC = 8;   // threads that update one tile together
 
 __device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -50,7 +50,8 @@ struct F64 : lup::F64 {
     typedef lup::F64::Mat Mat;
     // staged diagonal block: the triangle in logical order, column by column
     static constexpr int DELEMS = NB * NB;
-    static constexpr int P = 1;      // block rows per update
+    static constexpr int P = 1, H = 1;   // block rows per update: P per thread group, H groups
+    static constexpr int THREADS = GROUP * H;
     static __device__ __forceinline__ V fma(V a, V b, V c) { return cfma(a, b, c); }
     static __device__ __forceinline__ V shfl(V v, int l) {
         return cmk(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
@@ -167,18 +168,19 @@ __device__ __forceinline__ void compose(int *w, const int32_t *ipiv, int n) {
 }
 
 template <typename T, int NC>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(T::THREADS, 1)
     trsv_kernel(int n, int m, int lower_, int unit_, typename T::Mat A,
                 const float *Dinv, typename T::Mat X, const int32_t *ipiv, int64_t sP, int C,
                 int chunks, Groups gr_) {
     typedef typename T::V V;
-    constexpr int XS = Smem<T, NC>::XS;
+    constexpr int XS = Smem<T, NC>::XS, THREADS = T::THREADS;
     extern __shared__ __align__(16) unsigned char trc_sm[];
     V *D = (V *)trc_sm;              // staged diagonal block
     V *xs = D + T::DELEMS;           // [3][NB][XS]
     V *rs = xs + 3 * NB * XS;        // [own blocks][NB][NC]
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int rl = wid * 8 + (lane & 7), q = lane >> 3;   // tile row, column group
+    // thread group, tile row, column group
+    const int hg = tid / GROUP, rl = (wid & 7) * 8 + (lane & 7), q = lane >> 3;
     const bool lower = lower_, unit = unit_;
     const int me = C > 1 ? (int)lup::cluster_rank() : 0;
     const int64_t unitid = blockIdx.x / C;
@@ -234,13 +236,13 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     };
     // tiles (i, k), (i + C, k), ...: 16 entries of each per thread (row rl,
-    // columns 4 kk + q); P tiles together share the reads of x
-    constexpr int P = T::P;
+    // columns 4 kk + q); a thread group takes P tiles, which share the reads of x
+    constexpr int P = T::P, H = T::H;
     auto fetch = [&](int i, int k, V (&t)[P][16]) {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            const bool on = i + p * C < nb;
-            const int gr = on ? phys(i + p * C) * NB + rl : n;
+            const int it = i + (hg * P + p) * C;
+            const int gr = it < nb ? phys(it) * NB + rl : n;
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk) {
                 const int gc = phys(k) * NB + 4 * kk + q;
@@ -265,13 +267,13 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            if (i + p * C >= nb) break;
+            if (i + (hg * P + p) * C >= nb) break;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 acc[p][c] = T::add(acc[p][c], T::shfl_xor(acc[p][c], 8));
                 acc[p][c] = T::add(acc[p][c], T::shfl_xor(acc[p][c], 16));
             }
-            V *r = rs + (((i - me) / C + p) * NB + rl) * NC;
+            V *r = rs + (((i - me) / C + hg * P + p) * NB + rl) * NC;
 #pragma unroll
             for (int c = 0; c < NC; ++c)
                 if ((c & 3) == q) r[c] = T::sub(r[c], acc[p][c]);
@@ -280,13 +282,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     V cur[P][16];
     // the tiles in the order of their use: column k, owned block rows i > k
-    // ascending, P at a time
+    // ascending, P H at a time
     int ti = me, tk = 0;             // next tiles to fetch
     auto first_row = [&](int k) { return k + 1 + ((me - (k + 1)) % C + C) % C; };
     ti = first_row(0);
     auto valid = [&]() { return ti < nb; };
     auto advance = [&]() {
-        ti += P * C;
+        ti += P * H * C;
         if (ti >= nb) {
             ++tk;
             ti = first_row(tk);
@@ -350,7 +352,7 @@ int launch_trsv(cudaStream_t s, bool lower, bool unit, int n, int m, const Group
     MNPB_TRY(smem_opt_in(trsv_kernel<T, NC>, smem, "trc::trsv_kernel"));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(gr.per * gr.groups * chunks * C));
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(T::THREADS);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
