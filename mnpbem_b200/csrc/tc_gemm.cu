@@ -18,7 +18,7 @@
 // memory and returns.
 //
 // Measured, one tile of K = 128: 18.2 us when four warps read C after the last
-// MMA, 11.1 with eight that have C one chunk ahead; 27 x
+// MMA, 11.1 with eight that have C one chunk ahead, 7.3 with 32 columns; 27 x
 // 2884 x 128 x 128 59 -> 50 us (bound by C's traffic, 4.8 TB/s), 1440 x 2884 x
 // 1440 113 -> 84 us.  Large batched products are bound by the power limit and the
 // shared-memory traffic of the operands: 27 x 1440 x 1440 x 1440 1191 -> 1168 us
@@ -815,9 +815,21 @@ static int launch_tf32(cudaStream_t s, const CUtensorMap &mA, const CUtensorMap 
 
 template <bool AMN>
 static int launch_any(cudaStream_t s, const CUtensorMap &mA, const CUtensorMap &mAi,
-                      const CMatF &B, int M, int N, int K, int Kp, int Mp, int batch, Epi ep) {
-    if (N <= 32) return launch_tf32<32, AMN>(s, mA, mAi, B, M, N, K, Kp, Mp, batch, ep);
-    if (N <= 64 || g_cfg_bn.load(std::memory_order_relaxed) == 64)
+                      const CMatF &B, int M, int N, int K, int Kp, int Mp, int batch, Epi ep,
+                      bool in_place) {
+    // Narrow tiles while those are one wave: such a product is bound by one
+    // tile's latency (loads of K, then its epilogue), not by the tensor cores.
+    // M, N, K, matrices: 32 / 64 / 128 columns 2884, 128, 128, 1 (92 / 46 / 23
+    // tiles) 7.4 / 8.8 / 11.6 us; 892, 892, 256, 1 (196 / 98 / 49) 20.0 / 12.2 /
+    // 15.0; 768, 768, 768, 2 (288 / 144 / 72) 45.3 / 25.3 / 27.4; 1440, 1440,
+    // 128, 1 (540 / 276 / 144) 26.3 / 16.6 / 11.8.  Not where C overwrites A:
+    // one tile has to span the columns that its rows are read from.
+    const int64_t rows = (int64_t)Mp / BM * batch;
+    auto one_wave = [&](int bn) { return !in_place && rows * ceil_div(N, bn) <= num_sms(); };
+    if (N <= 32 || one_wave(32))
+        return launch_tf32<32, AMN>(s, mA, mAi, B, M, N, K, Kp, Mp, batch, ep);
+    if (N <= 64 || one_wave(64) ||
+        (!in_place && g_cfg_bn.load(std::memory_order_relaxed) == 64))
         return launch_tf32<64, AMN>(s, mA, mAi, B, M, N, K, Kp, Mp, batch, ep);
     return launch_tf32<128, AMN>(s, mA, mAi, B, M, N, K, Kp, Mp, batch, ep);
 }
@@ -849,7 +861,7 @@ int cgemm_tf32(cudaStream_t s, int M, int N, int K, int batch, float alpha, CMat
                           CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B));
         ProfScope ps(s, PC_TCGEMM, 8.0 * M * N * (double)K * batch);
         prof_tag("M=%d N=%d K=%d B=%d mn", M, N, K, batch);
-        return launch_any<true>(s, mAr, mAi, B, M, N, K, Kp, Mp, batch, ep);
+        return launch_any<true>(s, mAr, mAi, B, M, N, K, Kp, Mp, batch, ep, A.p == C.p);
     }
     if (work_bytes < cgemm_tf32_workspace(M, K, batch)) {
         set_error("tc_gemm: workspace too small");
@@ -872,7 +884,7 @@ int cgemm_tf32(cudaStream_t s, int M, int N, int K, int batch, float alpha, CMat
     MNPB_TRY(make_map(&mA, work, Kp, Mp, (uint64_t)batch * 2, Kp, (uint64_t)Mp * Kp, BM));
     ProfScope ps(s, PC_TCGEMM, 8.0 * M * N * (double)K * batch);
     prof_tag("M=%d N=%d K=%d B=%d", M, N, K, batch);
-    return launch_any<false>(s, mA, mA, B, M, N, K, Kp, Mp, batch, ep);
+    return launch_any<false>(s, mA, mA, B, M, N, K, Kp, Mp, batch, ep, false);
 }
 
 int tc_error_read_and_clear(cudaStream_t s, int *code) {
