@@ -7,6 +7,7 @@
 // other matrices in the batch.
 #include "common.cuh"
 #include "dense_f64.cuh"
+#include "fork.cuh"
 #include "lu_panel.cuh"
 #include "interchange.cuh"
 #include "trsv_cluster.cuh"
@@ -707,15 +708,42 @@ static int leaf(cudaStream_t s, int n, int off, int w, int batch, cd *A, int64_t
 }
 
 // Interchanges of the pivots of columns [off, off + w) on the columns
-// [j0, j1) without the pivots' own, and L^-1 on the rows [off, off + w) of
-// those right of them.
-static int swap_solve(cudaStream_t s, int off, int w, int j0, int j1, int batch, cd *A,
+// [j0, off) and [r0, j1), r0 >= off + w, and L^-1 on the rows [off, off + w) of
+// the latter.
+static int swap_solve(cudaStream_t s, int off, int w, int j0, int r0, int j1, int batch, cd *A,
                       int64_t lda, int64_t sA, const int32_t *ipiv, int64_t sP) {
-    const int skip0 = off - j0, skip1 = off + w - j0, nvec = j1 - j0;
+    if (j0 >= off && r0 >= j1) return MNPB_OK;
+    const int skip0 = off - j0, skip1 = r0 - j0, nvec = j1 - j0;
     StripArgs g{0,    w,         A + off + (int64_t)off * lda, lda, sA,
                 A + off + (int64_t)j0 * lda, lda, sA, nvec,
                 ipiv + off, sP, off, skip1, skip0, skip1};
     return launch_strip(s, g, batch);
+}
+
+// The columns [j0, j1) of a block, leaf by leaf.
+static int block_getrf(cudaStream_t s, int n, int j0, int j1, int batch, cd *A, int64_t lda,
+                       int64_t sA, int32_t *ipiv, int64_t sP, int32_t *info) {
+    for (int off = j0; off < j1;) {
+        const int w = min(leaf_width(n - off), j1 - off), c1 = off + w;
+        MNPB_TRY(leaf(s, n, off, w, batch, A, lda, sA, ipiv, sP, info));
+        MNPB_TRY(swap_solve(s, off, w, j0, c1, j1, batch, A, lda, sA, ipiv, sP));
+        MNPB_TRY(zgemm(s, n - c1, j1 - c1, w, batch, cmk(-1, 0), A + c1 + (int64_t)off * lda,
+                       lda, sA, A + off + (int64_t)c1 * lda, lda, sA, cmk(1, 0),
+                       A + c1 + (int64_t)c1 * lda, lda, sA));
+        off = c1;
+    }
+    return MNPB_OK;
+}
+
+// A block's interchanges on the columns [0, j0) (left) and [r0, r1), and its
+// update of the latter.
+static int block_update(cudaStream_t s, int n, int j0, int j1, bool left, int r0, int r1,
+                        int batch, cd *A, int64_t lda, int64_t sA, const int32_t *ipiv,
+                        int64_t sP) {
+    MNPB_TRY(swap_solve(s, j0, j1 - j0, left ? 0 : j0, r0, r1, batch, A, lda, sA, ipiv, sP));
+    return zgemm(s, n - j1, r1 - r0, j1 - j0, batch, cmk(-1, 0), A + j1 + (int64_t)j0 * lda, lda,
+                 sA, A + j0 + (int64_t)r0 * lda, lda, sA, cmk(1, 0), A + j1 + (int64_t)r0 * lda,
+                 lda, sA);
 }
 
 // Right-looking LU in blocks of SN columns; inside a block, leaf by leaf.  A
@@ -725,25 +753,45 @@ static int swap_solve(cudaStream_t s, int off, int w, int j0, int j1, int batch,
 // update's depth of 128 already runs at the GEMM's full rate.  One matrix of
 // 2884: 17.6 -> 11.2 ms, 1365 6.1 -> 4.0 ms, 284 0.79 -> 0.63 ms (with the
 // panels' reductions by redux.sync); 41 of 1148 14.5 -> 11.0 ms.
+//
+// While one wave holds the panels of all matrices, the chain panel, update of the
+// next block, panel runs on a stream of its own (high priority: its launches need
+// whole SMs) and the caller's stream has the updates of the columns beyond.  The
+// chain at block k + 1 waits for the bulk of block k before it reads the columns
+// of block k + 2, the bulk of block k for the panels of block k.  One stream ->
+// two: 2884 x 1 / 2 / 16 10.2 / 12.8 / 47.9 -> 8.9 / 10.6 / 45.2 ms, 2044 x 4 8.8 ->
+// 7.4, 1148 x 41 9.8 -> 9.1, 700 x 20 2.49 -> 2.21, 1365 x 1 3.68 -> 3.61; too little
+// to overlap below (1148 x 1 2.89 -> 2.95, 700 x 1 1.62 -> 1.66, 500 x 3 the same).
 int getrf(cudaStream_t s, int n, int batch, cd *A, int64_t lda, int64_t sA, int32_t *ipiv,
           int64_t sP, int32_t *info) {
+    int C, threads;
+    if (n > 2 * SN && (int64_t)n * batch > 1280 && lup::panel_shape(n, 1, C, threads) &&
+        (int64_t)C * batch <= device_sms()) {
+        ForkLease lease(s);
+        if (const Fork *f = lease.get()) {
+            auto chain = [&]() -> int {
+                for (int j0 = 0; j0 < n; j0 += SN) {
+                    const int j1 = min(n, j0 + SN), j2 = min(n, j1 + SN);
+                    MNPB_TRY(block_getrf(f->p, n, j0, j1, batch, A, lda, sA, ipiv, sP, info));
+                    // es: the bulk of the block before, which updated [j1, j2)
+                    if (j0 > 0) MNPB_TRY(stream_after(f->p, s, f->es));
+                    MNPB_TRY(stream_after(s, f->p, f->ep));
+                    MNPB_TRY(block_update(f->p, n, j0, j1, false, j1, j2, batch, A, lda, sA, ipiv,
+                                          sP));
+                    MNPB_TRY(block_update(s, n, j0, j1, true, j2, n, batch, A, lda, sA, ipiv, sP));
+                }
+                return MNPB_OK;
+            };
+            MNPB_TRY(stream_after(f->p, s, f->es));
+            const int rc = chain();
+            const int rj = stream_after(s, f->p, f->ep);   // also after an error
+            return rc != MNPB_OK ? rc : rj;
+        }
+    }
     for (int j0 = 0; j0 < n; j0 += SN) {
         const int j1 = min(n, j0 + SN);
-        for (int off = j0; off < j1;) {
-            const int w = min(leaf_width(n - off), j1 - off), c1 = off + w;
-            MNPB_TRY(leaf(s, n, off, w, batch, A, lda, sA, ipiv, sP, info));
-            if (j1 - j0 > w)
-                MNPB_TRY(swap_solve(s, off, w, j0, j1, batch, A, lda, sA, ipiv, sP));
-            MNPB_TRY(zgemm(s, n - c1, j1 - c1, w, batch, cmk(-1, 0), A + c1 + (int64_t)off * lda,
-                           lda, sA, A + off + (int64_t)c1 * lda, lda, sA, cmk(1, 0),
-                           A + c1 + (int64_t)c1 * lda, lda, sA));
-            off = c1;
-        }
-        if (n == j1 && j0 == 0) break;
-        MNPB_TRY(swap_solve(s, j0, j1 - j0, 0, n, batch, A, lda, sA, ipiv, sP));
-        MNPB_TRY(zgemm(s, n - j1, n - j1, j1 - j0, batch, cmk(-1, 0), A + j1 + (int64_t)j0 * lda,
-                       lda, sA, A + j0 + (int64_t)j1 * lda, lda, sA, cmk(1, 0),
-                       A + j1 + (int64_t)j1 * lda, lda, sA));
+        MNPB_TRY(block_getrf(s, n, j0, j1, batch, A, lda, sA, ipiv, sP, info));
+        MNPB_TRY(block_update(s, n, j0, j1, true, j1, n, batch, A, lda, sA, ipiv, sP));
     }
     return MNPB_OK;
 }

@@ -1,0 +1,40 @@
+// A second, high-priority stream beside the caller's, for the dependent chain of
+// a factorisation while the caller's stream carries the bulk of its updates.
+#pragma once
+#include "common.cuh"
+
+namespace mnpb {
+
+struct Fork {
+    cudaStream_t p;            // non-blocking, highest priority
+    cudaEvent_t ep, es;        // recorded on p, on the caller's stream
+    int dev;
+};
+
+// Takes a Fork of the current device from a pool for the time of one call.  None
+// (get() is null, the caller runs everything on its own stream) while `s` is being
+// captured, which would outlive the lease, or when kForks of the device are in
+// use.  A Fork goes back with its last user's work still queued: the next user's
+// follows it in stream order.
+class ForkLease {
+  public:
+    explicit ForkLease(cudaStream_t s);
+    ~ForkLease();
+    ForkLease(const ForkLease &) = delete;
+    ForkLease &operator=(const ForkLease &) = delete;
+    Fork *get() const { return f_; }
+
+  private:
+    Fork *f_;
+};
+
+// Work queued on `to` from here on follows all that `from` holds now.
+inline int stream_after(cudaStream_t to, cudaStream_t from, cudaEvent_t ev) {
+    if (cudaEventRecord(ev, from) != cudaSuccess || cudaStreamWaitEvent(to, ev, 0) != cudaSuccess) {
+        set_error("stream ordering failed: %s", cudaGetErrorString(cudaGetLastError()));
+        return MNPB_ECUDA;
+    }
+    return MNPB_OK;
+}
+
+}  // namespace mnpb

@@ -1,5 +1,6 @@
 // Error state, launch accounting and the host-side near-pair classification.
 #include "common.cuh"
+#include "fork.cuh"
 
 #include <cmath>
 #include <mutex>
@@ -74,6 +75,48 @@ int smem_opt_in(const void *fn, int bytes, const char *what) {
         }
     g_attr.push_back({fn, dev, bytes});
     return MNPB_OK;
+}
+
+static std::mutex g_fork_mu;
+static std::vector<Fork *> g_fork_free;
+static constexpr int kForks = 8;                 // per device
+static int g_fork_made[64];
+
+ForkLease::ForkLease(cudaStream_t s) : f_(nullptr) {
+    cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cst) != cudaSuccess || cst != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
+    }
+    const int dev = current_device();
+    if (dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_fork_mu);
+    for (size_t i = 0; i < g_fork_free.size(); ++i)
+        if (g_fork_free[i]->dev == dev) {
+            f_ = g_fork_free[i];
+            g_fork_free.erase(g_fork_free.begin() + (long)i);
+            return;
+        }
+    if (g_fork_made[dev] >= kForks) return;
+    int lo = 0, hi = 0;
+    Fork f{nullptr, nullptr, nullptr, dev};
+    if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&f.p, cudaStreamNonBlocking, hi) != cudaSuccess ||
+        cudaEventCreateWithFlags(&f.ep, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&f.es, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        if (f.ep) cudaEventDestroy(f.ep);
+        if (f.p) cudaStreamDestroy(f.p);
+        return;
+    }
+    ++g_fork_made[dev];
+    f_ = new Fork(f);
+}
+
+ForkLease::~ForkLease() {
+    if (!f_) return;
+    std::lock_guard<std::mutex> lk(g_fork_mu);
+    g_fork_free.push_back(f_);
 }
 
 int device_sms() {
