@@ -1,4 +1,4 @@
-"""The FP64 LU on two streams: ordered with the caller's stream on both sides,
+"""The FP64 LU and solves on two streams: ordered with the caller's stream on both sides,
 from more threads at once than there are second streams, and under the caller's
 own capture, where it stays on one stream."""
 import threading
@@ -95,3 +95,47 @@ def test_captured_by_the_caller(gpu_ok):
     g.replay()
     g.replay()
     f.check()
+
+
+def test_solves_in_halves_repeat(gpu_ok):
+    """The factorisation of a wavelength's matrices (solves split over two
+    streams) from eight threads at once: bitwise what one thread alone gets."""
+    n, B = 700, 2
+    L = _lib.lib()
+    g = torch.Generator(device='cuda').manual_seed(3)
+    kw = dict(dtype=torch.complex128, device='cuda', generator=g)
+    G0 = torch.randn(2, B, n, n, **kw) + 10 * torch.eye(n, device='cuda')
+    H0 = torch.randn(2, B, n, n, **kw)
+    eps = torch.tensor([1.77, 0.0, -4.0, 0.9] * B, dtype=torch.float64, device='cuda')
+    kv = torch.full((B,), 0.0125, dtype=torch.float64, device='cuda')
+    nv = torch.randn(n, 3, dtype=torch.float64, device='cuda', generator=g)
+    torch.cuda.synchronize()
+
+    def init():
+        G, H, D = G0.clone(), H0.clone(), torch.empty(B, n, n, dtype=torch.complex128,
+                                                      device='cuda')
+        piv = torch.zeros(3, B, n, dtype=torch.int32, device='cuda')
+        info = torch.zeros(2, B, dtype=torch.int32, device='cuda')
+        work = torch.empty(int(L.mnpb_bemret_workspace_f64(n, B)), dtype=torch.uint8,
+                           device='cuda')
+        call('mnpb_bemret_init_f64', _lib.stream_handle(), n, B, ptr(G[0]), ptr(G[1]), ptr(H[0]),
+             ptr(H[1]), ptr(D), n, n * n, ptr(eps), ptr(kv), ptr(nv), 0, ptr(piv), ptr(info),
+             ptr(work), work.numel())
+        torch.cuda.current_stream().synchronize()
+        return G, H, D
+
+    want = init()
+    assert all(bool(torch.isfinite(torch.view_as_real(x)).all()) for x in want)
+    got, ts = [None] * 8, []
+
+    def work_(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[i] = init()
+
+    for i in range(8):
+        ts.append(threading.Thread(target=work_, args=(i,)))
+        ts[-1].start()
+    for t in ts:
+        t.join()
+    for r in got:
+        assert r is not None and all(torch.equal(a, b) for a, b in zip(r, want))
