@@ -121,6 +121,18 @@ struct PlanarTri : Planar {
     // rows per thread, 12 columns (whose diagonal solves get a warp each) take
     // 0.240 instead of 0.277 ms, 1 and 4 columns 1 to 3 % less
     static constexpr int P = 1, H = 2, THREADS = trc::GROUP * H;
+    // 16 entries of one row, four columns apart
+    static __device__ __forceinline__ void load16(const Mat &m, int64_t b, int row, int col,
+                                                  V (&t)[16]) {
+        const float *re = m.A + b * m.sA + col * m.lda + row, *im = re + m.plane;
+        const int64_t step = 4 * m.lda;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            t[k] = fmk(*re, *im);
+            re += step;
+            im += step;
+        }
+    }
     static __device__ __forceinline__ void stage(V *D, const Mat &A, const float *dinv, int64_t b,
                                                  int n, int blk, bool lower, int tid) {
         const int nb32 = (n + 31) / 32;

@@ -20,8 +20,8 @@
 //
 // Measured, FP64, both triangles with the interchanges, against the recursion
 // of many-right-hand-side leaves this replaces: n = 2884, 1 / 4 columns 5.14 /
-// 5.31 -> 0.75 / 0.96 ms; 1365, 12 columns 2.49 -> 0.40; 284, 1 column 452 ->
-// 71 us, 41 matrices 4 columns 486 -> 86 us; 41 x 1148, 3 columns 2.48 -> 0.53.
+// 5.31 -> 0.62 / 0.87 ms; 1365, 12 columns 2.49 -> 0.39; 284, 1 column 452 ->
+// 71 us, 41 matrices 4 columns 486 -> 86 us; 41 x 1148, 3 columns 2.48 -> 0.45.
 //
 // FP32 (512 threads, two block rows per update, the diagonal blocks through their halves'
 // inverses, G1 and G2 in one launch) against the solves it replaces, per
@@ -52,6 +52,14 @@ struct F64 : lup::F64 {
     static constexpr int DELEMS = NB * NB;
     static constexpr int P = 1, H = 1;   // block rows per update: P per thread group, H groups
     static constexpr int THREADS = GROUP * H;
+    // 16 entries of one row, four columns apart
+    static __device__ __forceinline__ void load16(const Mat &m, int64_t b, int row, int col,
+                                                  V (&t)[16]) {
+        const cd *p = m.A + b * m.sA + col * m.lda + row;
+        const int64_t step = 4 * m.lda;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) t[k] = p[k * step];
+    }
     static __device__ __forceinline__ V fma(V a, V b, V c) { return cfma(a, b, c); }
     static __device__ __forceinline__ V shfl(V v, int l) {
         return cmk(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
@@ -243,6 +251,13 @@ __global__ void __launch_bounds__(T::THREADS, 1)
         for (int p = 0; p < P; ++p) {
             const int it = i + (hg * P + p) * C;
             const int gr = it < nb ? phys(it) * NB + rl : n;
+            // a tile inside the matrix: no bounds and addresses by steps, which
+            // were as many instructions as the products (FP64 2884, 1 / 4 columns
+            // 0.71 / 1.00 -> 0.62 / 0.87 ms; FP32 27 x 2884 5 to 9 % less)
+            if (it < nb && max(phys(it), phys(k)) * NB + NB <= n) {
+                T::load16(A, b, gr, phys(k) * NB + q, t[p]);
+                continue;
+            }
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk) {
                 const int gc = phys(k) * NB + 4 * kk + q;
