@@ -149,7 +149,7 @@ struct PlanarTri : Planar {
                 const int sb = 2 * blk + (w == 0 ? h0 : h1);
                 if (sb < nb32) {
                     const float *d = dinv + ((b * nb32 + sb) * 2) * 1024 + t * 32 + i;
-                    v[q] = fmk(__ldg(d), __ldg(d + 1024));
+                    v[q] = fmk(d[0], d[1024]);
                 }
             }
         }
@@ -191,12 +191,12 @@ struct PlanarRows : Planar {
                                                 V (&a)[R]) {
         const float *p = m.A + b * m.sA + col * m.lda + row;
         if constexpr (R == 2) {
-            const float2 x = __ldg(reinterpret_cast<const float2 *>(p));
-            const float2 y = __ldg(reinterpret_cast<const float2 *>(p + m.plane));
+            const float2 x = *reinterpret_cast<const float2 *>(p);
+            const float2 y = *reinterpret_cast<const float2 *>(p + m.plane);
             a[0] = fmk(x.x, y.x);
             a[1] = fmk(x.y, y.y);
         } else {
-            a[0] = fmk(__ldg(p), __ldg(p + m.plane));
+            a[0] = fmk(p[0], p[m.plane]);
         }
     }
     static __device__ __forceinline__ void out(const Mat &m, int64_t b, int64_t row, int64_t col,
@@ -629,6 +629,7 @@ constexpr int SSV = 32, SST = SSV + 1;
 __global__ void __launch_bounds__(128) swap_solve_kernel(int off, int kb, int j0, int j1, float *A,
                                                          int64_t lda, int64_t plane, int64_t sA,
                                                          const int32_t *ipiv, int64_t sP) {
+    grid_wait();
     __shared__ cf X[32][SST], L[32][SST];
     __shared__ swp::Swaps sw;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -735,6 +736,7 @@ struct SwpSegs {
 __global__ void laswp_kernel(float *A, int64_t lda, int64_t plane, int64_t sA, int j0, int j1,
                              const int32_t *ipiv, int64_t sP, int c0, int c1, int forward,
                              const SwpSegs segs, int use_segs) {
+    grid_wait();
     __shared__ int2 list[SWP_CHUNK];
     const int64_t b = blockIdx.y;
     const int j = j0 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -871,6 +873,7 @@ __device__ __forceinline__ int tri_at(bool lower, int i, int k) {
 __global__ void __launch_bounds__(TINV_THREADS, 2) tri_inv_kernel(int n, int lower_, const float *A,
                                                                   int64_t lda, int64_t plane,
                                                                   int64_t sA, float *out, int nb) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char tinv_smem[];
     cf *Tc = reinterpret_cast<cf *>(tinv_smem);   // [TL (TL + 1) / 2]
     __shared__ cf dinv[TL];
@@ -981,6 +984,7 @@ __global__ void __launch_bounds__(TINV_THREADS, 2) tri_inv_kernel(int n, int low
 constexpr int RT_COLS = 8;
 __global__ void __launch_bounds__(128) round_tf32_kernel(float *B, int64_t ldb, int64_t plane,
                                                          int64_t sB, int rows, int cols) {
+    grid_wait();
     const int i = threadIdx.x;
     if (i >= rows) return;
     const int c0 = blockIdx.x * RT_COLS, c1 = min(cols, c0 + RT_COLS);
@@ -1200,9 +1204,9 @@ static int trsm_rec(Ctx &c, int mode, int n, int m, CMatF T, CMatF B, const InvS
         if (fresh) {
             ProfScope ps(c.s, PC_PACK, 16.0 * (double)n * m * c.batch);   // bytes read + written
             prof_tag("round n=%d m=%d B=%d", n, m, c.batch);
-            round_tf32_kernel<<<dim3(ceil_div(m, RT_COLS), c.batch), TL, 0, c.s>>>(
-                B.p, B.ld, B.plane, B.stride, n, m);
-            MNPB_LAUNCH_CHECK("round_tf32_kernel");
+            MNPB_TRY(launch_chained("round_tf32_kernel", round_tf32_kernel,
+                                    dim3(ceil_div(m, RT_COLS), c.batch), dim3(TL), 0, c.s, 1, B.p,
+                                    B.ld, B.plane, B.stride, n, m));
         }
         return gemm(c, n, m, n, 1.f, I, B, 0.f, B, true, true);
     }
@@ -1243,10 +1247,9 @@ static int tri_inv(Ctx &c, int n, bool lower, CMatF T, float *inv, int nb) {
     const int parts = 4 * blocks <= room ? 4 : 2 * blocks <= room ? 2 : 1;
     ProfScope ps(c.s, PC_TRSM, 8.0 * TL * TL * TL / 3.0 * nb * c.batch);
     prof_tag("tri_inv n=%d B=%d %s", n, c.batch, lower ? "L" : "U");
-    tri_inv_kernel<<<dim3(nb, c.batch, parts), TINV_THREADS / parts, SMEM, c.s>>>(
-        n, lower ? 1 : 0, T.p, T.ld, T.plane, T.stride, inv, nb);
-    MNPB_LAUNCH_CHECK("tri_inv_kernel");
-    return MNPB_OK;
+    return launch_chained("tri_inv_kernel", tri_inv_kernel, dim3(nb, c.batch, parts),
+                          dim3(TINV_THREADS / parts), SMEM, c.s, 1, n, lower ? 1 : 0, T.p, T.ld,
+                          T.plane, T.stride, inv, nb);
 }
 
 // Packed-operand bytes of the largest GEMM trsm_rec issues with 128-leaves.
@@ -1342,10 +1345,8 @@ int laswp(Ctx &c, CMatF A, int j0, int j1, const int32_t *ipiv, int64_t sP, int 
     dim3 grid(ceil_div(j1 - j0, 128), c.batch);
     ProfScope ps(c.s, PC_SWAP, 0.0);
     SwpSegs none{};
-    laswp_kernel<<<grid, 128, 0, c.s>>>(A.p, A.ld, A.plane, A.stride, j0, j1, ipiv, sP, c0, c1,
-                                        forward ? 1 : 0, none, 0);
-    MNPB_LAUNCH_CHECK("laswp_kernel(f32)");
-    return MNPB_OK;
+    return launch_chained("laswp_kernel(f32)", laswp_kernel, grid, dim3(128), 0, c.s, 1, A.p, A.ld,
+                          A.plane, A.stride, j0, j1, ipiv, sP, c0, c1, forward ? 1 : 0, none, 0);
 }
 
 // One launch of the segment table t (forward order): columns [t.brk[0],
@@ -1358,10 +1359,8 @@ static int laswp_segs(Ctx &c, CMatF A, const int32_t *ipiv, int64_t sP, const Sw
     if (j1 <= j0 || t.end <= c0) return MNPB_OK;
     dim3 grid(ceil_div(j1 - j0, 128), c.batch);
     ProfScope ps(c.s, PC_SWAP, 0.0);
-    laswp_kernel<<<grid, 128, 0, c.s>>>(A.p, A.ld, A.plane, A.stride, j0, j1, ipiv, sP, c0,
-                                        t.end, 1, t, 1);
-    MNPB_LAUNCH_CHECK("laswp_kernel(f32, segments)");
-    return MNPB_OK;
+    return launch_chained("laswp_kernel(f32, segments)", laswp_kernel, grid, dim3(128), 0, c.s, 1,
+                          A.p, A.ld, A.plane, A.stride, j0, j1, ipiv, sP, c0, t.end, 1, t, 1);
 }
 
 // append segment [j0, j1) -> interchanges [cs, t.end) to table t
@@ -1442,9 +1441,9 @@ static int block_getrf(Ctx &c, int n, int off, int w, CMatF A, int32_t *ipiv, in
         {
             ProfScope ps(c.s, PC_SWAP, 0.0);
             const int strips = ceil_div(c0 - off, SSV) + ceil_div(end - c1, SSV);
-            swap_solve_kernel<<<dim3(strips, c.batch), 128, 0, c.s>>>(
-                c0, kb, off, end, A.p, A.ld, A.plane, A.stride, ipiv, sP);
-            MNPB_LAUNCH_CHECK("swap_solve_kernel");
+            MNPB_TRY(launch_chained("swap_solve_kernel", swap_solve_kernel, dim3(strips, c.batch),
+                                    dim3(128), 0, c.s, 1, c0, kb, off, end, A.p, A.ld, A.plane,
+                                    A.stride, ipiv, sP));
         }
         // L21 and U12 are stored rounded to TF32: read in place
         MNPB_TRY(gemm(c, n - c1, end - c1, kb, -1.f, A.sub(c1, c0), A.sub(c0, c1), 1.f,

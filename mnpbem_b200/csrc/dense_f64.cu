@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(GTHREADS) zgemm_kernel(int m, int n, int k, cd
                                                          const cd *__restrict__ A, int64_t lda,
                                                          int64_t sA, const cd *__restrict__ B,
                                                          int64_t ldb, int64_t sB, cd beta,
-                                                         cd *__restrict__ C, int64_t ldc,
+                                                         cd *C, int64_t ldc,
                                                          int64_t sC) {
+    grid_wait();
     constexpr int AS = BM + 2;               // A column (fixed k) stride
     constexpr int MI = BM / 32, NI = BN / 16;   // 16 x 8 fragments per warp
     extern __shared__ __align__(16) cd zsm[];
@@ -367,6 +368,7 @@ struct StripArgs {
 
 template <int SV>
 __global__ void __launch_bounds__(STHREADS) trsm_strip_kernel(StripArgs g) {
+    grid_wait();
     constexpr int SST = SV + 2;                // X's stride
     constexpr int LV = STHREADS / SV, RL = 32 / LV;   // lanes per vector, rows per lane
     constexpr int NJ = SV / 16;                // 8-column fragments per warp
@@ -553,10 +555,8 @@ static int launch_zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha
     const int smem = GSTAGES * (GK * (BM + 2) + BN * GBS) * (int)sizeof(cd);
     MNPB_TRY(smem_opt_in(zgemm_kernel<BM, BN>, smem, "zgemm_kernel"));
     dim3 grid(ceil_div(m, BM), ceil_div(n, BN), batch);
-    zgemm_kernel<BM, BN><<<grid, GTHREADS, smem, s>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB,
-                                                      beta, C, ldc, sC);
-    MNPB_LAUNCH_CHECK("zgemm_kernel");
-    return MNPB_OK;
+    return launch_chained("zgemm_kernel", zgemm_kernel<BM, BN>, grid, dim3(GTHREADS), smem, s, 1, m,
+                          n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
 }
 
 int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A, int64_t lda,
@@ -591,9 +591,8 @@ static int launch_strip_sv(cudaStream_t s, const StripArgs &g, int strips, int b
     const int smem = (SN * (SV + 2) + 2 * 32 * MST) * (int)sizeof(cd);
     MNPB_TRY(smem_opt_in(trsm_strip_kernel<SV>, smem, "trsm_strip_kernel"));
     ProfScope ps(s, PC_TRSM, 4.0 * g.kb * g.kb * (double)g.nvec * batch);
-    trsm_strip_kernel<SV><<<dim3(strips, batch), STHREADS, smem, s>>>(g);
-    MNPB_LAUNCH_CHECK("trsm_strip_kernel");
-    return MNPB_OK;
+    return launch_chained("trsm_strip_kernel", trsm_strip_kernel<SV>, dim3(strips, batch),
+                          dim3(STHREADS), smem, s, 1, g);
 }
 
 // vectors [0, g.skip0) and [g.skip1, g.nvec)

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
     __shared__ int cand_p[2][MAXC];
     __shared__ S red_v[2][MAXW];
     __shared__ int red_p[2][MAXW];
+    grid_wait();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nw = blockDim.x >> 5;
     const uint32_t me = C > 1 ? cluster_rank() : 0;
@@ -287,24 +288,8 @@ inline bool panel_shape(int m, int R, int &C, int &threads) {
 template <typename T, int W, int R>
 int launch_panel(cudaStream_t s, int n, int k0, int kb, typename T::Mat A, int32_t *ipiv,
                  int64_t sP, int32_t *info, int batch, int C, int threads) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(batch * C));
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = C > 1 ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, panel_kernel<T, W, R>, n, k0, kb, A, ipiv, sP, info, C) !=
-        cudaSuccess) {
-        set_error("LU panel: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        return MNPB_ECUDA;
-    }
-    MNPB_LAUNCH_CHECK("lup::panel_kernel");
-    return MNPB_OK;
+    return launch_chained("lup::panel_kernel", panel_kernel<T, W, R>, dim3((unsigned)(batch * C)),
+                          dim3((unsigned)threads), 0, s, C, n, k0, kb, A, ipiv, sP, info, C);
 }
 
 }  // namespace lup

@@ -31,7 +31,7 @@ struct F64 {
     static __device__ __forceinline__ V add(V a, V b) { return cadd(a, b); }
     static __device__ __forceinline__ V fma(V a, V b, V c) { return cfma(a, b, c); }
     static __device__ __forceinline__ V load(const Mat &m, int64_t b, int64_t row, int64_t col) {
-        return __ldg(m.A + b * m.sA + col * m.lda + row);
+        return m.A[b * m.sA + col * m.lda + row];
     }
     static __device__ __forceinline__ void rows(const Mat &m, int64_t b, int64_t row, int64_t col,
                                                 V (&a)[R]) {
@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(THREADS) kernel(int m, int n, int k, typename 
     typedef typename T::V V;
     constexpr int R = T::R, ROWS = ROWT * R;
     static_assert(KT % (LANES * T::U) == 0, "chunk");
+    grid_wait();
     extern __shared__ __align__(16) unsigned char skn_sm[];
     V *xs = (V *)skn_sm;                       // [KT][NC]
     V *part = xs + KT * NC;                    // [LANES][ROWS][NC], then [C][ROWS][NC] in CTA 0
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(THREADS, NC <= 8 ? 2 : 1) mma_kernel(int m, in
     // row stride 2 XS of x: 4 k rows x 4 columns of a load meet 16 banks of 8 bytes
     constexpr int NT = NC / 4, XS = 8 * NT + 2;
     constexpr int STEPS = KT / (4 * LANES);
+    grid_wait();
     extern __shared__ __align__(16) unsigned char skn_sm[];
     double *xs = (double *)skn_sm;             // [2][KT][2 XS]: both operands of a k row
     cd *part = (cd *)(xs + 4 * KT * XS);
@@ -325,26 +327,8 @@ int launch(cudaStream_t s, int m, int n, int k, int batch, typename T::Scale alp
             return kernel<T, NC>;
     }();
     if (smem > 48 * 1024) MNPB_TRY(smem_opt_in(f, 220 * 1024, "skn::kernel"));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ceil_div(m, ROWS) * C), (unsigned)batch);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = C > 1 ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, f, m, n, k, alpha, A, X, beta, Y, C) !=
-        cudaSuccess) {
-        set_error("matrix times vectors: launch failed: %s",
-                  cudaGetErrorString(cudaGetLastError()));
-        return MNPB_ECUDA;
-    }
-    MNPB_LAUNCH_CHECK("skn::kernel");
-    return MNPB_OK;
+    return launch_chained("skn::kernel", f, dim3((unsigned)(ceil_div(m, ROWS) * C), (unsigned)batch),
+                          dim3(THREADS), (size_t)smem, s, C, m, n, k, alpha, A, X, beta, Y, C);
 }
 
 // n <= 16 columns.

@@ -208,8 +208,8 @@ __device__ __forceinline__ void epi_fetch(const Epi &ep, const float *Cr, int ro
     const float *p = Cr + (int64_t)col * ep.ldc + row;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-        cr[c] = c < ncol ? __ldg(p + (int64_t)c * ep.ldc) : 0.f;
-        ci[c] = c < ncol ? __ldg(p + (int64_t)c * ep.ldc + ep.planeC) : 0.f;
+        cr[c] = c < ncol ? p[(int64_t)c * ep.ldc] : 0.f;
+        ci[c] = c < ncol ? p[(int64_t)c * ep.ldc + ep.planeC] : 0.f;
     }
 }
 
@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
                       const __grid_constant__ CUtensorMap tmBr,
                       const __grid_constant__ CUtensorMap tmBi, Epi ep, int STAGES) {
     using TL = Tile<BN>;
+    grid_wait();
     constexpr int STAGE_BYTES = TL::STAGE_BYTES;
     constexpr int TILE_BYTES = TILE_A_BYTES;
     constexpr int TMEM_COLS = TL::TMEM_COLS;
@@ -408,6 +409,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                           const __grid_constant__ CUtensorMap tmBi, Epi ep, int STAGES, int MT,
                           int NT, int ntiles) {
     using TL = Tile<BN>;
+    grid_wait();
     constexpr int STAGE_BYTES = TL::STAGE_BYTES;
     constexpr int TILE_BYTES = TILE_A_BYTES;
     constexpr int ACC_COLS = 2 * BN;
@@ -802,15 +804,13 @@ static int launch_tf32(cudaStream_t s, const CUtensorMap &mA, const CUtensorMap 
                              "cgemm_tf32_persistent"));
         const int pst = maxst;
         const int grid = (int)(ntiles < num_sms() ? ntiles : num_sms());
-        cgemm_tf32_persistent<BN, AMN><<<grid, GEMM_THREADS, TL::smem_bytes(pst), s>>>(
-            mA, mAi, mBr, mBi, ep, pst, MT, NT, (int)ntiles);
-        MNPB_LAUNCH_CHECK("cgemm_tf32_persistent");
-        return MNPB_OK;
+        return launch_chained("cgemm_tf32_persistent", cgemm_tf32_persistent<BN, AMN>, dim3(grid),
+                              dim3(GEMM_THREADS), TL::smem_bytes(pst), s, 1, mA, mAi, mBr, mBi, ep,
+                              pst, MT, NT, (int)ntiles);
     }
     dim3 grid(MT, NT, batch);
-    cgemm_tf32_kernel<BN, AMN><<<grid, GEMM_THREADS, dyn, s>>>(mA, mAi, mBr, mBi, ep, nst);
-    MNPB_LAUNCH_CHECK("cgemm_tf32_kernel");
-    return MNPB_OK;
+    return launch_chained("cgemm_tf32_kernel", cgemm_tf32_kernel<BN, AMN>, grid,
+                          dim3(GEMM_THREADS), dyn, s, 1, mA, mAi, mBr, mBi, ep, nst);
 }
 
 template <bool AMN>

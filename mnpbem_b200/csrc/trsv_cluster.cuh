@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(T::THREADS, 1)
                 int chunks, Groups gr_) {
     typedef typename T::V V;
     constexpr int XS = Smem<T, NC>::XS, THREADS = T::THREADS;
+    grid_wait();
     extern __shared__ __align__(16) unsigned char trc_sm[];
     V *D = (V *)trc_sm;              // staged diagonal block
     V *xs = D + T::DELEMS;           // [3][NB][XS]
@@ -365,25 +366,10 @@ int launch_trsv(cudaStream_t s, bool lower, bool unit, int n, int m, const Group
     const int chunks = ceil_div(m, NC);
     const int smem = (int)Smem<T, NC>::bytes(n, C);
     MNPB_TRY(smem_opt_in(trsv_kernel<T, NC>, smem, "trc::trsv_kernel"));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(gr.per * gr.groups * chunks * C));
-    cfg.blockDim = dim3(T::THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = C > 1 ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, trsv_kernel<T, NC>, n, m, lower ? 1 : 0, unit ? 1 : 0, A, Dinv,
-                           X, ipiv, sP, C, chunks, gr) != cudaSuccess) {
-        set_error("triangular solve: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        return MNPB_ECUDA;
-    }
-    MNPB_LAUNCH_CHECK("trc::trsv_kernel");
-    return MNPB_OK;
+    return launch_chained("trc::trsv_kernel", trsv_kernel<T, NC>,
+                          dim3((unsigned)(gr.per * gr.groups * chunks * C)), dim3(T::THREADS),
+                          (size_t)smem, s, C, n, m, lower ? 1 : 0, unit ? 1 : 0, A, Dinv, X, ipiv,
+                          sP, C, chunks, gr);
 }
 
 }  // namespace trc
