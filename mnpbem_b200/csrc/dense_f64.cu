@@ -883,32 +883,21 @@ static int permute_cols(cudaStream_t s, cd *X, int64_t ldx, int64_t sX, int m, i
     return MNPB_OK;
 }
 
-// A solve with m right-hand sides in two halves on two streams: the strips of one
-// (bound by their chains) run beside the products of the other (bound by the FP64
-// pipe).  part(stream, first, end) does right-hand sides [first, end).  The four
-// LUs, two right solves and one inverse of a wavelength, n x batch: 2884 x 1 55.7 ->
-// 53.8 ms, 2044 x 1 29.9 -> 28.6, 284 x 41 4.29 -> 4.04, 700 x 16 14.2 -> 13.8; nothing
-// to gain below (508 x 2 and 284 x 1 the same).
-template <typename F>
-static int in_halves(cudaStream_t s, int n, int m, int batch, F part) {
-    const int h = ceil_div(m, 128) * 64;
-    if (n > 2 * SN && (int64_t)m * batch > 1024) {
-        ForkLease lease(s);
-        if (const Fork *f = lease.get()) {
-            MNPB_TRY(stream_after(f->p, s, f->es));
-            int rc = part(f->p, 0, h);
-            if (rc == MNPB_OK) rc = part(s, h, m);
-            const int rj = stream_after(s, f->p, f->ep);   // also after an error
-            return rc != MNPB_OK ? rc : rj;
-        }
-    }
-    return part(s, 0, m);
+// Whether the right-hand sides of a solve are cut in halves (in_halves, fork.cuh):
+// the strips of one, bound by their chains, run beside the products of the other,
+// bound by the FP64 pipe.  The four LUs, two right solves and one inverse of a
+// wavelength, n x batch: 2884 x 1 55.7 -> 53.8 ms, 2044 x 1 29.9 -> 28.6, 284 x 41
+// 4.29 -> 4.04, 700 x 16 14.2 -> 13.8; nothing to gain below (508 x 2 and 284 x 1 the
+// same).
+static bool worth_halves(int n, int m, int batch) {
+    return n > 2 * SN && (int64_t)m * batch > 1024;
 }
 
 // X A = B in place on B (m x n), A = P^T L U from getrf.
 int right_solve(cudaStream_t s, int n, int m, int batch, const cd *LU, int64_t lda, int64_t sA,
                 const int32_t *ipiv, int64_t sP, cd *B, int64_t ldb, int64_t sB) {
-    MNPB_TRY(in_halves(s, n, m, batch, [&](cudaStream_t st, int i0, int i1) -> int {
+    const bool cut = worth_halves(n, m, batch);
+    MNPB_TRY(in_halves(s, m, cut, [&](cudaStream_t st, int i0, int i1) -> int {
         MNPB_TRY(trsm_run(st, n, i1 - i0, batch, LU, lda, sA, B + i0, ldb, sB));
         return trsm_rlu(st, n, i1 - i0, batch, LU, lda, sA, B + i0, ldb, sB);
     }));
@@ -935,7 +924,8 @@ int getri(cudaStream_t s, int n, int batch, const cd *LU, int64_t lda, int64_t s
           const int32_t *ipiv, int64_t sP, cd *X, int64_t ldx, int64_t sX) {
     MNPB_TRY(set_identity(s, n, batch, X, ldx, sX));
     MNPB_TRY(trsm_llu_eye(s, n, batch, LU, lda, sA, X, ldx, sX));
-    MNPB_TRY(in_halves(s, n, n, batch, [&](cudaStream_t st, int j0, int j1) -> int {
+    const bool cut = worth_halves(n, n, batch);
+    MNPB_TRY(in_halves(s, n, cut, [&](cudaStream_t st, int j0, int j1) -> int {
         return trsm_lun(st, n, j1 - j0, batch, LU, lda, sA, X + (int64_t)j0 * ldx, ldx, sX);
     }));
     return permute_cols(s, X, ldx, sX, n, n, ipiv, sP, batch);

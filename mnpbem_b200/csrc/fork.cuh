@@ -37,4 +37,23 @@ inline int stream_after(cudaStream_t to, cudaStream_t from, cudaEvent_t ev) {
     return MNPB_OK;
 }
 
+// The right-hand sides [0, m) in two halves (`cut`), the first on a second stream:
+// part(stream, first, end) does [first, end).  The halves meet at a multiple of 64;
+// up to 64 right-hand sides are one part.
+template <typename F>
+inline int in_halves(cudaStream_t s, int m, bool cut, F part) {
+    const int h = ceil_div(m, 128) * 64;
+    if (cut && h < m) {
+        ForkLease lease(s);
+        if (const Fork *f = lease.get()) {
+            MNPB_TRY(stream_after(f->p, s, f->es));
+            int rc = part(f->p, 0, h);
+            if (rc == MNPB_OK) rc = part(s, h, m);
+            const int rj = stream_after(s, f->p, f->ep);   // also after an error
+            return rc != MNPB_OK ? rc : rj;
+        }
+    }
+    return part(s, 0, m);
+}
+
 }  // namespace mnpb
