@@ -761,31 +761,37 @@ static int block_update(cudaStream_t s, int n, int j0, int j1, bool left, int r0
 // two: 2884 x 1 / 2 / 16 10.2 / 12.8 / 47.9 -> 8.9 / 10.6 / 45.2 ms, 2044 x 4 8.8 ->
 // 7.4, 1148 x 41 9.8 -> 9.1, 700 x 20 2.49 -> 2.21, 1365 x 1 3.68 -> 3.61; too little
 // to overlap below (1148 x 1 2.89 -> 2.95, 700 x 1 1.62 -> 1.66, 500 x 3 the same).
+// Where no second stream is to be had (more calls at once than the pool has, or the
+// caller captures) the columns are cut the same way on one: a product's kernel and
+// its order of summation follow from its columns, and the factors must not depend on
+// what other threads do.
 int getrf(cudaStream_t s, int n, int batch, cd *A, int64_t lda, int64_t sA, int32_t *ipiv,
           int64_t sP, int32_t *info) {
     int C, threads;
     if (n > 2 * SN && (int64_t)n * batch > 1280 && lup::panel_shape(n, 1, C, threads) &&
         (int64_t)C * batch <= device_sms()) {
         ForkLease lease(s);
-        if (const Fork *f = lease.get()) {
-            auto chain = [&]() -> int {
-                for (int j0 = 0; j0 < n; j0 += SN) {
-                    const int j1 = min(n, j0 + SN), j2 = min(n, j1 + SN);
-                    MNPB_TRY(block_getrf(f->p, n, j0, j1, batch, A, lda, sA, ipiv, sP, info));
+        const Fork *f = lease.get();
+        const cudaStream_t p = f ? f->p : s;      // no second stream: the same pieces in turn
+        auto chain = [&]() -> int {
+            for (int j0 = 0; j0 < n; j0 += SN) {
+                const int j1 = min(n, j0 + SN), j2 = min(n, j1 + SN);
+                MNPB_TRY(block_getrf(p, n, j0, j1, batch, A, lda, sA, ipiv, sP, info));
+                if (f) {
                     // es: the bulk of the block before, which updated [j1, j2)
-                    if (j0 > 0) MNPB_TRY(stream_after(f->p, s, f->es));
-                    MNPB_TRY(stream_after(s, f->p, f->ep));
-                    MNPB_TRY(block_update(f->p, n, j0, j1, false, j1, j2, batch, A, lda, sA, ipiv,
-                                          sP));
-                    MNPB_TRY(block_update(s, n, j0, j1, true, j2, n, batch, A, lda, sA, ipiv, sP));
+                    if (j0 > 0) MNPB_TRY(stream_after(p, s, f->es));
+                    MNPB_TRY(stream_after(s, p, f->ep));
                 }
-                return MNPB_OK;
-            };
-            MNPB_TRY(stream_after(f->p, s, f->es));
-            const int rc = chain();
-            const int rj = stream_after(s, f->p, f->ep);   // also after an error
-            return rc != MNPB_OK ? rc : rj;
-        }
+                MNPB_TRY(block_update(p, n, j0, j1, false, j1, j2, batch, A, lda, sA, ipiv, sP));
+                MNPB_TRY(block_update(s, n, j0, j1, true, j2, n, batch, A, lda, sA, ipiv, sP));
+            }
+            return MNPB_OK;
+        };
+        if (!f) return chain();
+        MNPB_TRY(stream_after(p, s, f->es));
+        const int rc = chain();
+        const int rj = stream_after(s, p, f->ep);   // also after an error
+        return rc != MNPB_OK ? rc : rj;
     }
     for (int j0 = 0; j0 < n; j0 += SN) {
         const int j1 = min(n, j0 + SN);

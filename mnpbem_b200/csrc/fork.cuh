@@ -39,21 +39,20 @@ inline int stream_after(cudaStream_t to, cudaStream_t from, cudaEvent_t ev) {
 
 // The right-hand sides [0, m) in two halves (`cut`), the first on a second stream:
 // part(stream, first, end) does [first, end).  The halves meet at a multiple of 64;
-// up to 64 right-hand sides are one part.
+// up to 64 right-hand sides are one part.  Without a second stream the halves follow
+// each other: a product may be summed in another order when its size is another, and
+// the result must not depend on whether the pool had a stream left.
 template <typename F>
 inline int in_halves(cudaStream_t s, int m, bool cut, F part) {
     const int h = ceil_div(m, 128) * 64;
-    if (cut && h < m) {
-        ForkLease lease(s);
-        if (const Fork *f = lease.get()) {
-            MNPB_TRY(stream_after(f->p, s, f->es));
-            int rc = part(f->p, 0, h);
-            if (rc == MNPB_OK) rc = part(s, h, m);
-            const int rj = stream_after(s, f->p, f->ep);   // also after an error
-            return rc != MNPB_OK ? rc : rj;
-        }
-    }
-    return part(s, 0, m);
+    if (!cut || h >= m) return part(s, 0, m);
+    ForkLease lease(s);
+    const Fork *f = lease.get();
+    if (f) MNPB_TRY(stream_after(f->p, s, f->es));
+    int rc = part(f ? f->p : s, 0, h);
+    if (rc == MNPB_OK) rc = part(s, h, m);
+    const int rj = f ? stream_after(s, f->p, f->ep) : MNPB_OK;   // also after an error
+    return rc != MNPB_OK ? rc : rj;
 }
 
 }  // namespace mnpb

@@ -71,3 +71,10 @@ def test_second_stream_is_used_where_there_is_enough_to_cut(calls):
     for m in (65, 128, 257, 700):
         assert [p[0] for p in calls[1, 1, m]] == [1, 0]
     assert calls[1, 0, 700] == [(0, 0, 700)]
+
+
+def test_cut_does_not_depend_on_the_second_stream(calls):
+    for cut in range(2):
+        for m in range(1, 701):
+            assert [p[1:] for p in calls[0, cut, m]] == [p[1:] for p in calls[1, cut, m]]
+            assert all(on == 0 for on, _, _ in calls[0, cut, m])
