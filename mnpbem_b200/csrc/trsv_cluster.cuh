@@ -138,13 +138,30 @@ struct Smem {
 // V(c), the row whose value sits in row c before step c, is V of the last
 // earlier step that targeted c, or c itself; row c ends with V of the last
 // earlier step with the same target as step c, or with the target's own row.
+// That takes ipiv[c] >= c, as an LU gives it; a caller's sequence with other
+// targets, whose chains could close to a ring, is followed step by step instead.
 __device__ __forceinline__ void compose(int *w, const int32_t *ipiv, int n) {
     int *p = w, *head = w + n, *next = w + 2 * n, *par = w + 3 * n;
+    int down = 1;
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
         p[c] = ipiv[c];
         head[c] = -1;
+        if (p[c] < c) down = 0;
     }
-    __syncthreads();
+    if (!__syncthreads_and(down)) {
+        for (int c = threadIdx.x; c < n; c += blockDim.x) head[c] = c;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int c = 0; c < n; ++c) {
+                const int t = p[c], r = head[c];
+                head[c] = head[t];
+                head[t] = r;
+            }
+        __syncthreads();
+        for (int c = threadIdx.x; c < n; c += blockDim.x) p[c] = head[c];
+        __syncthreads();
+        return;
+    }
     for (int c = threadIdx.x; c < n; c += blockDim.x)
         if (p[c] != c) next[c] = atomicExch(&head[p[c]], c);
     __syncthreads();
