@@ -145,6 +145,8 @@ class BatchedBEMRet(object):
 
             self._allocate('meta', n, B, K, measure)
             need = max(need, total[0])
+        if not shapes:                # no particles: nothing to hold, and no device to ask
+            return
         if self._arena is None or self._arena.numel() < need:
             self._bufs = self._arena = None
             self._arena = torch.empty(need, dtype=torch.uint8, device=self.tables[0].device)
