@@ -57,7 +57,8 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
     """Restarted, right-preconditioned GMRES on complex128 device vectors.
 
     ``apply_A(v) -> A v`` and ``apply_M(v) -> M v`` take and return flat
-    complex128 device tensors.  Stops when |b - A x| <= tol |b| (scipy
+    complex128 device tensors; ``counter.matvecs`` counts the calls of apply_A,
+    with the product that a cycle may have issued ahead of its last step.  Stops when |b - A x| <= tol |b| (scipy
     semantics, bem_iter.py:79-89: restart = min(n, maxit), at most ``maxit``
     restart cycles).  ``r0``: b - A x0 when the caller already has it.
 
@@ -175,7 +176,6 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
                 w = A(M(V[j]))
             else:
                 w, ahead = ahead, None
-                count.matvecs += 1
             w = w.reshape(-1).contiguous()
             if kc == 0:
                 call('mnpb_gmres_arnoldi', sh, L, j, ptr(V), L, ptr(w), ptr(H[j]), ptr(nrm),
@@ -198,7 +198,7 @@ def gmres(apply_A, b, tol=1e-6, maxit=200, restart=None, x0=None, apply_M=None,
             # a solve that converges at once pays for no product it drops
             if m < restart and len(known) >= 3 and \
                     known[-1] * (known[-1] / known[-2]) ** 2 > tol * bnorm:
-                ahead = apply_A(M(V[m]))
+                ahead = A(M(V[m]))
             done.synchronize()
             hn, hr = nr_host.tolist()
             known.append(hr)
