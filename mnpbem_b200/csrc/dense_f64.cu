@@ -46,10 +46,9 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, do
 
 template <int BM, int BN>
 __global__ void __launch_bounds__(GTHREADS) zgemm_kernel(int m, int n, int k, cd alpha,
-                                                         const cd *__restrict__ A, int64_t lda,
-                                                         int64_t sA, const cd *__restrict__ B,
-                                                         int64_t ldb, int64_t sB, cd beta,
-                                                         cd *C, int64_t ldc,
+                                                         const cd *A, int64_t lda, int64_t sA,
+                                                         const cd *B, int64_t ldb, int64_t sB,
+                                                         cd beta, cd *C, int64_t ldc,
                                                          int64_t sC) {
     grid_wait();
     constexpr int AS = BM + 2;               // A column (fixed k) stride
