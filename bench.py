@@ -105,11 +105,11 @@ def run_probe(args):
     * assemble: the mixed-path assembly (c128 + planar FP32 copies of G1, H1,
       G2, H2) of the 2884-face sphere for 4 wavelengths;
     * solve: mixed factorisation + FP64-refined solve of the 2884-face sphere
-      for 4 wavelengths (the streamed few-RHS triangular solves run here);
+      for 4 wavelengths (the few-column triangular solves and products run here);
     * hmat: the four-matrix H-matrix product of trirod(20, 80, [61, 31, 101])
       (9600 faces) at 600 nm, ACA cleaf 64 htol 1e-6, 4 right-hand sides;
-    * lu: mixed-precision LU (recursive, tensor-core updates, shared-memory
-      slab leaves) of 8 random 2884 x 2884 complex matrices."""
+    * lu: mixed-precision LU (blocks of 128 columns with cluster panels,
+      tensor-core updates) of 8 random 2884 x 2884 complex matrices."""
     import torch
     from mnpbem_b200 import _lib
     from mnpbem_b200._lib import call, ptr

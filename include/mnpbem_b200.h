@@ -270,8 +270,9 @@ int mnpb_bemret_solve_refine(void *stream, int64_t n, int64_t batch, int64_t nrh
 /* Batched LU / LU solve of planar FP32 matrices with TF32 tensor-core
  * updates (LU recursive down to blocks of 128 columns; triangular solves with
  * >= 128 right-hand sides apply the 128 x 128 diagonal blocks through their
- * inverses, also on the tensor cores).  Leading dimensions, planes and strides are multiples of 4 floats
- * and base pointers 16-byte aligned (tensor-core operand rule).
+ * inverses, also on the tensor cores).  Leading dimensions, planes and strides
+ * are multiples of 4 floats and base pointers 16-byte aligned (tensor-core
+ * operand rule).
  * work: mnpb_f32_workspace(n, batch) bytes. */
 int64_t mnpb_f32_workspace(int64_t n, int64_t batch);
 int mnpb_getrf_c32p(void *stream, int64_t n, int64_t batch, float *A, int64_t ld, int64_t plane,
@@ -386,13 +387,14 @@ int mnpb_tc_error(void *stream, int32_t *code);
 
 /* Failure-path check of the bounded device waits (no reference counterpart:
  * the reference's GPU path catches exceptions and falls back to the CPU,
- * mnpbem/bem/bem_ret.py:321-355).  Launches one thread that waits, with the
- * helper the kernels use, on something nothing completes -- kind 0: an
- * mbarrier (tensor-core GEMM), kind 1: a flag spin (`flag`, one device int),
- * kind 2: an mbarrier, the second helper (the triangular solves themselves
- * wait on hardware cluster barriers only) -- for at most limit_ns (<= 2e9).  The wait gives up, records its error word like
- * a kernel would, and returns; the probe then reads and clears the word and
- * returns MNPB_ETIMEOUT with a message.  The device context stays usable. */
+ * mnpbem/bem/bem_ret.py:321-355).  Launches one thread that waits on something
+ * nothing completes -- kind 0: an mbarrier, with the helper of the tensor-core
+ * GEMM; kinds 1 and 2: a flag spin (`flag`, one device int) and an mbarrier,
+ * with helpers that only this probe runs since the triangular solves wait on
+ * hardware cluster barriers -- for at most limit_ns (<= 2e9).  The wait gives
+ * up, records its error word and returns; the probe then reads and clears the
+ * word and returns MNPB_ETIMEOUT with a message.  The device context stays
+ * usable. */
 int mnpb_wait_probe(void *stream, int32_t kind, int64_t limit_ns, int32_t *flag);
 
 /* Quasistatic matrix for a batch of wavelengths: M_b = -(diag(lambda_b) + F)

@@ -62,6 +62,7 @@ int check_launch(const char *what);
 __device__ __forceinline__ void grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Number of SMs of the current device (cached per device; 148 if unknown).
 int device_sms();
 template <typename... P, typename... A>
 inline int launch_chained(const char *what, void (*k)(P...), dim3 grid, dim3 block, size_t smem,
@@ -104,8 +105,6 @@ int smem_opt_in(const void *fn, int bytes, const char *what);
 template <typename F> inline int smem_opt_in(F *fn, int bytes, const char *what) {
     return smem_opt_in((const void *)fn, bytes, what);
 }
-// Number of SMs of the current device (cached per device; 148 if unknown).
-int device_sms();
 // MNPB_EINVAL unless stream `s` belongs to the current device (the legacy
 // and per-thread default streams always do).
 int check_stream_device(cudaStream_t s, const char *what);
@@ -212,6 +211,16 @@ __device__ __forceinline__ cd cexpi(cd k, double d) {
     sincos(k.x * d, &s, &c);
     double m = exp(-k.y * d);
     return cmk(m * c, m * s);
+}
+
+// d += a b on the FP64 tensor path, one m16n8k4 tile: a 16 x 4 (rows lane / 4 and
+// lane / 4 + 8, column lane % 4), b 4 x 8 (row lane % 4, column lane / 4), d 16 x 8
+// (the rows of a, columns 2 (lane % 4) and the next)
+__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
+                 "{%6}, {%0,%1,%2,%3};"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a0), "d"(a1), "d"(b));
 }
 
 }  // namespace mnpb

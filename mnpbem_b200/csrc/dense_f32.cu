@@ -15,8 +15,6 @@
 #include "skinny.cuh"
 #include "trsv_cluster.cuh"
 
-#include <cuda.h>
-
 namespace mnpb {
 namespace f32 {
 
@@ -616,8 +614,12 @@ __global__ void __launch_bounds__(SLAB_THREADS, SW == 4 ? 2 : 1) panel_slab_kern
 
 // The pivots of a leaf's columns [off, off + kb) (kb <= 32) on the other columns
 // [j0, j1) of its block: the interchanges, composed into a gather, and for the
-// columns right of the leaf U12 = L11^-1 A12 on its rows, stored as TF32 (later
-// rows are eliminated with the stored values).  One CTA per 32 columns, four
+// columns right of the leaf U12 = L11^-1 A12 on its rows, stored as TF32.  A row is
+// rounded when it is final and the rows after it are eliminated with what is stored,
+// as the panels do: the rounding of U12 then enters A - L U once, not again through
+// the rows below.  Rounding the finished FP32 rows instead leaves a larger residual
+// of the stored factors (random matrices, relative: n = 256 1.41e-3 against 1.01e-3,
+// 512 1.70e-3 against 1.37e-3, 1024 2.10e-3 against 1.86e-3).  One CTA per 32 columns, four
 // lanes per column with eight rows each.  It replaces, inside a block of 128
 // columns, an interchange launch and one or more 32-row solve leaves per level
 // of the recursion (about 11 launches of 5 to 10 us per block become 4).
@@ -930,7 +932,8 @@ __global__ void __launch_bounds__(TINV_THREADS, 2) tri_inv_kernel(int n, int low
                     const int k = 32 * r + kk;
                     cf t[4];
 #pragma unroll
-                    for (int r2 = 0; r2 < 4; ++r2) t[r2] = r2 >= r ? Tc[tri_at(true, 32 * r2 + lane, k)] : fmk(0.f, 0.f);
+                    for (int r2 = 0; r2 < 4; ++r2)
+                        t[r2] = r2 >= r ? Tc[tri_at(true, 32 * r2 + lane, k)] : fmk(0.f, 0.f);
 #pragma unroll
                     for (int c = 0; c < TINV_CPW; ++c) {
                         const cf xk = fmk(__shfl_sync(0xffffffffu, x[c][r].x, kk),
@@ -950,7 +953,8 @@ __global__ void __launch_bounds__(TINV_THREADS, 2) tri_inv_kernel(int n, int low
                     const int k = 32 * r + kk;
                     cf t[4];
 #pragma unroll
-                    for (int r2 = 0; r2 < 4; ++r2) t[r2] = r2 <= r ? Tc[tri_at(false, 32 * r2 + lane, k)] : fmk(0.f, 0.f);
+                    for (int r2 = 0; r2 < 4; ++r2)
+                        t[r2] = r2 <= r ? Tc[tri_at(false, 32 * r2 + lane, k)] : fmk(0.f, 0.f);
                     const cf dk = dinv[k];
 #pragma unroll
                     for (int c = 0; c < TINV_CPW; ++c) {
@@ -998,8 +1002,10 @@ __global__ void __launch_bounds__(128) round_tf32_kernel(float *B, int64_t ldb, 
 }
 
 // ---------------------------------------------------------------------------
-// Few-RHS triangular solves: inverses of the 32 x 32 diagonal blocks, and the
-// bounded device waits that the failure-path probe runs.
+// Few-RHS triangular solves: inverses of the 32 x 32 diagonal blocks.  Then the
+// flag and mbarrier waits of mnpb_wait_probe, kinds 1 and 2: bounded waits for code
+// that waits on device memory or a barrier.  The solves themselves wait on
+// hardware cluster barriers only and record no error.
 // ---------------------------------------------------------------------------
 constexpr int TB = 32;
 
@@ -1583,11 +1589,11 @@ int getrs_few_pair(Ctx &c, int n, int m, CMatF LU, const float *LU2, const int32
     return getrs(c, n, m, L2, ipiv2, sP, B2);
 }
 
-// Failure-path probe of the triangular solves' two wait helpers: kind 1
-// spins with wait_flag on a zeroed flag for the value 1 (which nothing
-// writes), kind 2 waits with sbar_wait on an mbarrier that expects one
-// arrival and never gets it.  Each gives up after `limit_ns`, records code 9
-// in the error word as a solve would, and returns.
+// Failure-path probe of the two wait helpers above: kind 1 spins with
+// wait_flag on a zeroed flag for the value 1 (which nothing writes), kind 2
+// waits with sbar_wait on an mbarrier that expects one arrival and never gets
+// it.  Each gives up after `limit_ns`, records code 9 in the error word and
+// returns.
 __global__ void trsv_wait_probe_kernel(int kind, const int *flag, uint64_t limit_ns) {
     __shared__ __align__(8) uint64_t bar;
     bool ok;

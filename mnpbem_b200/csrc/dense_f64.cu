@@ -37,12 +37,6 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool ok) {
                  "r"(ok ? 16 : 0)
                  : "memory");
 }
-__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
-                 "{%6}, {%0,%1,%2,%3};"
-                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
 
 template <int BM, int BN>
 __global__ void __launch_bounds__(GTHREADS) zgemm_kernel(int m, int n, int k, cd alpha,
@@ -564,10 +558,10 @@ int zgemm(cudaStream_t s, int m, int n, int k, int batch, cd alpha, const cd *A,
     if (m <= 0 || n <= 0 || batch <= 0) return MNPB_OK;
     ProfScope ps(s, PC_ZGEMM, 8.0 * m * n * (double)(k > 0 ? k : 0) * batch);
     // C = beta C for k <= 0
-    // 64 x 64 tiles once two CTAs per SM have one; smaller tiles until then,
-    // so that small updates and few right-hand sides spread over the SMs
-    // (2800 x 32 x 32, 2 matrices: 20.7 -> 14.6 us; 2884 x 4 x 2884, which a
-    // 64-column tile padded 16-fold: 795 -> 157 us)
+    // 64 x 64 tiles once two CTAs per SM have one; smaller tiles until then, so that
+    // small updates spread over the SMs (2800 x 32 x 32, 2 matrices: 20.7 -> 14.6 us).
+    // Up to 16 columns go to the few-vector kernels (2884 x 4 x 2884, which a
+    // 64-column tile padded 16-fold: 795 us, on 32 x 32 tiles 157, there 40)
     const int kk = k > 0 ? k : 0;
     if (n <= 16 && kk > 0)
         return skn::run<skn::F64>(s, m, n, kk, batch, alpha, {(cd *)A, lda, sA},

@@ -355,7 +355,8 @@ extern "C" int mnpb_gmres_update(void *stream, int64_t L, int64_t m, const doubl
     if (m == 0) return MNPB_OK;
     MNPB_REQUIRE(H && g && V && y && x, "gmres_update: null pointer");
     cudaStream_t s = as_stream(stream);
-    gm::backsub_kernel<<<1, gm::BS_T, (size_t)m * 16, s>>>((int)m, (const cd *)H, ldh, (const cd *)g, (cd *)y);
+    gm::backsub_kernel<<<1, gm::BS_T, (size_t)m * 16, s>>>((int)m, (const cd *)H, ldh,
+                                                           (const cd *)g, (cd *)y);
     gm::update_kernel<<<(unsigned)((L + 255) / 256), 256, (size_t)m * 16, s>>>(
         L, (int)m, (const cd *)V, ldv, (const cd *)y, (cd *)x);
     count_launch(1);

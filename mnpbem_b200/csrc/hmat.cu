@@ -294,12 +294,6 @@ __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ float2 ld_stream(const float2 *p) { return __ldcs(p); }
-__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
-                 "{%6}, {%0,%1,%2,%3};"
-                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
 
 // A unit of MT 16-row tiles and 4 S columns, S = 8 / MT, in the fragment
 // layout: a[s][m][h] is row 16 m + g + 8 h, column 4 s + t (g = lane / 4,

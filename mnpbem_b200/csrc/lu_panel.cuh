@@ -2,9 +2,12 @@
 // block cluster.
 //
 // One cluster of C CTAs factors the columns [k0, k0 + kb) (kb <= W) of one
-// matrix over the rows [k0, n).  Every thread keeps R rows x W columns in
-// registers from load to store, so a column step touches no memory but the
-// pivot row: the rows are dealt to the CTAs in blocks of R * blockDim.x.
+// matrix over the rows [k0, n).  Every thread keeps R rows x W columns from load
+// to store, so a column step touches no memory but the pivot row: the rows are
+// dealt to the CTAs in blocks of R * blockDim.x.  In registers, but for what does not
+// fit in the 168 that 384 threads leave each: FP64 spills 44 bytes of stores and 356
+// of loads (-Xptxas -v) with 32 columns, 40 and 108 with 16 of two rows, 416 and 624
+// with 8 of four; FP32 with 32 columns takes 122 registers and none.
 //
 // What bounds it: the chain of kb dependent pivot steps.  A step is a warp
 // and CTA reduction of the pivot candidates, one exchange between the CTAs,

@@ -388,7 +388,7 @@ __device__ __forceinline__ void point_entry(const PointTables &t, cd k, int64_t 
 //
 // Bound by the FP64 pipe (sine and cosine, the square root and the division of
 // every pair) once enough warps are resident: the accumulators are those of NC
-// columns, not of the most a chunk can have (102 registers for one column, 166
+// columns, not of the most a chunk can have (96 registers for one column, 166
 // for four).  Membership in the refined list is one bit per face in shared
 // memory; only set bits search the list.  3072 points x 1564 faces, one column:
 // 131 -> 89 us; two points per CTA sharing a face's loads took 110 (156
@@ -398,12 +398,10 @@ constexpr int PG_CH = 4;
 constexpr int PG_BITS = 32 * 1024;        // shared memory for the bits
 
 template <int NC>
-__global__ void __launch_bounds__(PG_T, NC == 1 ? 5 : NC == 2 ? 4 : 3) point_green_kernel(PointTables t, int mode, int K,
-                                                           int diag, int use_bits,
-                                                           const double *__restrict__ k0v,
-                                                           const cd *__restrict__ sol,
-                                                           cd *__restrict__ o1,
-                                                           cd *__restrict__ o2) {
+__global__ void __launch_bounds__(PG_T, NC == 1 ? 5 : NC == 2 ? 4 : 3)
+    point_green_kernel(PointTables t, int mode, int K, int diag, int use_bits,
+                       const double *__restrict__ k0v, const cd *__restrict__ sol,
+                       cd *__restrict__ o1, cd *__restrict__ o2) {
     extern __shared__ uint32_t pg_bits[];
     const int64_t i = blockIdx.x;
     const int64_t b = blockIdx.z;

@@ -151,6 +151,9 @@ __global__ void __launch_bounds__(THREADS) kernel(int m, int n, int k, typename 
 #pragma unroll
         for (int c = 0; c < NC; ++c) part[(kl * ROWS + rt * R + r) * NC + c] = acc[r][c];
     __syncthreads();
+    // finish() written out: with the call the loop above is compiled another way (FP64, 4
+    // columns: 70 registers instead of 80), and 81 wavelengths of 2884 faces take 425
+    // instead of 393 ms, 13 of six uneven particles 148.5 instead of 146.1
     if (C > 1) {
         // sum the k lanes, send to CTA 0
         V s[(ROWS * NC + THREADS - 1) / THREADS];
@@ -184,13 +187,6 @@ __global__ void __launch_bounds__(THREADS) kernel(int m, int n, int k, typename 
     }
 }
 
-__device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
-                 "{%6}, {%0,%1,%2,%3};"
-                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
-
 // FP64 products with more than four columns.  4 NC FMAs per 16-byte element of A
 // take the FP64 pipe about as long as the memory, and in the kernel above every
 // group of four also reads x from shared memory.  Here X becomes two real
@@ -202,9 +198,9 @@ __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, doubl
 // columns 511 -> 273, 620 -> 401, 960 -> 513 us; 41 x 284, 12 columns 51 -> 42 us;
 // with four columns or fewer that one is at 3.7 to 5.7 TB/s and stays.
 template <int NC>
-__global__ void __launch_bounds__(THREADS, NC <= 8 ? 2 : 1) mma_kernel(int m, int n, int k, cd alpha,
-                                                         F64::Mat A, F64::Mat X, cd beta,
-                                                         F64::Mat Y, int C) {
+__global__ void __launch_bounds__(THREADS, NC <= 8 ? 2 : 1)
+    mma_kernel(int m, int n, int k, cd alpha, F64::Mat A, F64::Mat X, cd beta, F64::Mat Y,
+               int C) {
     // row stride 2 XS of x: 4 k rows x 4 columns of a load meet 16 banks of 8 bytes
     constexpr int NT = NC / 4, XS = 8 * NT + 2;
     constexpr int STEPS = KT / (4 * LANES);
@@ -273,13 +269,13 @@ __global__ void __launch_bounds__(THREADS, NC <= 8 ? 2 : 1) mma_kernel(int m, in
             }
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-                dmma(acc[0][j], a[u][0].x, a[u][1].x, x1[j]);
-                dmma(acc[1][j], a[u][2].x, a[u][3].x, x1[j]);
+                mma_f64(acc[0][j], a[u][0].x, a[u][1].x, x1[j]);
+                mma_f64(acc[1][j], a[u][2].x, a[u][3].x, x1[j]);
             }
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-                dmma(acc[0][j], a[u][0].y, a[u][1].y, x2[j]);
-                dmma(acc[1][j], a[u][2].y, a[u][3].y, x2[j]);
+                mma_f64(acc[0][j], a[u][0].y, a[u][1].y, x2[j]);
+                mma_f64(acc[1][j], a[u][2].y, a[u][3].y, x2[j]);
             }
             aload(a[u], k0 + KT + 4 * (kl + u * LANES) + t);
         }
@@ -327,8 +323,9 @@ int launch(cudaStream_t s, int m, int n, int k, int batch, typename T::Scale alp
             return kernel<T, NC>;
     }();
     if (smem > 48 * 1024) MNPB_TRY(smem_opt_in(f, 220 * 1024, "skn::kernel"));
-    return launch_chained("skn::kernel", f, dim3((unsigned)(ceil_div(m, ROWS) * C), (unsigned)batch),
-                          dim3(THREADS), (size_t)smem, s, C, m, n, k, alpha, A, X, beta, Y, C);
+    const dim3 grid((unsigned)(ceil_div(m, ROWS) * C), (unsigned)batch);
+    return launch_chained("skn::kernel", f, grid, dim3(THREADS), (size_t)smem, s, C, m, n, k,
+                          alpha, A, X, beta, Y, C);
 }
 
 // n <= 16 columns.

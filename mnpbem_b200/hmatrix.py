@@ -84,7 +84,9 @@ class HTopology(object):
         # most SEG entries of the leaf's list, first row << 6 | rows): one
         # warp per item
         # (6, fewer while that leaves the GPU short of warps: four matrices run
-        # in one launch, and about 32 warps per SM keep its loads in flight)
+        # in one launch, and about 32 warps on each of a B200's 148 SMs keep its
+        # loads in flight.  A constant, not the present device's count: the cut
+        # is the order of the sums, and also made where there is no device)
         total = sum(int(lptr[L + 1] - lptr[L]) * -(-int(lsize[L]) // 32)
                     for L in range(self.nleaf))
         SEG = min(6, max(2, 4 * total // (32 * 148)))
