@@ -77,10 +77,13 @@ int smem_opt_in(const void *fn, int bytes, const char *what) {
     return MNPB_OK;
 }
 
-static std::mutex g_fork_mu;
-static std::vector<Fork *> g_fork_free;
+// The second streams: fixed tables, so that taking and giving back allocate nothing
+// and cannot throw through a C entry point.
 static constexpr int kForks = 8;                 // per device
+static std::mutex g_fork_mu;
+static Fork g_forks[64][kForks];
 static int g_fork_made[64];
+static bool g_fork_busy[64][kForks];
 
 ForkLease::ForkLease(cudaStream_t s) : f_(nullptr) {
     cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
@@ -91,32 +94,32 @@ ForkLease::ForkLease(cudaStream_t s) : f_(nullptr) {
     const int dev = current_device();
     if (dev < 0 || dev >= 64) return;
     std::lock_guard<std::mutex> lk(g_fork_mu);
-    for (size_t i = 0; i < g_fork_free.size(); ++i)
-        if (g_fork_free[i]->dev == dev) {
-            f_ = g_fork_free[i];
-            g_fork_free.erase(g_fork_free.begin() + (long)i);
+    int i = 0;
+    while (i < g_fork_made[dev] && g_fork_busy[dev][i]) ++i;
+    if (i == kForks) return;
+    if (i == g_fork_made[dev]) {
+        int lo = 0, hi = 0;
+        Fork f{nullptr, nullptr, nullptr, dev};
+        if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
+            cudaStreamCreateWithPriority(&f.p, cudaStreamNonBlocking, hi) != cudaSuccess ||
+            cudaEventCreateWithFlags(&f.ep, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&f.es, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            if (f.ep) cudaEventDestroy(f.ep);
+            if (f.p) cudaStreamDestroy(f.p);
             return;
         }
-    if (g_fork_made[dev] >= kForks) return;
-    int lo = 0, hi = 0;
-    Fork f{nullptr, nullptr, nullptr, dev};
-    if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&f.p, cudaStreamNonBlocking, hi) != cudaSuccess ||
-        cudaEventCreateWithFlags(&f.ep, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&f.es, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        if (f.ep) cudaEventDestroy(f.ep);
-        if (f.p) cudaStreamDestroy(f.p);
-        return;
+        g_forks[dev][i] = f;
+        ++g_fork_made[dev];
     }
-    ++g_fork_made[dev];
-    f_ = new Fork(f);
+    g_fork_busy[dev][i] = true;
+    f_ = &g_forks[dev][i];
 }
 
 ForkLease::~ForkLease() {
     if (!f_) return;
     std::lock_guard<std::mutex> lk(g_fork_mu);
-    g_fork_free.push_back(f_);
+    g_fork_busy[f_->dev][f_ - g_forks[f_->dev]] = false;
 }
 
 int device_sms() {
